@@ -363,13 +363,16 @@ int qnb_get_energies_dev(qnb_context* ctx, qnb_energies* E, qnb_qenergies* EQ, d
 int qnb_set_graphs(qnb_context* ctx, int32_t enable);
 int qnb_profile_collect(qnb_context* ctx);
 
-/* Branches of the mixed form's evaluation (on by default): after the
-   coordinate pack the solute rows run on the context's stream, the water
-   rows and the step's further terms (qq, bonded, restraints, watpol) on a
-   second stream, the Q-environment and LRF Taylor kernels on a third, all
-   joined before the fixed-point gradient apply.  Every sum is fixed point,
-   so results are the same with enable = 0, which runs them in one stream
-   (each kernel then has the device to itself, e.g. for per-kernel timing). */
+/* Branches of the evaluation (on by default): after the coordinate pack the
+   solute pairs run on the context's stream; the water pairs, the
+   Q-environment terms, the LRF Taylor and further terms (qq, bonded,
+   restraints), and the solvent boundary terms on streams of their own, all
+   joined before the fixed-point gradient apply.  The FP64 form does the same
+   on the sphere unless excluded atoms are frozen; its box path runs in one
+   stream.  The mixed form's sums are fixed point, so its results are the same
+   with enable = 0, which runs everything in one stream (each kernel then has
+   the device to itself, e.g. for per-kernel timing); the FP64 form's atomics
+   agree to rounding, as they do between two calls. */
 int qnb_set_concurrency(qnb_context* ctx, int32_t enable);
 
 /* A group of contexts (systems of different sizes, e.g. replicas of uneven

@@ -71,11 +71,11 @@ struct qnb_context {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;   // list build: the LRF accumulation runs beside the row build
-    // mixed form's evaluation: after the coordinate pack the rows run on the
-    // main stream, the Q-environment / LRF Taylor kernels on stream2 and the
-    // rest of the step's terms on stream3, joined before the gradient apply
-    cudaStream_t stream3 = nullptr;
-    cudaEvent_t ev_pk = nullptr, ev_jb = nullptr, ev_jc = nullptr;
+    // the evaluation's branches beside the main stream (eval_branches): the
+    // Q-environment kernels on stream2, the water rows, the boundary
+    // restraints and the step's further terms on the others
+    cudaStream_t stream3 = nullptr, stream4 = nullptr, stream5 = nullptr;
+    cudaEvent_t ev_pk = nullptr, ev_j[4] = {};
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int mixed = 0;
     int use_lrf = 1;
@@ -92,7 +92,7 @@ struct qnb_context {
     DevState* d_states = nullptr;  // the same, on the device
     double* x_all = nullptr;       // [nwin][natom][3]
     double* e_all = nullptr;       // [nwin][kNumE] FP64 energy slots
-    unsigned long long* efix_all = nullptr;   // [nwin][kNumE] fixed-point slots
+    unsigned long long* efix_all = nullptr;   // [nwin][kNumE] fixed-point slots, behind e_all's
     int* cnt_all = nullptr;        // [nwin][C_NUM] list counters
     double* d_all = nullptr;       // [nwin][natom][3]
     int* d_iwhich = nullptr;
@@ -126,7 +126,7 @@ struct qnb_context {
     // variant (watpol theta_corr update step or not), valid while its key
     // (launch-geometry epoch, Tfree) matches
     bool use_graphs = true;
-    bool branches = true;            // mixed form: the evaluation's parallel branches (qnb_set_concurrency)
+    bool branches = true;            // the evaluation's parallel branches (qnb_set_concurrency)
     uint64_t epoch = 1;            // bumped whenever launch parameters change
     struct Pending {
         int k;
@@ -987,8 +987,9 @@ int alloc_state(qnb_context* c) {
     c->st.assign(W, DevState{});
     TRY(c->alloc(&c->x_all, n3 * W));
     TRY(c->alloc(&c->d_all, n3 * W));
-    TRY(c->alloc(&c->e_all, (size_t)kNumE * W));
-    TRY(c->alloc(&c->efix_all, (size_t)kNumE * W));
+    static_assert(sizeof(double) == sizeof(unsigned long long), "one block holds both kinds of slots");
+    TRY(c->alloc(&c->e_all, (size_t)2 * kNumE * W));   // FP64 slots, then the fixed-point slots
+    c->efix_all = reinterpret_cast<unsigned long long*>(c->e_all + (size_t)kNumE * W);
     TRY(c->alloc(&c->cnt_all, (size_t)C_NUM * W));
     CU(cudaMemset(c->cnt_all, 0, sizeof(int) * C_NUM * W));
     CU(cudaMemset(c->d_all, 0, sizeof(double) * n3 * W));
@@ -1076,6 +1077,10 @@ int alloc_state(qnb_context* c) {
 }
 
 int zero_acc(qnb_context* c, int nw) {
+    if (nw == c->nwin) {
+        CU(cudaMemsetAsync(c->e_all, 0, sizeof(double) * 2 * kNumE * nw, c->stream));
+        return QNB_OK;
+    }
     CU(cudaMemsetAsync(c->e_all, 0, sizeof(double) * kNumE * nw, c->stream));
     CU(cudaMemsetAsync(c->efix_all, 0, sizeof(unsigned long long) * kNumE * nw, c->stream));
     return QNB_OK;
@@ -1084,6 +1089,10 @@ int zero_acc(qnb_context* c, int nw) {
 // energies of the first nw windows: out[w*kNumE + k] (FP64 slots + fixed-point slots)
 // the energy records of nw windows copied to the pinned h_e (enqueued)
 int enqueue_energies(qnb_context* c, int nw) {
+    if (nw == c->nwin) {
+        CU(cudaMemcpyAsync(c->h_e, c->e_all, sizeof(double) * 2 * kNumE * nw, cudaMemcpyDeviceToHost, c->stream));
+        return QNB_OK;
+    }
     CU(cudaMemcpyAsync(c->h_e, c->e_all, sizeof(double) * kNumE * nw, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaMemcpyAsync(c->h_e + (size_t)kNumE * c->nwin, c->efix_all, sizeof(double) * kNumE * nw,
                        cudaMemcpyDeviceToHost, c->stream));
@@ -1258,10 +1267,55 @@ int build_lists(qnb_context* c, const Cut& cut, int nw) {
     return fail(QNB_ERR_CAPACITY, "pair lists kept overflowing");
 }
 
-// side: the caller's further terms of the step (qq, bonded, restraints,
-// watpol), enqueued on the Launch it is given
-using SideWork = std::function<int(const Launch&)>;
+// side: the caller's further terms of the step (qq, bonded, restraints), and
+// the solvent boundary terms (restrain_solvent, watpol), each enqueued on the
+// Launch it is given
+using SideWork = std::function<int(const Launch& terms, const Launch& boundary)>;
 
+// One evaluation's kernels in five branches after the coordinate pack: the
+// solute pairs on the main stream, the water pairs, the Q-environment terms,
+// the LRF Taylor and further terms, and the solvent boundary terms beside
+// them.  No branch reads what another writes, and every sum is an atomic one
+// (fixed point in the mixed form, so its result does not depend on their
+// interleaving).  A small system's step is as long as its longest branch
+// (the water rows, qq, restrain_solvent and watpol in one branch took 55 us
+// of the 104 us step of a 1,358-atom droplet); a large batch fills the device
+// from any of them.  One stream when the branches are off.
+struct EvalBranches {
+    Launch main, ww, q, side, wat;
+};
+EvalBranches fork_branches(qnb_context* c, const Launch& L, bool parallel, int* rc) {
+    EvalBranches b{L, L, L, L, L};
+    *rc = QNB_OK;
+    if (!parallel) return b;
+    b.q.st = c->stream2;
+    b.ww.st = c->stream3;
+    b.side.st = c->stream4;
+    b.wat.st = c->stream5;
+    auto fork = [&]() -> int {
+        CU(cudaEventRecord(c->ev_pk, c->stream));
+        for (cudaStream_t st : {c->stream2, c->stream3, c->stream4, c->stream5})
+            CU(cudaStreamWaitEvent(st, c->ev_pk, 0));
+        return QNB_OK;
+    };
+    *rc = fork();
+    return b;
+}
+int join_branches(qnb_context* c, bool parallel) {
+    if (!parallel) return QNB_OK;
+    const cudaStream_t st[4] = {c->stream2, c->stream3, c->stream4, c->stream5};
+    for (int k = 0; k < 4; ++k) {
+        CU(cudaEventRecord(c->ev_j[k], st[k]));
+        CU(cudaStreamWaitEvent(c->stream, c->ev_j[k], 0));
+    }
+    return QNB_OK;
+}
+
+// src/potene.f90:340-379 (in a box 326-343).  Mixed form: gather rows, the
+// water rows carrying ww + the water side of pw and the solute group rows
+// pp + the solute side of pw (each row adds its energies to the window's
+// fixed-point slots itself); in a box at each unit pair's image.  Box paths
+// without rows run on one stream.
 int compute_nonbond(qnb_context* c, int md, int nw, const SideWork& side = SideWork()) {
     if (!c->lists_built) return fail(QNB_ERR_STATE, "pair lists not built");
     Launch L = nw == 1 ? c->one() : c->all();
@@ -1270,100 +1324,54 @@ int compute_nonbond(qnb_context* c, int md, int nw, const SideWork& side = SideW
         timed(c, K_PACK, [&] { launch_pack(L); });
         ++nl;
     }
-    if (mx && (!c->m.box || c->m.box_rows)) {
-        const bool br = c->branches;
-        // three branches after the pack (every sum is fixed point, so the
-        // result does not depend on their interleaving); src/potene.f90:340-379
-        // for the nonbonded terms' meaning (in a box 326-343: the rows at each
-        // unit pair's image, the box Q kernels)
-        Launch LB = L, LC = L;
-        if (br) {
-            CU(cudaEventRecord(c->ev_pk, c->stream));
-            CU(cudaStreamWaitEvent(c->stream2, c->ev_pk, 0));
-            CU(cudaStreamWaitEvent(c->stream3, c->ev_pk, 0));
-            LB.st = c->stream2;
-            LC.st = c->stream3;
-        }
-        // rows: pp + the solute side of pw on the main stream, ww + the water
-        // side of pw first on the third branch (each row adds its energies to
-        // the window's fixed-point slots itself)
-        if (md) {
-            if (c->m.natom > c->m.nat_solute) timed_on(c, LC.st, K_WW, [&] { launch_rows_water(LC); }), ++nl;
-            timed(c, K_PP, [&] { launch_rows_solute(L, c->maxg); });   // the class times the solute rows alone
-            ++nl;
-            c->rows_pending = true;   // frow holds this evaluation's row gradients
-        }
-        // Q environment, solvent internal pairs, LRF Taylor terms
-        if (c->m.box) {
-            int nb = 0;
-            timed_on(c, LB.st, K_QW, [&] { nb = launch_box_nonbond(LB, md, mx, c->d_iwhich, c->last_cut.rcq2, 0); });
-            nl += nb;
-            c->qenv_pending = true;   // the box Q terms store the environment atoms' gradients in fq
-            if (md && c->nsi) timed_on(c, LB.st, K_WW, [&] { launch_solvent_internal(LB, c->d_si, c->d_sip, c->nsi, mx); }), ++nl;
-        } else {
-            if (c->m.natom > c->m.nat_solute) {
-                timed_on(c, LB.st, K_QW, [&] { launch_qw(LB, mx); }), ++nl;
-                if (md && c->nsi) timed_on(c, LB.st, K_WW, [&] { launch_solvent_internal(LB, c->d_si, c->d_sip, c->nsi, mx); }), ++nl;
-            }
-            timed_on(c, LB.st, K_QP, [&] { launch_qp(LB, mx); }), ++nl;
-            c->qenv_pending = true;   // fq holds this evaluation's Q-environment gradients
-        }
-        if (c->use_lrf && md) timed_on(c, LB.st, K_LRF_TAYLOR, [&] { launch_lrf_taylor(LB, c->d_iwhich, mx); }), ++nl;
-        // the caller's further terms
-        int rc = side ? side(LC) : QNB_OK;
-        if (br) {
-            CU(cudaEventRecord(c->ev_jb, c->stream2));
-            CU(cudaEventRecord(c->ev_jc, c->stream3));
-            CU(cudaStreamWaitEvent(c->stream, c->ev_jb, 0));
-            CU(cudaStreamWaitEvent(c->stream, c->ev_jc, 0));
-        }
-        c->launches += nl;
-        TRY(rc);
-        return check_launch();
-    }
-    if (c->m.box) {   // periodic box: the *_box routines, src/potene.f90:326-343
+    const bool rows = mx && (!c->m.box || c->m.box_rows);
+    // excluded_freeze writes coordinates inside the FP64 form's step (its pair
+    // kernels read them directly): one stream then
+    const bool par = c->branches && (rows || (!mx && !c->m.box && !c->freeze));
+    int rc = QNB_OK;
+    EvalBranches b = fork_branches(c, L, par, &rc);
+    TRY(rc);
+    const bool water = c->m.natom > c->m.nat_solute;
+    if (c->m.box && !rows) {   // the *_box routines
         int nb = 0;
         timed(c, K_PP, [&] { nb = launch_box_nonbond(L, md, mx, c->d_iwhich, c->last_cut.rcq2, 1); });
+        nl += nb;
         if (mx) c->qenv_pending = true;   // the box Q terms store the environment atoms' gradients in fq
-        // src/potene.f90:326-339 and 373-377: solvent internal pairs, then the LRF Taylor terms
-        if (md && c->nsi) timed(c, K_WW, [&] { launch_solvent_internal(L, c->d_si, c->d_sip, c->nsi, mx); }), ++nl;
-        if (c->use_lrf && md) timed(c, K_LRF_TAYLOR, [&] { launch_lrf_taylor(L, c->d_iwhich, mx); }), ++nl;
-        c->launches += nl + nb;
-        if (side) TRY(side(L));
-        return check_launch();
-    }
-    // call order of pot_energy_nonbonds, src/potene.f90:340-379
-    if (mx) {
-        // gather rows: water rows carry ww + the water side of pw, solute
-        // group rows pp + the solute side of pw
-        if (c->m.natom > c->m.nat_solute) {
-            if (md) timed(c, K_WW, [&] { launch_rows_water(L); }), ++nl;
-            timed(c, K_QW, [&] { launch_qw(L, mx); }), ++nl;
-            // src/potene.f90:361-366
-            if (md && c->nsi) timed(c, K_WW, [&] { launch_solvent_internal(L, c->d_si, c->d_sip, c->nsi, mx); }), ++nl;
+    } else {
+        if (md && water) {
+            timed_on(c, b.ww.st, K_WW, [&] { rows ? launch_rows_water(b.ww) : launch_ww(b.ww, mx); });
+            ++nl;
         }
         if (md) {
-            timed(c, K_PP, [&] { launch_rows_solute(L, c->maxg); });
+            if (rows) {
+                timed(c, K_PP, [&] { launch_rows_solute(L, c->maxg); });   // the class times the solute rows alone
+                c->rows_pending = true;   // frow holds this evaluation's row gradients
+            } else {
+                if (water) timed(c, K_PW, [&] { launch_pw(L, mx); }), ++nl;
+                timed(c, K_PP, [&] { launch_pp(L, mx); });
+            }
             ++nl;
-            c->rows_pending = true;   // frow holds this evaluation's row gradients
         }
-    } else {
-        if (c->m.natom > c->m.nat_solute) {
-            if (md) timed(c, K_WW, [&] { launch_ww(L, mx); }), ++nl;
-            timed(c, K_QW, [&] { launch_qw(L, mx); }), ++nl;
-            if (md && c->nsi) timed(c, K_WW, [&] { launch_solvent_internal(L, c->d_si, c->d_sip, c->nsi, mx); }), ++nl;
-            if (md) timed(c, K_PW, [&] { launch_pw(L, mx); }), ++nl;
+        if (c->m.box) {
+            int nb = 0;
+            timed_on(c, b.q.st, K_QW, [&] { nb = launch_box_nonbond(b.q, md, mx, c->d_iwhich, c->last_cut.rcq2, 0); });
+            nl += nb;
+        } else {
+            if (water) timed_on(c, b.q.st, K_QW, [&] { launch_qw(b.q, mx); }), ++nl;
+            timed_on(c, b.q.st, K_QP, [&] { launch_qp(b.q, mx); }), ++nl;
         }
-        if (md) timed(c, K_PP, [&] { launch_pp(L, mx); }), ++nl;
+        if (mx) c->qenv_pending = true;   // fq holds this evaluation's Q-environment gradients
     }
-    timed(c, K_QP, [&] { launch_qp(L, mx); }), ++nl;
-    if (mx) c->qenv_pending = true;   // fq holds this evaluation's Q-environment gradients
-    if (c->use_lrf && md) {
-        timed(c, K_LRF_TAYLOR, [&] { launch_lrf_taylor(L, c->d_iwhich, mx); });
-        ++nl;
-    }
+    // src/potene.f90:361-366 (326-339 in a box), then the LRF Taylor terms
+    if (md && c->nsi && water)
+        timed_on(c, b.ww.st, K_WW, [&] { launch_solvent_internal(b.ww, c->d_si, c->d_sip, c->nsi, mx); }), ++nl;
+    if (c->use_lrf && md) timed_on(c, b.side.st, K_LRF_TAYLOR, [&] { launch_lrf_taylor(b.side, c->d_iwhich, mx); }), ++nl;
+    // the caller's further terms; with excluded_freeze the boundary terms
+    // stay behind the kernel that puts the excluded atoms back
+    if (side) rc = side(b.side, c->freeze ? b.side : b.wat);
     c->launches += nl;
-    if (side) TRY(side(L));
+    TRY(join_branches(c, par));
+    TRY(rc);
     return check_launch();
 }
 
@@ -1483,9 +1491,13 @@ int qnb_create_batch(const qnb_topology* t, const qnb_options* opt, int32_t nwin
     if (cudaSetDevice(c->device) != cudaSuccess || cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->stream4, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->stream5, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_pk, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_jb, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_jc, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_j[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_j[1], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_j[2], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_j[3], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess)
         rc = fail(QNB_ERR_CUDA, "stream creation failed");
@@ -1526,10 +1538,11 @@ int qnb_destroy(qnb_context* c) {
     if (c->h_e) cudaFreeHost(c->h_e);
     if (c->h_md_rec) cudaFreeHost(c->h_md_rec);
     if (c->stream2) cudaStreamSynchronize(c->stream2), cudaStreamDestroy(c->stream2);
-    if (c->stream3) cudaStreamSynchronize(c->stream3), cudaStreamDestroy(c->stream3);
+    for (cudaStream_t st : {c->stream3, c->stream4, c->stream5})
+        if (st) cudaStreamSynchronize(st), cudaStreamDestroy(st);
     if (c->ev_pk) cudaEventDestroy(c->ev_pk);
-    if (c->ev_jb) cudaEventDestroy(c->ev_jb);
-    if (c->ev_jc) cudaEventDestroy(c->ev_jc);
+    for (cudaEvent_t e : c->ev_j)
+        if (e) cudaEventDestroy(e);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1829,9 +1842,9 @@ namespace {
 int enqueue_compute(qnb_context* c, double Tfree, int istep) {
     Launch L = c->all();
     TRY(zero_acc(c, c->nwin));
-    // the step's terms beside the nonbonded ones (their own branch in the
-    // mixed form: none reads what the pair kernels write)
-    auto side = [&](const Launch& S) -> int {
+    // the step's terms beside the nonbonded ones (none reads what the pair
+    // kernels write)
+    auto side = [&](const Launch& S, const Launch& B) -> int {
         const cudaStream_t st = S.st;
         timed_on(c, st, K_QQ, [&] { launch_nonbond_qq(S, c->mixed); });
         c->launches++;
@@ -1856,10 +1869,10 @@ int enqueue_compute(qnb_context* c, double Tfree, int istep) {
             c->launches++;
         }
         if (c->have_solv) {
-            timed_on(c, st, K_RESTRAIN, [&] { launch_restrain_solvent(S, c->solv, Tfree, c->mixed, c->d_wsw, c->d_heavy_solv); });
+            timed_on(c, B.st, K_RESTRAIN, [&] { launch_restrain_solvent(B, c->solv, Tfree, c->mixed, c->d_wsw, c->d_heavy_solv); });
             c->launches++;
             int nl = 0;
-            timed_on(c, st, K_WATPOL, [&] { nl = launch_watpol(S, c->solv, istep, 1, c->mixed); });
+            timed_on(c, B.st, K_WATPOL, [&] { nl = launch_watpol(B, c->solv, istep, 1, c->mixed); });
             c->launches += nl;
         }
         return check_launch();
@@ -2018,9 +2031,7 @@ int qnb_pot_energy_step(qnb_context* c, const double* x, double* d, double Tfree
     // stream order: the coordinate copy out of h_stage precedes this copy into it
     CU(cudaMemcpyAsync(c->h_stage, c->st[0].d, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CU(cudaMemsetAsync(c->st[0].d, 0, n * sizeof(double), c->stream));
-    CU(cudaMemcpyAsync(c->h_e, c->e_all, sizeof(double) * kNumE, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemcpyAsync(c->h_e + (size_t)kNumE * c->nwin, c->efix_all, sizeof(double) * kNumE,
-                       cudaMemcpyDeviceToHost, c->stream));
+    TRY(enqueue_energies(c, 1));
     CU(cudaStreamSynchronize(c->stream));
     for (size_t k = 0; k < n; ++k) d[k] += c->h_stage[k];
     const long long* fx = (const long long*)(c->h_e + (size_t)kNumE * c->nwin);

@@ -42,47 +42,56 @@ __device__ __forceinline__ double lan_uniform(unsigned long long seed, int w, in
     return (double)(z >> 11) * (1.0 / 9007199254740992.0);
 }
 
+// One atom's newvel: v and x are updated, xx takes the position before the
+// move; an atom in no temperature group keeps all three.
+__device__ __forceinline__ void newvel_atom(const MdDev& md, const MdWin& mw, int w, int i, const double* d, double* v,
+                                            double* x, double* xx) {
+    if (md.thermostat == 2) {   // newvel_lan, src/md.f90:1468-1503 (uniform random forces)
+        const double wi = md.winv[i];
+        const double step = md.vv ? 0.5 * md.dt : md.dt;
+        const double lf = 1.0 - md.lan_friction * step;
+        const double rs = sqrt(__ddiv_rn(md.lan_gkT, wi));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double re = __dmul_rn(rs, __dsub_rn(lan_uniform(md.lan_seed, w, md.istep, 3 * i + c), 0.5));
+            const double fd = __dmul_rn(__dmul_rn(__dsub_rn(d[c], re), wi), step);
+            double vk = __dsub_rn(__dmul_rn(v[c], lf), fd);
+            xx[c] = x[c];
+            x[c] = __dadd_rn(x[c], __dmul_rn(vk, md.dt));
+            if (md.vv) vk = __dsub_rn(__dmul_rn(vk, lf), fd);
+            v[c] = vk;
+        }
+        return;
+    }
+    const int g = md.thermostat == 1 ? 0 : tgroup_of(md, i);
+    if (g < 0) return;
+    const double sf = md.thermostat == 1 ? 1.0 : mw.sfact[g], wi = md.winv[i];
+    const double step = md.vv ? 0.5 * md.dt : md.dt;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double vk = __dmul_rn(__dsub_rn(v[c], __dmul_rn(__dmul_rn(d[c], wi), step)), sf);
+        xx[c] = x[c];
+        x[c] = __dadd_rn(x[c], __dmul_rn(vk, md.dt));
+        if (md.vv) vk = __dmul_rn(__dsub_rn(vk, __dmul_rn(__dmul_rn(d[c], wi), step)), sf);
+        v[c] = vk;
+    }
+}
+__device__ __forceinline__ void load3(double* r, const double* p) {
+    r[0] = p[0], r[1] = p[1], r[2] = p[2];
+}
+__device__ __forceinline__ void store3(double* p, const double* r) {
+    p[0] = r[0], p[1] = r[1], p[2] = r[2];
+}
+
 __global__ void k_md_newvel(MdDev md, const DevState* __restrict__ states) {
     const int w = blockIdx.y;
     const DevState& s = states[w];
     const size_t off = (size_t)w * 3 * md.natom;
-    double* __restrict__ v = md.v + off;
-    double* __restrict__ xx = md.xx + off;
-    double* __restrict__ x = s.x;
-    const double* __restrict__ d = s.d;
-    const MdWin& mw = md.win[w];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < md.natom; i += gridDim.x * blockDim.x) {
-        if (md.thermostat == 2) {   // newvel_lan, src/md.f90:1468-1503 (uniform random forces)
-            const double wi = md.winv[i];
-            const double step = md.vv ? 0.5 * md.dt : md.dt;
-            const double lf = 1.0 - md.lan_friction * step;
-            const double rs = sqrt(__ddiv_rn(md.lan_gkT, wi));
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int k = 3 * i + c;
-                const double re = __dmul_rn(rs, __dsub_rn(lan_uniform(md.lan_seed, w, md.istep, k), 0.5));
-                const double fd = __dmul_rn(__dmul_rn(__dsub_rn(d[k], re), wi), step);
-                double vk = __dsub_rn(__dmul_rn(v[k], lf), fd);
-                xx[k] = x[k];
-                x[k] = __dadd_rn(x[k], __dmul_rn(vk, md.dt));
-                if (md.vv) vk = __dsub_rn(__dmul_rn(vk, lf), fd);
-                v[k] = vk;
-            }
-            continue;
-        }
-        const int g = md.thermostat == 1 ? 0 : tgroup_of(md, i);
-        if (g < 0) continue;
-        const double sf = md.thermostat == 1 ? 1.0 : mw.sfact[g], wi = md.winv[i];
-        const double step = md.vv ? 0.5 * md.dt : md.dt;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int k = 3 * i + c;
-            double vk = __dmul_rn(__dsub_rn(v[k], __dmul_rn(__dmul_rn(d[k], wi), step)), sf);
-            xx[k] = x[k];
-            x[k] = __dadd_rn(x[k], __dmul_rn(vk, md.dt));
-            if (md.vv) vk = __dmul_rn(__dsub_rn(vk, __dmul_rn(__dmul_rn(d[k], wi), step)), sf);
-            v[k] = vk;
-        }
+        double d[3], v[3], x[3], xx[3];
+        load3(d, s.d + 3 * i), load3(v, md.v + off + 3 * i), load3(x, s.x + 3 * i), load3(xx, md.xx + off + 3 * i);
+        newvel_atom(md, md.win[w], w, i, d, v, x, xx);
+        store3(md.v + off + 3 * i, v), store3(s.x + 3 * i, x), store3(md.xx + off + 3 * i, xx);
     }
 }
 
@@ -134,6 +143,119 @@ __global__ void k_md_shake(MdDev md, const DevState* __restrict__ states, int mo
         }
         atomicAdd(&mw.shake_iters, (unsigned long long)nits);
         if (!ok) atomicCAS(md.fail + w, 0, m + 1);
+    }
+}
+
+// SHAKE of a rigid three-site molecule whose constraints are (a, b), (a, c),
+// (b, c) in this order (every 3-site water), with its positions in registers.
+// The sweep is k_md_shake's, operation for operation: 2 scp (wi + wj) is
+// formed as scp (2 (wi + wj)) and the two atoms share the products fx corr,
+// both exact regroupings (a factor of two, a sign), so every bit agrees.
+// FP64 throughput bounds it: about 40 operations per constraint and sweep at
+// two per clock and SM.  p: positions (corrected), r: reference positions,
+// atom-major; returns the sweeps, negative if they did not converge.
+__device__ int shake_triangle(double (&p)[9], const double (&r)[9], const double* __restrict__ dist2,
+                              const double* __restrict__ winv, int ia, int ib, int ic) {
+    constexpr int A[3] = {0, 0, 1}, B[3] = {1, 2, 2};
+    const double wi[3] = {winv[ia], winv[ib], winv[ic]};
+    double f[3][3], w2[3], d2[3], tol[3];
+    bool ready[3] = {false, false, false};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) f[c][k] = __dsub_rn(r[3 * A[c] + k], r[3 * B[c] + k]);
+        w2[c] = 2.0 * __dadd_rn(wi[A[c]], wi[B[c]]);
+        d2[c] = dist2[c];
+        tol[c] = __dmul_rn(0.0001, d2[c]);   // CONST_TOL
+    }
+    for (int nits = 1;; ++nits) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (ready[c]) continue;
+            const int i = 3 * A[c], j = 3 * B[c];
+            const double ex = __dsub_rn(p[i], p[j]), ey = __dsub_rn(p[i + 1], p[j + 1]),
+                         ez = __dsub_rn(p[i + 2], p[j + 2]);
+            const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
+            const double diff = __dsub_rn(d2[c], r2);
+            ready[c] = fabs(diff) < tol[c];
+            const double scp = __dadd_rn(__dadd_rn(__dmul_rn(ex, f[c][0]), __dmul_rn(ey, f[c][1])),
+                                         __dmul_rn(ez, f[c][2]));
+            const double corr = __ddiv_rn(diff, __dmul_rn(scp, w2[c]));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double t = __dmul_rn(f[c][k], corr);
+                p[i + k] = __dadd_rn(p[i + k], __dmul_rn(t, wi[A[c]]));
+                p[j + k] = __dsub_rn(p[j + k], __dmul_rn(t, wi[B[c]]));
+            }
+        }
+        if (ready[0] && ready[1] && ready[2]) return nits;
+        if (nits >= kShakeMaxIter) return -nits;
+    }
+}
+__device__ __forceinline__ void shake_done(const MdDev& md, int w, int m, int nits) {
+    // one count per warp: the lanes of one window's molecules add together
+    const unsigned act = __activemask();
+    const int sum = __reduce_add_sync(act, abs(nits));
+    if ((int)(threadIdx.x & 31) == __ffs(act) - 1) atomicAdd(&md.win[w].shake_iters, (unsigned long long)sum);
+    if (nits < 0) atomicCAS(md.fail + w, 0, m + 1);
+}
+// k_md_shake for contexts whose constrained molecules are all triangles
+__global__ void __launch_bounds__(32) k_md_shake_tri(MdDev md, const DevState* __restrict__ states, int mode) {
+    const int w = blockIdx.y, m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= md.nmol) return;
+    const size_t off = (size_t)w * 3 * md.natom;
+    double* X = mode == 0 ? states[w].x : md.xx + off;
+    const double* R = mode == 0 ? md.xx + off : states[w].x;
+    const int4 t = md.tri[m];
+    double p[9], r[9];
+    load3(p, X + 3 * t.x), load3(p + 3, X + 3 * t.y), load3(p + 6, X + 3 * t.z);
+    load3(r, R + 3 * t.x), load3(r + 3, R + 3 * t.y), load3(r + 6, R + 3 * t.z);
+    const int nits = shake_triangle(p, r, md.dist2 + t.w, md.winv, t.x, t.y, t.z);
+    store3(X + 3 * t.x, p), store3(X + 3 * t.y, p + 3), store3(X + 3 * t.z, p + 6);
+    shake_done(md, w, m, nits);
+}
+// The step's newvel, SHAKE and v = (x - xx)/dt in one pass, for contexts whose
+// constrained molecules are all triangles: one thread per molecule (its three
+// atoms) or per atom outside them (md.free_atoms).  Bound by SHAKE's FP64
+// operations, so the blocks are single warps that spread over all SMs; the
+// separate kernels moved every position through memory four times and ran
+// SHAKE on global memory (74 + 7 + 6 us per step of 16 windows of 1,113
+// waters; see k_md_shake for the general molecules).
+__global__ void __launch_bounds__(32) k_md_move_tri(MdDev md, const DevState* __restrict__ states) {
+    const int w = blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+    const DevState& s = states[w];
+    const size_t off = (size_t)w * 3 * md.natom;
+    double* __restrict__ V = md.v + off;
+    double* __restrict__ XX = md.xx + off;
+    const MdWin& mw = md.win[w];
+    if (t < md.nmol) {
+        const int4 q = md.tri[t];
+        const int at[3] = {q.x, q.y, q.z};
+        double p[9], r[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            double d[3], v[3];
+            load3(d, s.d + 3 * at[a]), load3(v, V + 3 * at[a]);
+            load3(p + 3 * a, s.x + 3 * at[a]), load3(r + 3 * a, XX + 3 * at[a]);
+            newvel_atom(md, mw, w, at[a], d, v, p + 3 * a, r + 3 * a);
+        }
+        const int nits = shake_triangle(p, r, md.dist2 + q.w, md.winv, q.x, q.y, q.z);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            double v[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = __ddiv_rn(__dsub_rn(p[3 * a + c], r[3 * a + c]), md.dt);
+            store3(V + 3 * at[a], v), store3(s.x + 3 * at[a], p + 3 * a), store3(XX + 3 * at[a], r + 3 * a);
+        }
+        shake_done(md, w, t, nits);
+    } else if (t < md.nmol + md.nfree) {
+        const int i = md.free_atoms[t - md.nmol];
+        double d[3], v[3], x[3], xx[3];
+        load3(d, s.d + 3 * i), load3(v, V + 3 * i), load3(x, s.x + 3 * i), load3(xx, XX + 3 * i);
+        newvel_atom(md, mw, w, i, d, v, x, xx);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] = __ddiv_rn(__dsub_rn(x[c], xx[c]), md.dt);
+        store3(V + 3 * i, v), store3(s.x + 3 * i, x), store3(XX + 3 * i, xx);
     }
 }
 
@@ -204,9 +326,8 @@ __global__ void k_md_copy_x(MdDev md, const DevState* __restrict__ states, int m
     if (blockIdx.x == 0 && threadIdx.x == 0) md.win[w].shake_iters = 0ull;
 }
 
-// temperature(): one block per window; kinetic energies summed per group
-// (all, non-excluded, excluded) by a fixed-order tree
-constexpr int kTempBlock = 256;
+constexpr int kTempBlock = 256;   // one-block-per-window kernels
+constexpr int kEkinBlock = 128;   // temperature(): atoms per block
 
 // put_back_in_box, src/simprep.f90:4177-4352: the box centre (boxcentre
 // fixed, or the plain mean of the solute atoms, else of all atoms), then every
@@ -255,59 +376,110 @@ __global__ void __launch_bounds__(kTempBlock) k_md_put_back(DevModel m, MdDev md
     }
 }
 
-__global__ void __launch_bounds__(kTempBlock) k_md_temperature(MdDev md, const uint8_t* __restrict__ excl) {
-    const int w = blockIdx.x;
-    const size_t off = (size_t)w * 3 * md.natom;
-    const double* __restrict__ v = md.v + off;
-    __shared__ double red[3 * kMaxTg][kTempBlock];
+// temperature(), src/md.f90:1379-1447: kEkinBlock atoms per block, whose
+// kinetic energies per group (all, non-excluded, excluded) are summed by a
+// fixed tree and stored; the window's last block to finish sums the blocks'
+// values in a fixed tree, so the totals depend on the atom count only.  With
+// rec it also writes the step's record.  One block per window (32 us for
+// 3,379 atoms) waited on 13 dependent rounds of loads.
+__device__ void write_record(const MdDev& md, int w, const double* e_all, const unsigned long long* efix_all,
+                             double* rec) {
+    double* r = rec + (size_t)w * kMdRec;
+    for (int k = threadIdx.x; k < kNumE; k += blockDim.x) {
+        r[k] = e_all[(size_t)w * kNumE + k];
+        reinterpret_cast<unsigned long long*>(r)[kNumE + k] = efix_all[(size_t)w * kNumE + k];
+    }
+    if (threadIdx.x == 0) {
+        const MdWin& mw = md.win[w];
+        r[2 * kNumE] = mw.ekin;
+        r[2 * kNumE + 1] = mw.temp;
+        r[2 * kNumE + 2] = mw.tfree;
+        r[2 * kNumE + 3] = (double)mw.shake_iters;
+    }
+}
+// block sums of a[0..n3) over the block's threads in a fixed tree; red[k][0] holds sum k
+__device__ __forceinline__ void tree_sums(double (*red)[kEkinBlock], const double* a, int n3) {
+#pragma unroll
+    for (int k = 0; k < 3 * kMaxTg; ++k)
+        if (k < n3) red[k][threadIdx.x] = a[k];
+    __syncthreads();
+    for (int h = kEkinBlock / 2; h > 0; h >>= 1) {
+        if (threadIdx.x < h)
+#pragma unroll
+            for (int k = 0; k < 3 * kMaxTg; ++k)
+                if (k < n3) red[k][threadIdx.x] = __dadd_rn(red[k][threadIdx.x], red[k][threadIdx.x + h]);
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(kEkinBlock) k_md_temperature(MdDev md, const uint8_t* __restrict__ excl,
+                                                               const double* __restrict__ e_all,
+                                                               const unsigned long long* __restrict__ efix_all,
+                                                               double* __restrict__ rec) {
+    const int w = blockIdx.y, n3 = 3 * md.ntg;
+    const double* __restrict__ v = md.v + (size_t)w * 3 * md.natom;
+    __shared__ double red[3 * kMaxTg][kEkinBlock];
+    __shared__ bool last;
     double a[3 * kMaxTg];
 #pragma unroll
     for (int k = 0; k < 3 * kMaxTg; ++k) a[k] = 0.0;
-    for (int i = threadIdx.x; i < md.natom; i += kTempBlock) {
-        int g = tgroup_of(md, i);
-        if (g < 0) continue;
+    const int i = blockIdx.x * kEkinBlock + threadIdx.x;
+    const int g = i < md.natom ? tgroup_of(md, i) : -1;
+    if (g >= 0) {
         const double vx = v[3 * i], vy = v[3 * i + 1], vz = v[3 * i + 2];
         double sq = __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz));
         double ek = __dmul_rn(__dmul_rn(0.5, md.mass[i]), sq);
 #pragma unroll
         for (int q = 0; q < kMaxTg; ++q) {
             if (q != g) continue;
-            a[3 * q] = __dadd_rn(a[3 * q], ek);
-            if (!excl[i]) a[3 * q + 1] = __dadd_rn(a[3 * q + 1], ek);
-            else a[3 * q + 2] = __dadd_rn(a[3 * q + 2], ek);
+            a[3 * q] = ek;
+            a[3 * q + 1] = excl[i] ? 0.0 : ek;
+            a[3 * q + 2] = excl[i] ? ek : 0.0;
         }
     }
-#pragma unroll
-    for (int k = 0; k < 3 * kMaxTg; ++k) red[k][threadIdx.x] = a[k];
-    __syncthreads();
-    for (int h = kTempBlock / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h)
-#pragma unroll
-            for (int k = 0; k < 3 * kMaxTg; ++k)
-                red[k][threadIdx.x] = __dadd_rn(red[k][threadIdx.x], red[k][threadIdx.x + h]);
-        __syncthreads();
-    }
-    if (threadIdx.x != 0) return;
+    tree_sums(red, a, n3);
     MdWin& mw = md.win[w];
-    const double boltz = md.boltz;
-    double temp = 0.0, tfree = 0.0;
-    for (int g = 0; g < md.ntg; ++g) {
-        tfree = __dadd_rn(tfree, red[3 * g + 1][0]);
-        temp = __dadd_rn(temp, red[3 * g][0]);
+    double* part = md.tpart + (size_t)w * gridDim.x * 3 * kMaxTg;
+    if (threadIdx.x < n3) part[blockIdx.x * 3 * kMaxTg + threadIdx.x] = red[threadIdx.x][0];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&mw.temp_blocks, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    if (threadIdx.x == 0) mw.temp_blocks = 0u;   // for the next call
+    __threadfence();
+#pragma unroll
+    for (int k = 0; k < 3 * kMaxTg; ++k) a[k] = 0.0;
+    for (int b = threadIdx.x; b < gridDim.x; b += kEkinBlock)
+#pragma unroll
+        for (int k = 0; k < 3 * kMaxTg; ++k)
+            if (k < n3) a[k] = __dadd_rn(a[k], __ldcg(part + b * 3 * kMaxTg + k));
+    __syncthreads();   // red is reused
+    tree_sums(red, a, n3);
+    if (threadIdx.x == 0) {
+        const double boltz = md.boltz;
+        double temp = 0.0, tfree = 0.0;
+        for (int g = 0; g < md.ntg; ++g) {
+            tfree = __dadd_rn(tfree, red[3 * g + 1][0]);
+            temp = __dadd_rn(temp, red[3 * g][0]);
+        }
+        mw.ekin = temp;
+        mw.temp = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, temp), boltz), md.ndegf);
+        mw.tfree = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, tfree), boltz), md.ndegfree);
+        for (int g = 0; g < md.ntg; ++g) {
+            mw.tg_temp[g] = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, red[3 * g][0]), boltz), md.tg_ndegf[g]);
+            mw.tg_tfree[g] = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, red[3 * g + 1][0]), boltz), md.tg_ndegfree[g]);
+            mw.tg_texcl[g] = md.tg_ndegf[g] != md.tg_ndegfree[g]
+                                 ? __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, red[3 * g + 2][0]), boltz),
+                                             __dsub_rn(md.tg_ndegf[g], md.tg_ndegfree[g]))
+                                 : red[3 * g + 2][0];
+            // Berendsen: a group with Tfree 0 keeps its previous factor inside the root
+            if (mw.tg_tfree[g] != 0.0) mw.sfact[g] = __dsub_rn(__ddiv_rn(md.temp0, mw.tg_tfree[g]), 1.0);
+            mw.sfact[g] = sqrt(__dadd_rn(1.0, __dmul_rn(__ddiv_rn(md.dt, md.tau), mw.sfact[g])));
+        }
     }
-    mw.ekin = temp;
-    mw.temp = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, temp), boltz), md.ndegf);
-    mw.tfree = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, tfree), boltz), md.ndegfree);
-    for (int g = 0; g < md.ntg; ++g) {
-        mw.tg_temp[g] = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, red[3 * g][0]), boltz), md.tg_ndegf[g]);
-        mw.tg_tfree[g] = __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, red[3 * g + 1][0]), boltz), md.tg_ndegfree[g]);
-        mw.tg_texcl[g] = md.tg_ndegf[g] != md.tg_ndegfree[g]
-                             ? __ddiv_rn(__ddiv_rn(__dmul_rn(2.0, red[3 * g + 2][0]), boltz),
-                                         __dsub_rn(md.tg_ndegf[g], md.tg_ndegfree[g]))
-                             : red[3 * g + 2][0];
-        // Berendsen: a group with Tfree 0 keeps its previous factor inside the root
-        if (mw.tg_tfree[g] != 0.0) mw.sfact[g] = __dsub_rn(__ddiv_rn(md.temp0, mw.tg_tfree[g]), 1.0);
-        mw.sfact[g] = sqrt(__dadd_rn(1.0, __dmul_rn(__ddiv_rn(md.dt, md.tau), mw.sfact[g])));
+    if (rec) {
+        __syncthreads();   // thread 0's temperatures
+        write_record(md, w, e_all, efix_all, rec);
     }
 }
 
@@ -387,23 +559,6 @@ __global__ void __launch_bounds__(kTempBlock) k_md_min_step(MdDev md, const DevS
     }
 }
 
-__global__ void k_md_record(MdDev md, int nwin, const double* __restrict__ e_all,
-                            const unsigned long long* __restrict__ efix_all, double* __restrict__ rec) {
-    const int w = blockIdx.x;
-    double* r = rec + (size_t)w * kMdRec;
-    for (int k = threadIdx.x; k < kNumE; k += blockDim.x) {
-        r[k] = e_all[(size_t)w * kNumE + k];
-        reinterpret_cast<unsigned long long*>(r)[kNumE + k] = efix_all[(size_t)w * kNumE + k];
-    }
-    if (threadIdx.x == 0) {
-        const MdWin& mw = md.win[w];
-        r[2 * kNumE] = mw.ekin;
-        r[2 * kNumE + 1] = mw.temp;
-        r[2 * kNumE + 2] = mw.tfree;
-        r[2 * kNumE + 3] = (double)mw.shake_iters;
-    }
-}
-
 // pot_energy's d = 0 and the step's SHAKE iteration count
 __global__ void k_md_clear(const DevState* __restrict__ states, size_t n3, MdWin* win) {
     double* d = states[blockIdx.y].d;
@@ -433,7 +588,21 @@ void launch_md_newvel(const Launch& L, const MdDev& md) {
 }
 void launch_md_shake(const Launch& L, const MdDev& md, int mode) {
     if (md.nmol == 0) return;
+    if (md.tri) {
+        k_md_shake_tri<<<dim3((md.nmol + 31) / 32, L.nwin), 32, 0, L.st>>>(md, L.ds, mode);
+        return;
+    }
     k_md_shake<<<atoms_grid(L, md.nmol, 64), 64, 0, L.st>>>(md, L.ds, mode);
+}
+int launch_md_move(const Launch& L, const MdDev& md) {
+    if (md.tri) {
+        k_md_move_tri<<<dim3((md.nmol + md.nfree + 31) / 32, L.nwin), 32, 0, L.st>>>(md, L.ds);
+        return 1;
+    }
+    launch_md_newvel(L, md);
+    launch_md_shake(L, md, 0);
+    if (md.nmol > 0) launch_md_velocity(L, md);
+    return md.nmol > 0 ? 3 : 1;
 }
 void launch_md_velocity(const Launch& L, const MdDev& md) {
     k_md_velocity<<<atoms_grid(L, 3 * (int64_t)md.natom, 256), 256, 0, L.st>>>(md, L.ds);
@@ -441,18 +610,17 @@ void launch_md_velocity(const Launch& L, const MdDev& md) {
 void launch_md_copy_x(const Launch& L, const MdDev& md, int mode) {
     k_md_copy_x<<<atoms_grid(L, 3 * (int64_t)md.natom, 256), 256, 0, L.st>>>(md, L.ds, mode);
 }
-void launch_md_temperature(const Launch& L, const MdDev& md, const uint8_t* excl) {
-    k_md_temperature<<<L.nwin, kTempBlock, 0, L.st>>>(md, excl);
+int md_temp_blocks(int natom) { return (natom + kEkinBlock - 1) / kEkinBlock; }
+size_t md_temp_part(int natom) { return (size_t)md_temp_blocks(natom) * 3 * kMaxTg; }
+void launch_md_temperature(const Launch& L, const MdDev& md, const uint8_t* excl, const double* e_all,
+                           const unsigned long long* efix_all, double* rec) {
+    k_md_temperature<<<dim3(md_temp_blocks(md.natom), L.nwin), kEkinBlock, 0, L.st>>>(md, excl, e_all, efix_all, rec);
 }
 void launch_md_stop_cm(const Launch& L, const MdDev& md) {
     k_md_stop_cm<<<L.nwin, kTempBlock, 0, L.st>>>(md);
 }
 void launch_md_min_step(const Launch& L, const MdDev& md, double step0, double fcut, double max_move) {
     k_md_min_step<<<L.nwin, kTempBlock, 0, L.st>>>(md, L.ds, step0, fcut, max_move);
-}
-void launch_md_record(const Launch& L, const MdDev& md, const double* e_all, const unsigned long long* efix_all,
-                      double* rec) {
-    k_md_record<<<L.nwin, 64, 0, L.st>>>(md, L.nwin, e_all, efix_all, rec);
 }
 void launch_md_clear_d(const Launch& L, const MdDev& md) {
     size_t n3 = 3 * (size_t)md.natom;

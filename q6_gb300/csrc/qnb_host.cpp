@@ -2489,6 +2489,32 @@ int qnb_md_init(qnb_context* c, const qnb_md_params* p, const double* mass, int3
     TRY(c->upload((int**)&md.mol_first, mf));
     TRY(c->upload((int2**)&md.con, con));
     TRY(c->upload((double**)&md.dist2, d2));
+    // triangles of atoms of their own (rigid 3-site waters): SHAKE in registers,
+    // fused with the move.  Any other molecule, or an atom in two molecules,
+    // keeps the general kernels for all of them.
+    std::vector<int4> tri(nmol);
+    std::vector<char> held(n, 0);
+    bool all_tri = nmol > 0;
+    for (int q = 0; q < nmol && all_tri; ++q) {
+        const int c0 = mf[q];
+        const int a = mf[q + 1] - c0 == 3 ? con[c0].x : -1;
+        all_tri = a >= 0 && con[c0 + 1].x == a && con[c0 + 2].x == con[c0].y && con[c0 + 2].y == con[c0 + 1].y;
+        if (!all_tri) break;
+        tri[q] = make_int4(a, con[c0].y, con[c0 + 1].y, c0);
+        for (int i : {tri[q].x, tri[q].y, tri[q].z}) {
+            all_tri = all_tri && !held[i];
+            held[i] = 1;
+        }
+    }
+    if (all_tri) {
+        std::vector<int> fr;
+        for (int i = 0; i < n; ++i)
+            if (!held[i]) fr.push_back(i);
+        md.nfree = (int)fr.size();
+        TRY(c->upload((int4**)&md.tri, tri));
+        TRY(c->upload((int**)&md.free_atoms, fr));
+    }
+    TRY(c->alloc(&md.tpart, md_temp_part(n) * c->nwin));
     const size_t n3 = 3 * (size_t)n;
     TRY(c->alloc(&md.ready, (size_t)std::max(1, ncons) * c->nwin));
     TRY(c->alloc(&md.v, n3 * c->nwin));
@@ -2708,16 +2734,11 @@ int qnb_md_run(qnb_context* c, int32_t nsteps, int32_t istep0, qnb_md_record* re
             c->md.istep = istep;
             timed(c, K_MD, [&] {
                 if (nh) launch_md_nh(L, c->md);
-                launch_md_newvel(L, c->md);
-                launch_md_shake(L, c->md, 0);
-                if (c->md.nmol > 0) {
-                    launch_md_velocity(L, c->md);
-                    if (nh) launch_md_nh(L, c->md);
-                }
-                launch_md_temperature(L, c->md, c->m.excl);
-                launch_md_record(L, c->md, c->e_all, c->efix_all, c->md_rec + (size_t)k * W * kMdRec);
+                c->launches += launch_md_move(L, c->md) + 1;
+                if (nh && c->md.nmol > 0) launch_md_nh(L, c->md);
+                launch_md_temperature(L, c->md, c->m.excl, c->e_all, c->efix_all, c->md_rec + (size_t)k * W * kMdRec);
             });
-            c->launches += 4 + (c->md.nmol > 0 ? 1 : 0) + (nh ? (c->md.nmol > 0 ? 4 : 2) : 0);
+            c->launches += nh ? (c->md.nmol > 0 ? 4 : 2) : 0;
             TRY(check_launch());
         }
         if (rec || EQ || Eb) {

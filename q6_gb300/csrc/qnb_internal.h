@@ -405,7 +405,7 @@ struct MdWin {                     // per window, device
     unsigned long long shake_iters;   // SHAKE iterations of the last step, summed over molecules
     double min_oldmax, min_scale, min_maxf;   // steepest descent: previous largest force, scale, largest force
     int min_state;                 // last minimisation step: 0 grown, 1 reset, 2 converged
-    int pad;
+    unsigned temp_blocks;          // temperature(): blocks of the window that stored their sums
 };
 struct MdDev {
     int natom, ntg, nmol;
@@ -434,6 +434,12 @@ struct MdDev {
     const double* dist2;           // [ncons] squared constraint distances
     uint8_t* ready;                // [nwin][ncons] SHAKE scratch
     int ncons;
+    // when every constrained molecule is a triangle (a, b), (a, c), (b, c) of
+    // atoms of its own: its atoms and first constraint, and the atoms outside
+    const int4* tri;               // [nmol] or null
+    const int* free_atoms;         // [nfree]
+    int nfree;
+    double* tpart;                 // [nwin][md_temp_part(natom)] temperature()'s block sums
     double* v;                     // [nwin][natom*3]
     double* xx;                    // [nwin][natom*3] positions before newvel
     MdWin* win;                    // [nwin]
@@ -442,6 +448,8 @@ struct MdDev {
 // a record of one window and step: FP64 energy slots, fixed-point slots, then
 // ekin, temp, tfree, SHAKE iterations
 constexpr int kMdRec = 2 * kNumE + 4;
+// newvel, SHAKE and (with constraints) v = (x - xx)/dt; returns the launches
+int launch_md_move(const Launch& L, const MdDev& md);
 void launch_md_newvel(const Launch& L, const MdDev& md);
 // nh_prop (chain update, one thread per window) and v *= s of every atom
 void launch_md_nh(const Launch& L, const MdDev& md);
@@ -451,11 +459,12 @@ void launch_md_put_back(const Launch& L, const MdDev& md);
 void launch_md_shake(const Launch& L, const MdDev& md, int mode);
 void launch_md_velocity(const Launch& L, const MdDev& md);
 void launch_md_copy_x(const Launch& L, const MdDev& md, int to_xx);   // xx = x (1) or the x - v dt of initial_constraint (2)
-void launch_md_temperature(const Launch& L, const MdDev& md, const uint8_t* excl);
+size_t md_temp_part(int natom);   // doubles of MdDev::tpart per window
+// with rec, the step's record of every window is written as well
+void launch_md_temperature(const Launch& L, const MdDev& md, const uint8_t* excl, const double* e_all = nullptr,
+                           const unsigned long long* efix_all = nullptr, double* rec = nullptr);
 void launch_md_stop_cm(const Launch& L, const MdDev& md);
 void launch_md_min_step(const Launch& L, const MdDev& md, double step0, double fcut, double max_move);
-void launch_md_record(const Launch& L, const MdDev& md, const double* e_all, const unsigned long long* efix_all,
-                      double* rec);
 void launch_md_clear_d(const Launch& L, const MdDev& md);   // d = 0, SHAKE count = 0
 
 // records msg as the calling thread's qnb_last_error text; returns code

@@ -673,12 +673,15 @@ int build_model(qnb_context* c, const qnb_topology* t) {
     TRY(c->upload(&c->d_heavy_solv, heavy_solv));
     // solvent atoms without LJ against every type (SPC hydrogens): their
     // solute pairs reduce to the Coulomb term exactly
-    m.wlj_mask = 0;
+    m.wlj_mask = m.wlj_mask_d = 0;
     if (t->nwat > 0)
         for (int a = 0; a < sa; ++a)
             for (int b = 0; b < nt; ++b) {
                 float4 p = ljpair[(size_t)b * nt + m.wtype[a]];
                 if (p.x != 0.f || p.y != 0.f) m.wlj_mask |= 1u << a;
+                const int code = t->ljcod[b * nt + m.wtype[a]];
+                double2 pd = lj[((size_t)(code - 1) * nt + b) * nt + m.wtype[a]];
+                if (pd.x != 0.0 || pd.y != 0.0) m.wlj_mask_d |= 1u << a;
             }
 
     // ---- Q atoms -------------------------------------------------------------
@@ -1342,7 +1345,7 @@ int compute_nonbond(qnb_context* c, int md, int nw, const SideWork& side = SideW
         if (mx) c->qenv_pending = true;   // the box Q terms store the environment atoms' gradients in fq
     } else {
         if (md && water) {
-            timed_on(c, b.ww.st, K_WW, [&] { rows ? launch_rows_water(b.ww) : launch_ww(b.ww, mx); });
+            timed_on(c, b.ww.st, K_WW, [&] { rows ? launch_rows_water(b.ww) : launch_ww(b.ww); });
             ++nl;
         }
         if (md) {
@@ -1350,8 +1353,8 @@ int compute_nonbond(qnb_context* c, int md, int nw, const SideWork& side = SideW
                 timed(c, K_PP, [&] { launch_rows_solute(L, c->maxg); });   // the class times the solute rows alone
                 c->rows_pending = true;   // frow holds this evaluation's row gradients
             } else {
-                if (water) timed(c, K_PW, [&] { launch_pw(L, mx); }), ++nl;
-                timed(c, K_PP, [&] { launch_pp(L, mx); });
+                if (water) timed(c, K_PW, [&] { launch_pw(L); }), ++nl;
+                timed(c, K_PP, [&] { launch_pp(L); });
             }
             ++nl;
         }

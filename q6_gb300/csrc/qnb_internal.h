@@ -105,7 +105,8 @@ struct DevModel {
     const uint8_t* ljcod;       // [natyps][natyps]
     const uint8_t* ljset;       // [3][natyps][natyps]: |A| or |B| > QREAL_EPS
     int wtype[kMaxSolv];        // solvent template (first molecule) atom types
-    unsigned wlj_mask;          // bit a: template atom a has LJ parameters with some solute type
+    unsigned wlj_mask;          // bit a: template atom a has LJ parameters (in FP32) with some solute type
+    unsigned wlj_mask_d;        // the same in FP64
     double wcrg[kMaxSolv];      // and charges
     float wcrgf[kMaxSolv];
     double wwA[kMaxSolv * kMaxSolv], wwB[kMaxSolv * kMaxSolv], wwE[kMaxSolv * kMaxSolv];  // ww_precomp
@@ -285,10 +286,10 @@ int box_cells(const DevModel& m, const Cut& c, int* n);
 void launch_build_box_pairs(const Launch& L, const Cut& c);
 void launch_rows_solute(const Launch& L, int maxg);
 void launch_rows_water(const Launch& L);
-void launch_ww(const Launch& L, int mixed);
+void launch_ww(const Launch& L);   // FP64 form
 void launch_qw(const Launch& L, int mixed);
-void launch_pw(const Launch& L, int mixed);
-void launch_pp(const Launch& L, int mixed);
+void launch_pw(const Launch& L);   // FP64 form
+void launch_pp(const Launch& L);   // FP64 form
 void launch_qp(const Launch& L, int mixed);
 void launch_nonbond_qq(const Launch& L, int mixed);
 void launch_lrf_taylor(const Launch& L, const int* iwhich, int mixed);

@@ -1378,18 +1378,25 @@ __global__ void __launch_bounds__(128) k_lrf_accumulate_any_box(DevModel m, cons
 // =============================================================================
 
 
-// one plain pair (nbe, src/nonbonded.f90:45-75); returns dv, vec via refs
+// one plain pair (nbe, src/nonbonded.f90:45-75); returns dv, vec via refs.
+// 1/distance comes from one rsqrt and its square is 1/distance^2: the FP64
+// form's kernels are bound by the FP64 pipe (84 % busy at two lanes per clock
+// and SM), where the reference's division and square root of the quotient
+// were 15 of a pair's 37 operations (16 windows of the 25 A sphere: pp 774 ->
+// 661 us, ww 269 -> 185, pw 212 -> 165).  Both orders are within a few ulp.
 struct PairD {
     double tx, ty, tz, dv, vel, vdw;
 };
-__device__ __forceinline__ PairD nbe_d(const double* x, int i, int j, double A, double B, double el,
+__device__ __forceinline__ void load_x(const double* __restrict__ x, int i, double (&r)[3]) {
+    r[0] = x[3 * i], r[1] = x[3 * i + 1], r[2] = x[3 * i + 2];
+}
+__device__ __forceinline__ PairD nbe_d(const double (&xi)[3], const double (&xj)[3], double A, double B, double el,
                                        bool lj) {
     PairD p;
-    p.tx = x[3 * j] - x[3 * i];
-    p.ty = x[3 * j + 1] - x[3 * i + 1];
-    p.tz = x[3 * j + 2] - x[3 * i + 2];
-    double r2 = 1.0 / (p.tx * p.tx + p.ty * p.ty + p.tz * p.tz);
-    double r = sqrt(r2);
+    p.tx = xj[0] - xi[0];
+    p.ty = xj[1] - xi[1];
+    p.tz = xj[2] - xi[2];
+    const double r = rsqrt(p.tx * p.tx + p.ty * p.ty + p.tz * p.tz), r2 = r * r;
     p.vel = el * r;
     if (lj) {
         double r6 = r2 * r2 * r2;
@@ -1427,134 +1434,114 @@ __device__ __forceinline__ PairF nbe_f(float4 a, float4 b, float A, float B, flo
     return p;
 }
 
-// nonbond_ww_spc / nonbond_ww, src/nonbondene.f90:5886-5975, 5509-5573
-template <bool MIX, bool SPC>
-__global__ void __launch_bounds__(256) k_ww(DevModel m, const DevState* __restrict__ states) {
+// -v by its sign bit: a negation that the compiler cannot fold into an operand
+// (the operand of an atomic) would be an operation of the FP64 pipe
+__device__ __forceinline__ double neg_bits(double v) {
+    return __longlong_as_double(__double_as_longlong(v) ^ (long long)0x8000000000000000ull);
+}
+__device__ __forceinline__ void grad_neg(const Acc<false>& acc, int i, double gx, double gy, double gz) {
+    acc.grad(i, neg_bits(gx), neg_bits(gy), neg_bits(gz));
+}
+
+// ---- FP64 form: half lists, FP64 atomics ------------------------------------
+// nonbond_ww_spc / nonbond_ww, src/nonbondene.f90:5886-5975, 5509-5573.  NS:
+// atoms per molecule known at compile time (3, positions and gradients of
+// both molecules in registers), or 0.
+template <bool SPC, int NS>
+__global__ void __launch_bounds__(128) k_ww(DevModel m, const DevState* __restrict__ states) {
     const DevState& s = states[blockIdx.y];
-    Acc<MIX> acc = make_acc<MIX>(s);
-    ESum<MIX> eel, evdw;
-    int n = min((int64_t)s.cnt[C_WW], s.cap_ww);
-    int sa = m.sa;
+    Acc<false> acc = make_acc<false>(s);
+    ESum<false> eel, evdw;
+    const int n = min((int64_t)s.cnt[C_WW], s.cap_ww), sa = NS ? NS : m.sa;
+    constexpr int N = NS ? NS : kMaxSolv;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        int2 e = s.ww[p];
-        int i0 = m.nat_solute + sa * e.x, j0 = m.nat_solute + sa * e.y;
-        if constexpr (!MIX) {
-            double gi[kMaxSolv][3] = {}, gj[kMaxSolv][3] = {};
-            for (int la = 0; la < sa; ++la)
-                for (int ka = 0; ka < sa; ++ka) {
-                    bool lj = !SPC || (la == 0 && ka == 0);
-                    int k = la * kMaxSolv + ka;
-                    PairD q = nbe_d(s.x, i0 + la, j0 + ka, m.wwA[k], m.wwB[k], m.wwE[k], lj);
-                    gi[la][0] -= q.tx * q.dv; gi[la][1] -= q.ty * q.dv; gi[la][2] -= q.tz * q.dv;
-                    gj[ka][0] += q.tx * q.dv; gj[ka][1] += q.ty * q.dv; gj[ka][2] += q.tz * q.dv;
-                    eel.add(q.vel);
-                    evdw.add(q.vdw);
-                }
-            for (int a = 0; a < sa; ++a) {
-                acc.grad(i0 + a, gi[a][0], gi[a][1], gi[a][2]);
-                acc.grad(j0 + a, gj[a][0], gj[a][1], gj[a][2]);
+        const int2 e = s.ww[p];
+        const int i0 = m.nat_solute + sa * e.x, j0 = m.nat_solute + sa * e.y;
+        double gj[N][3] = {}, xj[N][3];
+#pragma unroll
+        for (int b = 0; b < N; ++b)
+            if (b < sa) load_x(s.x, j0 + b, xj[b]);
+#pragma unroll
+        for (int la = 0; la < N; ++la) {
+            if (la >= sa) break;
+            double xi[3], gx = 0.0, gy = 0.0, gz = 0.0;
+            load_x(s.x, i0 + la, xi);
+#pragma unroll
+            for (int ka = 0; ka < N; ++ka) {
+                if (ka >= sa) break;
+                const bool lj = !SPC || (la == 0 && ka == 0);
+                const int k = la * kMaxSolv + ka;
+                const PairD q = nbe_d(xi, xj[ka], m.wwA[k], m.wwB[k], m.wwE[k], lj);
+                gx += q.tx * q.dv; gy += q.ty * q.dv; gz += q.tz * q.dv;
+                gj[ka][0] += q.tx * q.dv; gj[ka][1] += q.ty * q.dv; gj[ka][2] += q.tz * q.dv;
+                eel.add(q.vel);
+                if (lj) evdw.add(q.vdw);
             }
-        } else {
-            float gi[kMaxSolv][3] = {}, gj[kMaxSolv][3] = {};
-            float4 xi[kMaxSolv], xj[kMaxSolv];
-            for (int a = 0; a < sa; ++a) { xi[a] = s.xq[i0 + a]; xj[a] = s.xq[j0 + a]; }
-            for (int la = 0; la < sa; ++la)
-                for (int ka = 0; ka < sa; ++ka) {
-                    bool lj = !SPC || (la == 0 && ka == 0);
-                    int k = la * kMaxSolv + ka;
-                    PairF q = nbe_f(xi[la], xj[ka], m.wwAf[k], m.wwBf[k], m.wwEf[k], lj);
-                    gi[la][0] -= q.tx * q.dv; gi[la][1] -= q.ty * q.dv; gi[la][2] -= q.tz * q.dv;
-                    gj[ka][0] += q.tx * q.dv; gj[ka][1] += q.ty * q.dv; gj[ka][2] += q.tz * q.dv;
-                    eel.add(q.vel);
-                    evdw.add(q.vdw);
-                }
-            for (int a = 0; a < sa; ++a) {
-                acc.grad(i0 + a, gi[a][0], gi[a][1], gi[a][2]);
-                acc.grad(j0 + a, gj[a][0], gj[a][1], gj[a][2]);
-            }
+            grad_neg(acc, i0 + la, gx, gy, gz);
         }
+#pragma unroll
+        for (int b = 0; b < N; ++b)
+            if (b < sa) acc.grad(j0 + b, gj[b][0], gj[b][1], gj[b][2]);
     }
     eel.flush(acc, E_WW_EL);
     evdw.flush(acc, E_WW_VDW);
 }
 
-// nonbond_pw, src/nonbondene.f90:4856-4916 (pw_precomp, src/simprep.f90:3354-3386)
-template <bool MIX>
-__global__ void __launch_bounds__(256) k_pw(DevModel m, const DevState* __restrict__ states) {
+// nonbond_pw, src/nonbondene.f90:4856-4916 (pw_precomp, src/simprep.f90:3354-3386).
+// A solvent atom without LJ parameters against any solute type (wlj_mask_d;
+// the H of SPC) takes the Coulomb term alone: A = B = 0 add nothing.
+__global__ void __launch_bounds__(128) k_pw(DevModel m, const DevState* __restrict__ states) {
     const DevState& s = states[blockIdx.y];
-    Acc<MIX> acc = make_acc<MIX>(s);
-    ESum<MIX> eel, evdw;
-    int n = min((int64_t)s.cnt[C_PW], s.cap_pw);
-    int sa = m.sa;
+    Acc<false> acc = make_acc<false>(s);
+    ESum<false> eel, evdw;
+    const int n = min((int64_t)s.cnt[C_PW], s.cap_pw), sa = m.sa;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        int2 e = s.pw[p];
-        int i = e.x, j0 = m.nat_solute + sa * e.y;
-        int ti = m.iac[i];
-        if constexpr (!MIX) {
-            double g[3] = {0, 0, 0};
-            for (int a = 0; a < sa; ++a) {
-                int tw = m.wtype[a];
-                int code = m.ljcod[ti * m.natyps + tw];
-                double2 ab = m.lj[((code - 1) * m.natyps + ti) * m.natyps + tw];
-                PairD q = nbe_d(s.x, i, j0 + a, ab.x, ab.y, m.crg[i] * m.wcrg[a], true);
-                g[0] -= q.tx * q.dv; g[1] -= q.ty * q.dv; g[2] -= q.tz * q.dv;
-                acc.grad(j0 + a, q.tx * q.dv, q.ty * q.dv, q.tz * q.dv);
-                eel.add(q.vel);
-                evdw.add(q.vdw);
+        const int2 e = s.pw[p];
+        const int i = e.x, j0 = m.nat_solute + sa * e.y, ti = m.iac[i];
+        const double qi = m.crg[i];
+        double xi[3], xj[3], gx = 0.0, gy = 0.0, gz = 0.0;
+        load_x(s.x, i, xi);
+        for (int a = 0; a < sa; ++a) {
+            const bool lj = (m.wlj_mask_d >> a) & 1u;
+            double2 ab = make_double2(0.0, 0.0);
+            if (lj) {
+                const int tw = m.wtype[a], code = m.ljcod[ti * m.natyps + tw];
+                ab = m.lj[((code - 1) * m.natyps + ti) * m.natyps + tw];
             }
-            acc.grad(i, g[0], g[1], g[2]);
-        } else {
-            float g[3] = {0, 0, 0};
-            float4 xi = s.xq[i];
-            for (int a = 0; a < sa; ++a) {
-                int tw = m.wtype[a];
-                int code = m.ljcod[ti * m.natyps + tw];
-                float2 ab = m.ljf[((code - 1) * m.natyps + ti) * m.natyps + tw];
-                PairF q = nbe_f(xi, s.xq[j0 + a], ab.x, ab.y, xi.w * m.wcrgf[a], true);
-                g[0] -= q.tx * q.dv; g[1] -= q.ty * q.dv; g[2] -= q.tz * q.dv;
-                acc.grad(j0 + a, q.tx * q.dv, q.ty * q.dv, q.tz * q.dv);
-                eel.add(q.vel);
-                evdw.add(q.vdw);
-            }
-            acc.grad(i, g[0], g[1], g[2]);
+            load_x(s.x, j0 + a, xj);
+            const PairD q = nbe_d(xi, xj, ab.x, ab.y, qi * m.wcrg[a], lj);
+            const double fx = q.tx * q.dv, fy = q.ty * q.dv, fz = q.tz * q.dv;
+            gx += fx; gy += fy; gz += fz;
+            acc.grad(j0 + a, fx, fy, fz);
+            eel.add(q.vel);
+            if (lj) evdw.add(q.vdw);
         }
+        grad_neg(acc, i, gx, gy, gz);
     }
     eel.flush(acc, E_PW_EL);
     evdw.flush(acc, E_PW_VDW);
 }
 
 // nonbond_pp, src/nonbondene.f90:4694-4760 (pp_precomp values)
-template <bool MIX>
-__global__ void __launch_bounds__(256) k_pp(DevModel m, const DevState* __restrict__ states) {
+__global__ void __launch_bounds__(128) k_pp(DevModel m, const DevState* __restrict__ states) {
     const DevState& s = states[blockIdx.y];
-    Acc<MIX> acc = make_acc<MIX>(s);
-    ESum<MIX> eel, evdw;
-    int n = min((int64_t)s.cnt[C_PP], s.cap_pp);
+    Acc<false> acc = make_acc<false>(s);
+    ESum<false> eel, evdw;
+    const int n = min((int64_t)s.cnt[C_PP], s.cap_pp);
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        int2 e = s.pp[p];
-        int i = e.x, j = e.y & 0x0fffffff, code = e.y >> 28;
-        int ti = m.iac[i], tj = m.iac[j];
-        size_t t = ((size_t)(code - 1) * m.natyps + ti) * m.natyps + tj;
-        if constexpr (!MIX) {
-            double2 ab = m.lj[t];
-            double el = m.crg[i] * m.crg[j];
-            if (code == 3) el = el * m.el14;
-            PairD q = nbe_d(s.x, i, j, ab.x, ab.y, el, true);
-            acc.grad(i, -q.tx * q.dv, -q.ty * q.dv, -q.tz * q.dv);
-            acc.grad(j, q.tx * q.dv, q.ty * q.dv, q.tz * q.dv);
-            eel.add(q.vel);
-            evdw.add(q.vdw);
-        } else {
-            float2 ab = m.ljf[t];
-            float4 xi = s.xq[i], xj = s.xq[j];
-            float el = xi.w * xj.w;
-            if (code == 3) el *= m.el14f;
-            PairF q = nbe_f(xi, xj, ab.x, ab.y, el, true);
-            acc.grad(i, -q.tx * q.dv, -q.ty * q.dv, -q.tz * q.dv);
-            acc.grad(j, q.tx * q.dv, q.ty * q.dv, q.tz * q.dv);
-            eel.add(q.vel);
-            evdw.add(q.vdw);
-        }
+        const int2 e = s.pp[p];
+        const int i = e.x, j = e.y & 0x0fffffff, code = e.y >> 28;
+        const double2 ab = m.lj[((size_t)(code - 1) * m.natyps + m.iac[i]) * m.natyps + m.iac[j]];
+        double el = m.crg[i] * m.crg[j], xi[3], xj[3];
+        if (code == 3) el = el * m.el14;
+        load_x(s.x, i, xi);
+        load_x(s.x, j, xj);
+        const PairD q = nbe_d(xi, xj, ab.x, ab.y, el, true);
+        const double fx = q.tx * q.dv, fy = q.ty * q.dv, fz = q.tz * q.dv;
+        grad_neg(acc, i, fx, fy, fz);
+        acc.grad(j, fx, fy, fz);
+        eel.add(q.vel);
+        evdw.add(q.vdw);
     }
     eel.flush(acc, E_PP_EL);
     evdw.flush(acc, E_PP_VDW);
@@ -4044,12 +4031,15 @@ void launch_rows_water(const Launch& L) {
     } else if (spc) k_rows_water<true, false><<<g, 128, sm, L.st>>>(L.m, L.ds);
     else k_rows_water<false, false><<<g, 128, sm, L.st>>>(L.m, L.ds);
 }
-void launch_ww(const Launch& L, int mixed) {
+void launch_ww(const Launch& L) {
     if (L.m.nwat == 0) return;
-    dim3 g = grid_for(L.s0.cap_ww, 256, 8, L.nwin);
-    bool spc = L.m.spc != 0;
-    if (mixed) { if (spc) k_ww<true, true><<<g, 256, 0, L.st>>>(L.m, L.ds); else k_ww<true, false><<<g, 256, 0, L.st>>>(L.m, L.ds); }
-    else { if (spc) k_ww<false, true><<<g, 256, 0, L.st>>>(L.m, L.ds); else k_ww<false, false><<<g, 256, 0, L.st>>>(L.m, L.ds); }
+    dim3 g = grid_for(L.s0.cap_ww, 128, 16, L.nwin);
+    const bool three = L.m.sa == 3;
+    if (L.m.spc) {
+        if (three) k_ww<true, 3><<<g, 128, 0, L.st>>>(L.m, L.ds);
+        else k_ww<true, 0><<<g, 128, 0, L.st>>>(L.m, L.ds);
+    } else if (three) k_ww<false, 3><<<g, 128, 0, L.st>>>(L.m, L.ds);
+    else k_ww<false, 0><<<g, 128, 0, L.st>>>(L.m, L.ds);
 }
 #ifndef QNB_Q_LANES
 #define QNB_Q_LANES 1   // mixed form: k_qenv_lanes (1) or k_qenv (0)
@@ -4077,15 +4067,13 @@ void launch_qw(const Launch& L, int mixed) {
     if (L.m.nwat == 0 || L.m.nqat == 0) return;
     launch_qenv<true>(L, mixed, grid_for(L.s0.cap_qw * 32, kQBlock, L.tu.v[T_QW], L.nwin));
 }
-void launch_pw(const Launch& L, int mixed) {
+void launch_pw(const Launch& L) {
     if (L.m.nwat == 0 || L.m.ncgp_solute == 0) return;
-    dim3 g = grid_for(L.s0.cap_pw, 256, 8, L.nwin);
-    if (mixed) k_pw<true><<<g, 256, 0, L.st>>>(L.m, L.ds); else k_pw<false><<<g, 256, 0, L.st>>>(L.m, L.ds);
+    k_pw<<<grid_for(L.s0.cap_pw, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds);
 }
-void launch_pp(const Launch& L, int mixed) {
+void launch_pp(const Launch& L) {
     if (L.m.ncgp_solute == 0) return;
-    dim3 g = grid_for(L.s0.cap_pp, 256, 8, L.nwin);
-    if (mixed) k_pp<true><<<g, 256, 0, L.st>>>(L.m, L.ds); else k_pp<false><<<g, 256, 0, L.st>>>(L.m, L.ds);
+    k_pp<<<grid_for(L.s0.cap_pp, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds);
 }
 void launch_qp(const Launch& L, int mixed) {
     if (L.m.nqat == 0 || L.m.nat_solute == 0) return;

@@ -304,10 +304,8 @@ int qnb_set_solvent_internal(qnb_context* ctx, int32_t n, const int32_t* ij, con
    (the evaluation's parallel branches off, so each class runs alone), the
    candidate blocks-per-SM of each per-step kernel class and of the list
    build, one parameter at a time, and keeps the fastest.  Results are
-   independent of these choices.  The Q chunk (units per fixed-point
-   conversion of the Q energies, default 8) is kept: it sets the grouping of
-   FP32 partial sums, so changing it with qnb_set_tuning changes the Q
-   energies at the FP32 rounding level (deterministically).  Needs built lists;
+   independent of these choices.  The Q chunk is kept: it set the grouping of
+   partial sums in earlier Q kernels and no kernel reads it.  Needs built lists;
    restores the watpol running averages and clears the gradient
    accumulators.  values (may be NULL) receives the QNB_TUNE_COUNT choices:
    solute rows, water rows, qp, qw (blocks per SM), Q chunk (units), LRF

@@ -252,7 +252,8 @@ inline Cut make_cut(double rcq2, double rlrf2, double rcpp2, double rcpw2, doubl
 // window 0's host-side state (capacities are equal across windows) and ds the
 // device array of all windows' states.
 // Launch geometry chosen by the autotuner (qnb_autotune): blocks per SM of
-// the per-step kernels and of the list build, and the Q-kernel chunk size
+// the per-step kernels and of the list build (T_QCHUNK and T_LRF: ABI slots no
+// kernel reads)
 enum TuneParam { T_ROWS_SOLUTE, T_ROWS_WATER, T_QP, T_QW, T_QCHUNK, T_TAYLOR, T_LRF, T_BUILD, T_NUM };
 struct Tune {
     int v[T_NUM];

@@ -1548,15 +1548,6 @@ __global__ void __launch_bounds__(128) k_pp(DevModel m, const DevState* __restri
 }
 
 // nbe_qx soft-core pair for one state, src/nonbonded.f90:200-222
-__device__ __forceinline__ void nbe_qx_d(double r2, double r, double r6_hc, double A, double B, double el,
-                                         double sc, double lam, double& vel, double& vdw, double& dv) {
-    double r6 = 1.0 / (r6_hc + sc);
-    double r12 = r6 * r6;
-    vel = el * r;
-    double va = A * r12, vb = B * r6;
-    vdw = va - vb;
-    dv = r2 * (-vel - (12.0 * va - 6.0 * vb) * r6 * r6_hc) * lam;
-}
 __device__ __forceinline__ void nbe_qx_f(float r2, float r, float r6_hc, float A, float B, float el, float sc,
                                          float lam, float& vel, float& vdw, float& dv) {
     float r6 = __fdividef(1.0f, r6_hc + sc);
@@ -1570,71 +1561,11 @@ __device__ __forceinline__ void nbe_qx_f(float r2, float r, float r6_hc, float A
 constexpr int kMaxQ = 64;
 constexpr int kQBlock = 256;   // threads per block of the Q kernels
 
-// Q-atom gradients: every lane keeps its Q atoms' sums in registers; at the
-// end the warps of a block combine them in shared memory and the block adds
-// them once (fixed point in the mixed form).
-template <bool MIX>
-__device__ __forceinline__ void flush_q_grad(const DevModel& m, const DevState& s,
-                                             const unsigned long long (&gqx)[2][3], const double (&gqd)[2][3]) {
-    typedef typename std::conditional<MIX, unsigned long long, double>::type GT;
-    __shared__ GT red[3 * kMaxQ];
-    for (int k = threadIdx.x; k < 3 * m.nqat; k += blockDim.x) red[k] = GT(0);
-    __syncthreads();
-    int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < kMaxQ / 32; ++k) {
-        int iq = k * 32 + lane;
-        if (iq >= m.nqat) break;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            if constexpr (MIX) atomicAdd(&red[3 * iq + c], gqx[k][c]);
-            else atomicAdd(&red[3 * iq + c], gqd[k][c]);
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < 3 * m.nqat; k += blockDim.x) {
-        int i = m.iqseq[k / 3];
-        if constexpr (MIX) atomicAdd(s.fix + 3 * i + k % 3, (unsigned long long)red[k]);
-        else atomicAdd(s.d + 3 * i + k % 3, (double)red[k]);
-    }
-}
-
 // Per-lane Q-atom x environment-atom interaction for all states (soft-core
 // LJ + Coulomb when lj, Coulomb only otherwise): returns the lambda-weighted
 // dv sum over states and adds the per-state energies to pel/pvdw.
-template <bool MIX, int SMAX>
-struct QPairT;
 template <int SMAX>
-struct QPairT<false, SMAX> {
-    __device__ __forceinline__ static double run(const QPar* P, const double* lam, int S, bool lj, double r2, double r,
-                                                 double* pel, double* pvdw) {
-        double dvs = 0.0;
-        if (lj) {
-            double r6hc = 1.0 / (r2 * r2 * r2);
-#pragma unroll
-            for (int st = 0; st < SMAX; ++st) {
-                if (st >= S) break;
-                QPar q = P[st];
-                double vel, vdw, dv;
-                nbe_qx_d(r2, r, r6hc, q.A, q.B, q.el, q.sc, lam[st], vel, vdw, dv);
-                dvs += dv;
-                pel[st] += vel;
-                pvdw[st] += vdw;
-            }
-        } else {   // nbe_qspc, src/nonbonded.f90:226-243
-#pragma unroll
-            for (int st = 0; st < SMAX; ++st) {
-                if (st >= S) break;
-                double vel = P[st].el * r;
-                dvs += -r2 * vel * lam[st];
-                pel[st] += vel;
-            }
-        }
-        return dvs;
-    }
-};
-template <int SMAX>
-struct QPairT<true, SMAX> {
+struct QPairF {
     __device__ __forceinline__ static float run(const QParF* P, const float* lam, int S, bool lj, float r2, float r,
                                                 float* pel, float* pvdw) {
         float dvs = 0.0f;
@@ -1662,124 +1593,6 @@ struct QPairT<true, SMAX> {
         return dvs;
     }
 };
-
-// nonbond_qw_spc / nonbond_qw (src/nonbondene.f90:5658-5767, 5339-5418) and
-// nonbond_qp (src/nonbondene.f90:5157-5230): one warp per listed environment
-// unit (a water molecule, or one solute atom), lane = Q atom.  A warp takes
-// fixed chunks of qchunk consecutive units (autotuned); the per-state energies of a
-// chunk are summed in registers and converted once per chunk, so the fixed-
-// point totals do not depend on the grid.  An environment atom's gradient is
-// summed over the Q atoms in FP32 in a fixed shuffle order, then converted.
-
-template <bool MIX, bool SPC, bool WATER, int SMAX>
-__global__ void __launch_bounds__(kQBlock, 3) k_qenv(DevModel m, const DevState* __restrict__ states, int qchunk) {
-    typedef typename std::conditional<MIX, float, double>::type T;
-    const DevState& s = states[blockIdx.y];
-    Acc<MIX> acc = make_acc<MIX>(s);
-    ESum<MIX> eel[SMAX], evdw[SMAX];
-    float gqf[2][3] = {};              // this chunk's Q-atom gradient (mixed form)
-    unsigned long long gqx[2][3] = {}; // converted once per chunk: the sum over chunks is exact
-    double gqd[2][3] = {};
-    T lam[SMAX];
-#pragma unroll
-    for (int st = 0; st < SMAX; ++st) lam[st] = st < m.S ? (T)s.lambda[st] : T(0);
-    int lane = threadIdx.x & 31;
-    int n = WATER ? min((int64_t)s.cnt[C_QW], s.cap_qw) : min((int64_t)s.cnt[C_QP], s.cap_qp);
-    int S = m.S;
-    const int na = WATER ? m.sa : 1;
-    const int nchunk = (n + qchunk - 1) / qchunk;
-    for (int ch = warp_id_global(); ch < nchunk; ch += warps_total()) {
-      T pel[SMAX], pvdw[SMAX];
-#pragma unroll
-      for (int st = 0; st < SMAX; ++st) pel[st] = pvdw[st] = T(0);
-      const int pend = min(n, (ch + 1) * qchunk);
-      for (int p = ch * qchunk; p < pend; ++p) {
-        int j0 = WATER ? m.nat_solute + m.sa * s.qw[p] : s.qp[p];
-        for (int a = 0; a < na; ++a) {
-            int j = j0 + a;
-            bool lj = !WATER || !SPC || a == 0;
-            T gj[3] = {T(0), T(0), T(0)};
-#pragma unroll
-            for (int k = 0; k < kMaxQ / 32; ++k) {
-                int iq = k * 32 + lane;
-                if (iq >= m.nqat) break;
-                int i = m.iqseq[iq];
-                T tx, ty, tz, r2, r;
-                if constexpr (MIX) {
-                    float4 xi = s.xq[i], xj = s.xq[j];
-                    tx = xj.x - xi.x;
-                    ty = xj.y - xi.y;
-                    tz = xj.z - xi.z;
-                    r = rsqrtf(tx * tx + ty * ty + tz * tz);
-                    r2 = r * r;
-                } else {
-                    tx = s.x[3 * j] - s.x[3 * i];
-                    ty = s.x[3 * j + 1] - s.x[3 * i + 1];
-                    tz = s.x[3 * j + 2] - s.x[3 * i + 2];
-                    r2 = 1.0 / (tx * tx + ty * ty + tz * tz);
-                    r = sqrt(r2);
-                }
-                T dvs;
-                if constexpr (MIX) {
-                    const QParF* P = WATER ? m.qw_tabf + (iq * m.sa + a) * S : m.qp_tabf + ((size_t)j * m.nqat + iq) * S;
-                    dvs = QPairT<true, SMAX>::run(P, lam, S, lj, r2, r, pel, pvdw);
-                    gqf[k][0] -= tx * dvs; gqf[k][1] -= ty * dvs; gqf[k][2] -= tz * dvs;
-                } else {
-                    const QPar* P = WATER ? m.qw_tab + (iq * m.sa + a) * S : m.qp_tab + ((size_t)j * m.nqat + iq) * S;
-                    dvs = QPairT<false, SMAX>::run(P, lam, S, lj, r2, r, pel, pvdw);
-                    gqd[k][0] -= tx * dvs; gqd[k][1] -= ty * dvs; gqd[k][2] -= tz * dvs;
-                }
-                gj[0] += tx * dvs;
-                gj[1] += ty * dvs;
-                gj[2] += tz * dvs;
-            }
-            // environment atom gradient: sum over the warp's Q atoms.  Each
-            // atom is in one unit of the list, so the mixed form stores its
-            // FP32 sum (k_apply_fixed adds it) instead of a converted atomic
-            T v0 = warp_sum(gj[0]), v1 = warp_sum(gj[1]), v2 = warp_sum(gj[2]);
-            if (lane == 0) {
-                if constexpr (MIX) {
-                    s.fq[3 * j] = v0;
-                    s.fq[3 * j + 1] = v1;
-                    s.fq[3 * j + 2] = v2;
-                } else {
-                    acc.grad(j, v0, v1, v2);
-                }
-            }
-        }
-      }
-#pragma unroll
-      for (int st = 0; st < SMAX; ++st) {
-          if (st >= S) break;
-          if constexpr (MIX) {
-              eel[st].add_alu(pel[st]);
-              evdw[st].add_alu(pvdw[st]);
-          } else {
-              eel[st].add(pel[st]);
-              evdw[st].add(pvdw[st]);
-          }
-      }
-      if constexpr (MIX) {
-#pragma unroll
-          for (int k = 0; k < kMaxQ / 32; ++k) {
-              if (k * 32 >= m.nqat) break;   // warp-uniform
-#pragma unroll
-              for (int c = 0; c < 3; ++c) {
-                  gqx[k][c] += to_fix_alu(gqf[k][c]);
-                  gqf[k][c] = 0.f;
-              }
-          }
-      }
-    }
-    const int kel = WATER ? 4 : 2;
-#pragma unroll
-    for (int st = 0; st < SMAX; ++st) {
-        if (st >= S) break;
-        eel[st].flush(acc, eq_slot(st, kel));
-        evdw[st].flush(acc, eq_slot(st, kel + 1));
-    }
-    flush_q_grad<MIX>(m, s, gqx, gqd);
-}
 
 // ---------------------------------------------------------------------------
 // Adjoint of the Q-atom energies with respect to the Q parameters: for every
@@ -1817,8 +1630,8 @@ __device__ __forceinline__ float3 box_shift_f(const DevModel& m, float4 a, float
 // do.  Each sum pairs the lanes as warp_sum does (lane i with i + 16, then
 // with i + 8, ...), so it is the same FP32 value warp_sum gives, for N - 1
 // shuffles and additions instead of 5 N.
-template <int N>
-__device__ __forceinline__ float reduce_scatter(float (&g)[N], int lane) {
+template <int N, typename T>
+__device__ __forceinline__ T reduce_scatter(T (&g)[N], int lane) {
     static_assert(N == 16 || N == 32, "16 or 32 values");
     int o = 16;
 #pragma unroll
@@ -1826,12 +1639,12 @@ __device__ __forceinline__ float reduce_scatter(float (&g)[N], int lane) {
         const bool up = lane & o;
 #pragma unroll
         for (int i = 0; i < len / 2; ++i) {
-            const float keep = up ? g[i + len / 2] : g[i];
-            const float send = up ? g[i] : g[i + len / 2];
+            const T keep = up ? g[i + len / 2] : g[i];
+            const T send = up ? g[i] : g[i + len / 2];
             g[i] = keep + __shfl_xor_sync(kFull, send, o);
         }
     }
-    float v = g[0];
+    T v = g[0];
 #pragma unroll
     for (; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
     return v;
@@ -1923,7 +1736,7 @@ __global__ void __launch_bounds__(kQBlock) k_qenv_lanes(DevModel m, const DevSta
                         float r = rsqrtf(tx * tx + ty * ty + tz * tz), r2 = r * r;
                         const QParF* P = WATER ? m.qw_tabf + (iq * m.sa + a) * S
                                                : m.qp_tabft + ((size_t)iq * m.nat_solute + j0) * S;
-                        float dvs = QPairT<true, SMAX>::run(P, lam, S, lj, r2, r, pel, pvdw);
+                        float dvs = QPairF<SMAX>::run(P, lam, S, lj, r2, r, pel, pvdw);
                         gx -= tx * dvs; gy -= ty * dvs; gz -= tz * dvs;
                         gj[a][0] += tx * dvs; gj[a][1] += ty * dvs; gj[a][2] += tz * dvs;
                     }
@@ -1963,6 +1776,132 @@ __global__ void __launch_bounds__(kQBlock) k_qenv_lanes(DevModel m, const DevSta
     for (int k = threadIdx.x; k < 3 * nq; k += blockDim.x) {
         unsigned long long v = red[k];
         if (v) atomicAdd(s.fix + 3 * m.iqseq[k / 3] + k % 3, v);
+    }
+}
+
+// FP64 form of the Q-environment terms: nonbond_qw_spc / nonbond_qw
+// (src/nonbondene.f90:5658-5767, 5339-5418), nonbond_qp (5157-5230) and their
+// box forms (see k_qenv_lanes).  A warp takes 32 consecutive units (lane =
+// water or solute atom) against kQRed Q atoms: the environment atoms'
+// gradients stay in the lane, the Q atoms' are summed over the warp in one
+// transposed butterfly, both are added with FP64 atomics.  The FP64 pipe bounds
+// it: r^6 is d2^3 instead of 1/(1/d2)^3, 1/distance one rsqrt, and states whose
+// soft-core alpha equals the state before's (compared bit for bit) share the
+// division.  Splitting the Q atoms over warps as well spreads a single window
+// over the device (with lane = Q atom and eight units per warp, 6 Q atoms kept
+// 6 of 32 lanes busy on 56 warps: 118 us for 446 waters; 20 Q atoms and 16
+// windows of 1,020 waters 339 us, of 2,955 solute atoms 285 us; now 32, 109
+// and 137 us).
+template <bool SPC, bool WATER, int NA, int SMAX, bool BOX>
+__global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __restrict__ states,
+                                                const int* __restrict__ iwhich, double rcq2) {
+    const DevState& s = states[blockIdx.y];
+    const double* __restrict__ x = s.x;
+    Acc<false> acc = make_acc<false>(s);
+    const int lane = threadIdx.x & 31, S = m.S, nq = m.nqat, na = WATER ? m.sa : 1;
+    const int n = WATER ? min((int64_t)s.cnt[C_QW], s.cap_qw) : min((int64_t)s.cnt[C_QP], s.cap_qp);
+    const int nqb = (nq + kQRed - 1) / kQRed, items = (n + kWarp - 1) / kWarp * nqb;
+    ESum<false> eel[SMAX], evdw[SMAX];
+    for (int it = warp_id_global(); it < items; it += warps_total()) {
+        const int p = it / nqb * kWarp + lane, q0 = it % nqb * kQRed;
+        const bool act = p < n;
+        const int j0 = act ? (WATER ? m.nat_solute + m.sa * s.qw[p] : s.qp[p]) : 0;
+        double xj[NA][3], gj[NA][3];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            gj[a][0] = gj[a][1] = gj[a][2] = xj[a][0] = xj[a][1] = xj[a][2] = 0.0;
+            if (act && a < na) load_x(x, j0 + a, xj[a]);
+        }
+        double sh[3] = {0.0, 0.0, 0.0};   // the unit's lattice shift (BOX)
+        if (BOX && act) {
+            int ref = j0;
+            if (!WATER) {
+                const int g = iwhich[j0];
+                ref = m.gatom[m.gslot[g]];
+                for (int a = m.gslot[g]; a < m.gslot[g + 1]; ++a)
+                    if (box_d2(m, x, m.gatom[a], m.qswitch) <= rcq2) {
+                        ref = m.gatom[a];
+                        break;
+                    }
+            }
+            box_shift(m, x, m.qswitch, ref, sh[0], sh[1], sh[2]);
+        }
+        double g[16];
+#pragma unroll
+        for (int v = 0; v < 16; ++v) g[v] = 0.0;
+#pragma unroll
+        for (int b = 0; b < kQRed; ++b) {
+            const int iq = q0 + b;
+            if (iq >= nq) break;   // warp-uniform
+            double xi[3], gx = 0.0, gy = 0.0, gz = 0.0;
+            load_x(x, m.iqseq[iq], xi);
+            if (act) {
+#pragma unroll
+                for (int a = 0; a < NA; ++a) {
+                    if (a >= na) break;
+                    const bool lj = !WATER || !SPC || a == 0;
+                    double tx, ty, tz;
+                    if (BOX) {
+                        tx = sh[0] - (xi[0] - xj[a][0]), ty = sh[1] - (xi[1] - xj[a][1]), tz = sh[2] - (xi[2] - xj[a][2]);
+                    } else {
+                        tx = xj[a][0] - xi[0], ty = xj[a][1] - xi[1], tz = xj[a][2] - xi[2];
+                    }
+                    const double d2 = tx * tx + ty * ty + tz * tz, r = rsqrt(d2);
+                    const QPar* P = WATER ? m.qw_tab + (size_t)(iq * m.sa + a) * S
+                                          : m.qp_tab + ((size_t)j0 * nq + iq) * S;
+                    double sum = 0.0;   // -dv / r2
+                    if (lj) {           // nbe_qx, src/nonbonded.f90:200-222
+                        const double d6 = d2 * d2 * d2;
+                        double sc = 0.0, u = 0.0, u2 = 0.0, ud6 = 0.0;
+#pragma unroll
+                        for (int st = 0; st < SMAX; ++st) {
+                            if (st >= S) break;
+                            const QPar q = P[st];
+                            if (st == 0 || __double_as_longlong(q.sc) != __double_as_longlong(sc)) {
+                                sc = q.sc;
+                                u = 1.0 / (d6 + sc);
+                                u2 = u * u;
+                                ud6 = u * d6;
+                            }
+                            const double vel = q.el * r, va = q.A * u2, vb = q.B * u;
+                            sum += (vel + (12.0 * va - 6.0 * vb) * ud6) * s.lambda[st];
+                            eel[st].add(vel);
+                            evdw[st].add(va - vb);
+                        }
+                    } else {            // nbe_qspc, src/nonbonded.f90:226-243
+#pragma unroll
+                        for (int st = 0; st < SMAX; ++st) {
+                            if (st >= S) break;
+                            const double vel = P[st].el * r;
+                            sum += vel * s.lambda[st];
+                            eel[st].add(vel);
+                        }
+                    }
+                    const double dvs = -(r * r) * sum;
+                    gx -= tx * dvs; gy -= ty * dvs; gz -= tz * dvs;
+                    gj[a][0] += tx * dvs; gj[a][1] += ty * dvs; gj[a][2] += tz * dvs;
+                }
+            }
+            g[3 * b] = gx;
+            g[3 * b + 1] = gy;
+            g[3 * b + 2] = gz;
+        }
+        const double v = reduce_scatter<16>(g, lane);
+        const int idx = lane >> 1;   // the component this lane pair holds
+        if (!(lane & 1) && idx < 3 * kQRed && 3 * q0 + idx < 3 * nq)
+            atomicAdd(s.d + 3 * m.iqseq[q0 + idx / 3] + idx % 3, v);
+        if (act) {
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+                if (a < na) acc.grad(j0 + a, gj[a][0], gj[a][1], gj[a][2]);
+        }
+    }
+    const int kel = WATER ? 4 : 2;
+#pragma unroll
+    for (int st = 0; st < SMAX; ++st) {
+        if (st >= S) break;
+        eel[st].flush(acc, eq_slot(st, kel));
+        evdw[st].flush(acc, eq_slot(st, kel + 1));
     }
 }
 
@@ -4041,32 +3980,37 @@ void launch_ww(const Launch& L) {
     } else if (three) k_ww<false, 3><<<g, 128, 0, L.st>>>(L.m, L.ds);
     else k_ww<false, 0><<<g, 128, 0, L.st>>>(L.m, L.ds);
 }
-#ifndef QNB_Q_LANES
-#define QNB_Q_LANES 1   // mixed form: k_qenv_lanes (1) or k_qenv (0)
-#endif
+// Q-environment terms of the sphere (iwhich null) or the box
 template <bool WATER>
-void launch_qenv(const Launch& L, int mixed, dim3 g) {
-    bool spc = L.m.spc != 0;
-    bool s4 = L.m.S <= 4;
-#define QL(MIX, SPC, SM) k_qenv<MIX, SPC, WATER, SM><<<g, kQBlock, 0, L.st>>>(L.m, L.ds, L.tu.v[T_QCHUNK])
-#define QT(SPC, SM) k_qenv_lanes<SPC, WATER, SM><<<g, kQBlock, 0, L.st>>>(L.m, L.ds)
-    if (mixed && QNB_Q_LANES) {
-        if (spc) { if (s4) QT(true, 4); else QT(true, kMaxStates); }
-        else { if (s4) QT(false, 4); else QT(false, kMaxStates); }
-    } else if (mixed) {
-        if (spc) { if (s4) QL(true, true, 4); else QL(true, true, kMaxStates); }
-        else { if (s4) QL(true, false, 4); else QL(true, false, kMaxStates); }
-    } else {
-        if (spc) { if (s4) QL(false, true, 4); else QL(false, true, kMaxStates); }
-        else { if (s4) QL(false, false, 4); else QL(false, false, kMaxStates); }
-    }
-#undef QL
+void launch_qenv(const Launch& L, int mixed, int per_sm, const int* iwhich, double rcq2) {
+    const int units = WATER ? L.m.nwat : L.m.nat_solute;
+    if (units == 0 || L.m.nqat == 0) return;
+    const bool spc = L.m.spc != 0, s4 = L.m.S <= 4, box = iwhich != nullptr;
+    if (mixed) {
+        dim3 g = grid_for((int64_t)(WATER ? L.s0.cap_qw : L.s0.cap_qp) * 32, kQBlock, per_sm, L.nwin);
+        const float rq2 = (float)rcq2;
+#define QT(SPC, SM, BX) k_qenv_lanes<SPC, WATER, SM, BX><<<g, kQBlock, 0, L.st>>>(L.m, L.ds, iwhich, rq2)
+#define QS(SPC, SM) do { if (box) QT(SPC, SM, true); else QT(SPC, SM, false); } while (0)
+        if (spc) { if (s4) QS(true, 4); else QS(true, kMaxStates); }
+        else { if (s4) QS(false, 4); else QS(false, kMaxStates); }
+#undef QS
 #undef QT
+        return;
+    }
+    const int64_t items = (int64_t)((units + 31) / 32) * ((L.m.nqat + kQRed - 1) / kQRed);
+    dim3 g = grid_for(items * 32, 128, 2 * per_sm, L.nwin);
+#define Q64(SPC, NA, SM, BX) k_qenv64<SPC, WATER, NA, SM, BX><<<g, 128, 0, L.st>>>(L.m, L.ds, iwhich, rcq2)
+#define Q6S(SPC, NA, BX) do { if (s4) Q64(SPC, NA, 4, BX); else Q64(SPC, NA, kMaxStates, BX); } while (0)
+#define Q6B(SPC, NA) do { if (box) Q6S(SPC, NA, true); else Q6S(SPC, NA, false); } while (0)
+    if constexpr (!WATER) Q6B(true, 1);
+    else if (spc && L.m.sa <= 3) Q6B(true, 3);
+    else if (spc) Q6B(true, kMaxSolv);
+    else Q6B(false, kMaxSolv);
+#undef Q6B
+#undef Q6S
+#undef Q64
 }
-void launch_qw(const Launch& L, int mixed) {
-    if (L.m.nwat == 0 || L.m.nqat == 0) return;
-    launch_qenv<true>(L, mixed, grid_for(L.s0.cap_qw * 32, kQBlock, L.tu.v[T_QW], L.nwin));
-}
+void launch_qw(const Launch& L, int mixed) { launch_qenv<true>(L, mixed, L.tu.v[T_QW], nullptr, 0.0); }
 void launch_pw(const Launch& L) {
     if (L.m.nwat == 0 || L.m.ncgp_solute == 0) return;
     k_pw<<<grid_for(L.s0.cap_pw, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds);
@@ -4075,10 +4019,7 @@ void launch_pp(const Launch& L) {
     if (L.m.ncgp_solute == 0) return;
     k_pp<<<grid_for(L.s0.cap_pp, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds);
 }
-void launch_qp(const Launch& L, int mixed) {
-    if (L.m.nqat == 0 || L.m.nat_solute == 0) return;
-    launch_qenv<false>(L, mixed, grid_for(L.s0.cap_qp * 32, kQBlock, L.tu.v[T_QP], L.nwin));
-}
+void launch_qp(const Launch& L, int mixed) { launch_qenv<false>(L, mixed, L.tu.v[T_QP], nullptr, 0.0); }
 void launch_nonbond_qq(const Launch& L, int mixed) {
     if (L.s0.nqq == 0) return;
     dim3 g((L.s0.nqq + 255) / 256, L.nwin);
@@ -4939,87 +4880,6 @@ __global__ void __launch_bounds__(256) k_box_ww(DevModel m, const DevState* __re
     evdw.flush(acc, E_WW_VDW);
 }
 
-// nonbond_qp_box, src/nonbondene.f90:5234-5335, and nonbond_qw_box /
-// nonbond_qw_spc_box, 5422-5505, 5771-5881 (nbe_qx, nbe_qspc), FP64 form
-// (the mixed form runs k_qenv_lanes<..., BOX>): one thread per (listed unit,
-// Q atom); the unit's shift brings it next to qswitch, taken from the first
-// group atom inside Rcq (qp, nbqp_cgp) or the water's first atom (qw).
-// Per-state energies are summed in registers.
-template <bool MIX, bool WATER, bool SPC>
-__global__ void __launch_bounds__(256) k_box_q(DevModel m, const DevState* __restrict__ states,
-                                               const int* __restrict__ iwhich, double rcq2) {
-    const DevState& s = states[blockIdx.y];
-    Acc<MIX> acc = make_acc<MIX>(s);
-    const double* __restrict__ x = s.x;
-    const int S = m.S, nq = m.nqat;
-    ESum<MIX> eel[kMaxStates], evdw[kMaxStates];
-    int n = WATER ? min((int64_t)s.cnt[C_QW], s.cap_qw) : min((int64_t)s.cnt[C_QP], s.cap_qp);
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)n * nq;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        int u = (int)(t / nq), iq = (int)(t % nq);
-        int i = m.iqseq[iq];
-        double sx, sy, sz;
-        int j0, na;
-        if (WATER) {
-            j0 = m.nat_solute + m.sa * s.qw[u];
-            na = m.sa;
-            box_shift(m, x, m.qswitch, j0, sx, sy, sz);
-        } else {
-            j0 = s.qp[u];
-            na = 1;
-            int g = iwhich[j0], ref = m.gatom[m.gslot[g]];
-            for (int a = m.gslot[g]; a < m.gslot[g + 1]; ++a)
-                if (box_d2(m, x, m.gatom[a], m.qswitch) <= rcq2) {
-                    ref = m.gatom[a];
-                    break;
-                }
-            box_shift(m, x, m.qswitch, ref, sx, sy, sz);
-        }
-        double gi[3] = {0, 0, 0};
-        for (int a = 0; a < na; ++a) {
-            int j = j0 + a;
-            BoxPair q = box_pair(x, i, j, sx, sy, sz);
-            bool lj = !(WATER && SPC) || a == 0;
-            double dvs = 0.0;
-            double r6hc = 1.0 / (q.r2 * q.r2 * q.r2);
-            for (int st = 0; st < S; ++st) {
-                const QPar P = WATER ? m.qw_tab[((size_t)iq * m.sa + a) * S + st] : m.qp_tab[((size_t)j * nq + iq) * S + st];
-                double lam = s.lambda[st];
-                if (lj) {
-                    double vel, vdw, dv;
-                    nbe_qx_d(q.r2, q.r, r6hc, P.A, P.B, P.el, P.sc, lam, vel, vdw, dv);
-                    dvs += dv;
-                    eel[st].add(vel);
-                    evdw[st].add(vdw);
-                } else {   // nbe_qspc
-                    double vel = P.el * q.r;
-                    dvs += -q.r2 * vel * lam;
-                    eel[st].add(vel);
-                }
-            }
-            gi[0] -= q.tx * dvs;
-            gi[1] -= q.ty * dvs;
-            gi[2] -= q.tz * dvs;
-            box_grad<MIX>(acc, j, q.tx * dvs, q.ty * dvs, q.tz * dvs);
-        }
-        box_grad<MIX>(acc, i, gi[0], gi[1], gi[2]);
-    }
-    for (int st = 0; st < S; ++st) {
-        eel[st].flush(acc, eq_slot(st, WATER ? 4 : 2));
-        evdw[st].flush(acc, eq_slot(st, WATER ? 5 : 3));
-    }
-}
-
-// the mixed form's box Q terms (k_qenv_lanes<..., BOX>)
-template <bool WATER>
-void launch_box_qenv(const Launch& L, const int* iwhich, double rcq2, dim3 g) {
-    const bool spc = L.m.spc != 0, s4 = L.m.S <= 4;
-    const float rq2 = (float)rcq2;
-#define QB(SPC, SM) k_qenv_lanes<SPC, WATER, SM, true><<<g, kQBlock, 0, L.st>>>(L.m, L.ds, iwhich, rq2)
-    if (spc) { if (s4) QB(true, 4); else QB(true, kMaxStates); }
-    else { if (s4) QB(false, 4); else QB(false, kMaxStates); }
-#undef QB
-}
 int launch_box_nonbond(const Launch& L, int md, int mixed, const int* iwhich, double rcq2, int pairs) {
     const DevModel& m = L.m;
     int nl = 0;
@@ -5040,22 +4900,12 @@ int launch_box_nonbond(const Launch& L, int md, int mixed, const int* iwhich, do
             nl += 2;
         }
         if (m.nqat > 0) {
-            if (mixed) {   // lane = water, Q atoms looped (k_qenv_lanes' box form); environment gradient into fq
-                launch_box_qenv<true>(L, iwhich, rcq2, grid_for(L.s0.cap_qw * 32, kQBlock, L.tu.v[T_QW], L.nwin));
-            } else {
-                dim3 g = grid(L.s0.cap_qw * m.nqat);
-                if (m.spc) k_box_q<false, true, true><<<g, 256, 0, L.st>>>(m, L.ds, iwhich, rcq2); else k_box_q<false, true, false><<<g, 256, 0, L.st>>>(m, L.ds, iwhich, rcq2);
-            }
+            launch_qenv<true>(L, mixed, L.tu.v[T_QW], iwhich, rcq2);
             ++nl;
         }
     }
     if (m.nqat > 0 && m.nat_solute > 0) {
-        if (mixed) {
-            launch_box_qenv<false>(L, iwhich, rcq2, grid_for(L.s0.cap_qp * 32, kQBlock, L.tu.v[T_QP], L.nwin));
-        } else {
-            dim3 g = grid(L.s0.cap_qp * m.nqat);
-            k_box_q<false, false, false><<<g, 256, 0, L.st>>>(m, L.ds, iwhich, rcq2);
-        }
+        launch_qenv<false>(L, mixed, L.tu.v[T_QP], iwhich, rcq2);
         ++nl;
     }
     return nl;

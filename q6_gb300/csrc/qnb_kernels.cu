@@ -753,190 +753,6 @@ __device__ __forceinline__ bool lrf_pair(float r2f, const Band& rc, const Band& 
     return r2 > rc.c && r2 <= rl.c;
 }
 
-// One warp per target group g2 sums the far-field contributions of every
-// non-Q atom whose group is classified "LRF" against g2; the 40 coefficients
-// are then reduced across the warp.  The warps of a block take consecutive
-// targets and stream the source atoms through shared memory together: each
-// atom (position, charge, its group's distance atom) is loaded from global
-// memory once per block instead of once per target.  Mixed form: FP32 terms
-// (rsqrt on the SFU); FP64 form: FP64 terms.
-constexpr int kLrfBlock = 256;
-template <bool MIX>
-__global__ void __launch_bounds__(kLrfBlock) k_lrf_accumulate(DevModel m, const DevState* __restrict__ states, Cut c,
-                                                              const int* __restrict__ lrf_src) {
-    typedef typename std::conditional<MIX, float, double>::type T;
-    const Band bpp = band(c.rcpp2, c.fpp), bpw = band(c.rcpw2, c.fpw), bww = band(c.rcww2, c.fww),
-               blrf = band(c.rlrf2, c.flrf);
-    __shared__ float4 s_xs[kLrfBlock];                  // distance atom of the source's group
-    __shared__ int s_src[kLrfBlock];                    // lrf_src entry (-1: not a source)
-    __shared__ T s_xi[4 * kLrfBlock];                   // source x, y, z (centred in FP32), charge
-    const DevState& s = states[blockIdx.y];
-    const double* __restrict__ x = s.x;
-    const float4* __restrict__ xq = s.xq;
-    double* __restrict__ lrf = s.lrf;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kLrfBlock / 32;
-    for (int gbase = blockIdx.x * nw; gbase < m.ncgp; gbase += gridDim.x * nw) {   // block-uniform
-        const int g2 = gbase + warp;
-        int s2 = 0;
-        bool act = g2 < m.ncgp;
-        if (act) {
-            s2 = group_dist_atom(m, g2);
-            act = !m.excl[s2];
-        }
-        const bool sol2 = act && g2 < m.ncgp_solute;
-        const Band rc_s = sol2 ? bpp : bpw, rc_w = sol2 ? bpw : bww;
-        double cx = 0.0, cy = 0.0, cz = 0.0;
-        float4 x2 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (act) {
-            const double* L = lrf + (size_t)g2 * kLrfLen;
-            cx = L[0]; cy = L[1]; cz = L[2];
-            x2 = xq[s2];
-        }
-        const T ccx = MIX ? T(cx - m.xpcent[0]) : T(cx), ccy = MIX ? T(cy - m.xpcent[1]) : T(cy),
-                ccz = MIX ? T(cz - m.xpcent[2]) : T(cz);
-        T mom[kLrfMom];
-#pragma unroll
-        for (int k = 0; k < kLrfMom; ++k) mom[k] = T(0);
-        for (int i0 = 0; i0 < m.natom; i0 += kLrfBlock) {
-            __syncthreads();
-            {
-                int i = i0 + threadIdx.x, t = threadIdx.x;
-                int src = i < m.natom ? lrf_src[i] : -1;
-                s_src[t] = src;
-                if (src >= 0) {
-                    s_xs[t] = xq[src & 0x3fffffff];
-                    if constexpr (MIX) {
-                        float4 xi = xq[i];
-                        s_xi[4 * t] = xi.x; s_xi[4 * t + 1] = xi.y; s_xi[4 * t + 2] = xi.z; s_xi[4 * t + 3] = xi.w;
-                    } else {
-                        s_xi[4 * t] = x[3 * i]; s_xi[4 * t + 1] = x[3 * i + 1]; s_xi[4 * t + 2] = x[3 * i + 2];
-                        s_xi[4 * t + 3] = m.crg[i];
-                    }
-                }
-            }
-            __syncthreads();
-            if (!act) continue;
-            const int n = min(kLrfBlock, m.natom - i0);
-            for (int k = lane; k < n; k += kWarp) {
-                int src = s_src[k];   // distance atom of i's group | solute flag << 30
-                if (src < 0) continue;
-                int s1 = src & 0x3fffffff;
-                if (s1 == s2) continue;   // same group
-                const Band& rc2 = (src >> 30) ? rc_s : rc_w;
-                if (!lrf_pair(r2_f(x2, s_xs[k]), rc2, blrf, x, s2, s1)) continue;
-                lrf_terms<T>(s_xi[4 * k] - ccx, s_xi[4 * k + 1] - ccy, s_xi[4 * k + 2] - ccz, s_xi[4 * k + 3], mom);
-            }
-        }
-        if (!act) continue;
-        double tot[kLrfMom];
-#pragma unroll
-        for (int k = 0; k < kLrfMom; ++k) {
-            T v = mom[k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-            tot[k] = (double)v;
-        }
-        if (lane == 0) lrf_expand(tot, lrf + (size_t)g2 * kLrfLen + 3);
-    }
-}
-
-// Mixed form, two target groups per warp: every lane applies the source atom
-// it loaded to both targets, so the shared-memory loads and the loop
-// overhead of a source atom are paid once for two targets (the kernel is
-// issue-bound: about 90 instructions per target and source with one target
-// per warp).  Sums and their order per target are those of k_lrf_accumulate.
-constexpr int kLrfPair = 2;
-__global__ void __launch_bounds__(kLrfBlock) k_lrf_accumulate2(DevModel m, const DevState* __restrict__ states, Cut c,
-                                                               const int* __restrict__ lrf_src) {
-    const Band bpp = band(c.rcpp2, c.fpp), bpw = band(c.rcpw2, c.fpw), bww = band(c.rcww2, c.fww),
-               blrf = band(c.rlrf2, c.flrf);
-    __shared__ float4 s_xs[kLrfBlock];
-    __shared__ int s_src[kLrfBlock];
-    __shared__ float4 s_xi[kLrfBlock];
-    const DevState& s = states[blockIdx.y];
-    const double* __restrict__ x = s.x;
-    const float4* __restrict__ xq = s.xq;
-    double* __restrict__ lrf = s.lrf;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kLrfBlock / 32;
-    const int per_block = nw * kLrfPair;
-    for (int gbase = blockIdx.x * per_block; gbase < m.ncgp; gbase += gridDim.x * per_block) {   // block-uniform
-        int g2[kLrfPair], s2[kLrfPair];
-        bool act[kLrfPair];
-        Band rc_s[kLrfPair], rc_w[kLrfPair];
-        float4 x2[kLrfPair];
-        float ccx[kLrfPair], ccy[kLrfPair], ccz[kLrfPair];
-        float mom[kLrfPair][kLrfMom];
-#pragma unroll
-        for (int t = 0; t < kLrfPair; ++t) {
-            g2[t] = gbase + kLrfPair * warp + t;
-            s2[t] = 0;
-            act[t] = g2[t] < m.ncgp;
-            if (act[t]) {
-                s2[t] = group_dist_atom(m, g2[t]);
-                act[t] = !m.excl[s2[t]];
-            }
-            const bool sol2 = act[t] && g2[t] < m.ncgp_solute;
-            rc_s[t] = sol2 ? bpp : bpw;
-            rc_w[t] = sol2 ? bpw : bww;
-            double cx = 0.0, cy = 0.0, cz = 0.0;
-            x2[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (act[t]) {
-                const double* L = lrf + (size_t)g2[t] * kLrfLen;
-                cx = L[0]; cy = L[1]; cz = L[2];
-                x2[t] = xq[s2[t]];
-            }
-            ccx[t] = (float)(cx - m.xpcent[0]);
-            ccy[t] = (float)(cy - m.xpcent[1]);
-            ccz[t] = (float)(cz - m.xpcent[2]);
-#pragma unroll
-            for (int k = 0; k < kLrfMom; ++k) mom[t][k] = 0.f;
-        }
-        const bool any = act[0] || act[1];
-        for (int i0 = 0; i0 < m.natom; i0 += kLrfBlock) {
-            __syncthreads();
-            {
-                int i = i0 + threadIdx.x, t = threadIdx.x;
-                int src = i < m.natom ? lrf_src[i] : -1;
-                s_src[t] = src;
-                if (src >= 0) {
-                    s_xs[t] = xq[src & 0x3fffffff];
-                    s_xi[t] = xq[i];
-                }
-            }
-            __syncthreads();
-            if (!any) continue;
-            const int n = min(kLrfBlock, m.natom - i0);
-            for (int k = lane; k < n; k += kWarp) {
-                int src = s_src[k];   // distance atom of i's group | solute flag << 30
-                if (src < 0) continue;
-                const int s1 = src & 0x3fffffff;
-                const bool sol1 = (src >> 30) != 0;
-                const float4 xs = s_xs[k], xi = s_xi[k];
-#pragma unroll
-                for (int t = 0; t < kLrfPair; ++t) {
-                    if (!act[t] || s1 == s2[t]) continue;
-                    const Band& rc2 = sol1 ? rc_s[t] : rc_w[t];
-                    if (!lrf_pair(r2_f(x2[t], xs), rc2, blrf, x, s2[t], s1)) continue;
-                    lrf_terms<float>(xi.x - ccx[t], xi.y - ccy[t], xi.z - ccz[t], xi.w, mom[t]);
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < kLrfPair; ++t) {
-            if (!act[t]) continue;   // warp-uniform
-            double tot[kLrfMom];
-#pragma unroll
-            for (int k = 0; k < kLrfMom; ++k) {
-                float v = mom[t][k];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-                tot[k] = (double)v;
-            }
-            if (lane == 0) lrf_expand(tot, lrf + (size_t)g2[t] * kLrfLen + 3);
-        }
-    }
-}
-
 // lattice shift and minimum-image distance of two atoms (periodic box)
 __device__ __forceinline__ void box_shift(const DevModel& m, const double* __restrict__ x, int a, int b,
                                           double& sx, double& sy, double& sz) {
@@ -1174,14 +990,55 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
     lrf_expand(m24, s.lrf + (size_t)g2 * kLrfLen + 3);
 }
 
-// Unstaged variant: one warp per target group reads the source atoms straight
-// from global memory (lanes stride over the atoms, so loads are coalesced).
-template <bool MIX, bool BOX>
-__global__ void __launch_bounds__(128) k_lrf_accumulate_direct(DevModel m, const DevState* __restrict__ states, Cut c,
-                                                         const int* __restrict__ lrf_src) {
+// The 20 moment sums of one source atom at d = (dx, dy, dz) from the target's
+// centre, in the scaled vector e = d / r^2 and w = q / r:
+//   n[0] w   n[1..3] -w e   n[4..9] w e e (xx xy xz yy yz zz)
+//   n[10..19] w e e e (xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz)
+// w e e = q d d / r^5 and w e e e = q d d d / r^7, so S2 = 3 n and S3 = -15 n
+// (lrf_scale20).  The products of one order are the factors of the next, so a
+// term takes 38 operations and a reciprocal square root.
+__device__ __forceinline__ void lrf_terms_e(double dx, double dy, double dz, double q, double* n) {
+    const double ri = rsqrt(dx * dx + dy * dy + dz * dz), ri2 = ri * ri, w = q * ri;
+    const double ex = dx * ri2, ey = dy * ri2, ez = dz * ri2;
+    const double ax = w * ex, ay = w * ey, az = w * ez;
+    const double bxx = ax * ex, byy = ay * ey, bzz = az * ez, bxy = ax * ey;
+    n[0] += w;
+    n[1] -= ax;
+    n[2] -= ay;
+    n[3] -= az;
+    n[4] += bxx;
+    n[5] += bxy;
+    n[6] += ax * ez;
+    n[7] += byy;
+    n[8] += ay * ez;
+    n[9] += bzz;
+    n[10] += bxx * ex;
+    n[11] += bxx * ey;
+    n[12] += bxx * ez;
+    n[13] += byy * ex;
+    n[14] += bxy * ez;
+    n[15] += bzz * ex;
+    n[16] += byy * ey;
+    n[17] += byy * ez;
+    n[18] += bzz * ey;
+    n[19] += bzz * ez;
+}
+__device__ __forceinline__ void lrf_scale20(double* n) {
+#pragma unroll
+    for (int k = 4; k < 10; ++k) n[k] *= 3.0;
+#pragma unroll
+    for (int k = 10; k < kLrfMom20; ++k) n[k] *= -15.0;
+}
+
+// FP64 form: one warp per target group reads the source atoms straight from
+// global memory (lanes stride over the atoms, so loads are coalesced); its
+// terms bound it (the FP64 pipe: 16 windows of the 25 A sphere 20.6 ms with
+// two divisions, a square root and 24 sums per term, 13.4 ms with these).
+template <bool BOX>
+__global__ void __launch_bounds__(128) k_lrf_accumulate64(DevModel m, const DevState* __restrict__ states, Cut c,
+                                                          const int* __restrict__ lrf_src) {
     const Band bpp = band(c.rcpp2, c.fpp), bpw = band(c.rcpw2, c.fpw), bww = band(c.rcww2, c.fww),
                blrf = band(c.rlrf2, c.flrf);
-    typedef typename std::conditional<MIX, float, double>::type T;
     const DevState& s = states[blockIdx.y];
     const double* __restrict__ x = s.x;
     const float4* __restrict__ xq = s.xq;
@@ -1194,43 +1051,38 @@ __global__ void __launch_bounds__(128) k_lrf_accumulate_direct(DevModel m, const
         double* L = lrf + (size_t)g2 * kLrfLen;
         double cx = L[0], cy = L[1], cz = L[2];
         float4 x2 = xq[s2];
-        float cxf = (float)(cx - m.xpcent[0]), cyf = (float)(cy - m.xpcent[1]), czf = (float)(cz - m.xpcent[2]);
         const Band rc_s = sol2 ? bpp : bpw, rc_w = sol2 ? bpw : bww;
-        T mom[kLrfMom];
+        double mom[kLrfMom20];
 #pragma unroll
-        for (int k = 0; k < kLrfMom; ++k) mom[k] = T(0);
+        for (int k = 0; k < kLrfMom20; ++k) mom[k] = 0.0;
         for (int i = lane; i < m.natom; i += kWarp) {
             int src = lrf_src[i];   // distance atom of i's group | solute flag << 30, -1 if never a source
             if (src < 0) continue;
             int s1 = src & 0x3fffffff;
             if (s1 == s2) continue;   // same group
             const Band& rc2 = (src >> 30) ? rc_s : rc_w;
-            if constexpr (BOX) {   // FP64 minimum image and lattice shift (the FP64 form)
-                static_assert(!MIX, "the mixed form's box LRF is k_lrf_nbody<true>");
+            double sx = 0.0, sy = 0.0, sz = 0.0;
+            if constexpr (BOX) {   // FP64 minimum image and lattice shift
                 if (!lrf_pair_box_exact(m, x, s2, s1, rc2.c, blrf.c)) continue;
-                double sx = m.boxl[0] * round((x[3 * s1] - cx) * m.inv_boxl[0]);
-                double sy = m.boxl[1] * round((x[3 * s1 + 1] - cy) * m.inv_boxl[1]);
-                double sz = m.boxl[2] * round((x[3 * s1 + 2] - cz) * m.inv_boxl[2]);
-                lrf_terms<double>(x[3 * i] - cx - sx, x[3 * i + 1] - cy - sy, x[3 * i + 2] - cz - sz, m.crg[i], mom);
+                sx = m.boxl[0] * round((x[3 * s1] - cx) * m.inv_boxl[0]);
+                sy = m.boxl[1] * round((x[3 * s1 + 1] - cy) * m.inv_boxl[1]);
+                sz = m.boxl[2] * round((x[3 * s1 + 2] - cz) * m.inv_boxl[2]);
+            } else if (!lrf_pair(r2_f(x2, xq[s1]), rc2, blrf, x, s2, s1)) {
                 continue;
             }
-            if (!lrf_pair(r2_f(x2, xq[s1]), rc2, blrf, x, s2, s1)) continue;
-            if constexpr (MIX) {
-                float4 xi = xq[i];
-                lrf_terms<float>(xi.x - cxf, xi.y - cyf, xi.z - czf, xi.w, mom);
-            } else {
-                lrf_terms<double>(x[3 * i] - cx, x[3 * i + 1] - cy, x[3 * i + 2] - cz, m.crg[i], mom);
-            }
+            double dx = x[3 * i] - cx, dy = x[3 * i + 1] - cy, dz = x[3 * i + 2] - cz;
+            if constexpr (BOX) dx -= sx, dy -= sy, dz -= sz;
+            lrf_terms_e(dx, dy, dz, m.crg[i], mom);
         }
-        double tot[kLrfMom];
+        __syncwarp();
 #pragma unroll
-        for (int k = 0; k < kLrfMom; ++k) {
-            T v = mom[k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFull, v, o);
-            tot[k] = (double)v;
+        for (int k = 0; k < kLrfMom20; ++k) mom[k] = warp_sum(mom[k]);
+        if (lane == 0) {
+            double m24[kLrfMom];
+            lrf_scale20(mom);
+            lrf_moments24(mom, m24);
+            lrf_expand(m24, L + 3);
         }
-        if (lane == 0) lrf_expand(tot, L + 3);
     }
 }
 
@@ -3863,19 +3715,7 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
         else k_lrf_accumulate_any<false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
         return 1;
     }
-// FP64 form: the unstaged kernel measured faster (its FP64 terms, not the
-// loads, bound it, and the staged block holds more registers)
-#ifndef QNB_LRF_FP64_STAGED
-#define QNB_LRF_FP64_STAGED 0
-#endif
-#ifndef QNB_LRF_PAIR
-#define QNB_LRF_PAIR 1   // mixed form: two target groups per warp (k_lrf_accumulate2)
-#endif
-#ifndef QNB_LRF_NBODY
-#define QNB_LRF_NBODY 1  // mixed form: one thread per target group (k_lrf_nbody)
-#endif
-    dim3 g = grid_for((int64_t)L.m.ncgp * 32, kLrfBlock, L.tu.v[T_LRF], L.nwin);
-    if (mixed && QNB_LRF_NBODY) {
+    if (mixed) {
         // source ranges of at least one staged tile each; the split depends on
         // the topology only, so a window's coefficients are the same in a
         // batch of any size (51 windows of a 1,400-source-group system:
@@ -3886,15 +3726,10 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
         else k_lrf_nbody<false><<<g, kLrfNB, 0, L.st>>>(L.m, L.ds, c, nsplit);
         k_lrf_combine<<<dim3((L.m.ncgp + 127) / 128, L.nwin), 128, 0, L.st>>>(L.m, L.ds, nsplit);
         return 2;
-    } else if (mixed && QNB_LRF_PAIR)
-        k_lrf_accumulate2<<<grid_for((int64_t)L.m.ncgp * 32 / kLrfPair, kLrfBlock, L.tu.v[T_LRF], L.nwin), kLrfBlock, 0,
-                            L.st>>>(L.m, L.ds, c, lrf_src);
-    else if (mixed) k_lrf_accumulate<true><<<g, kLrfBlock, 0, L.st>>>(L.m, L.ds, c, lrf_src);
-    else if (QNB_LRF_FP64_STAGED) k_lrf_accumulate<false><<<g, kLrfBlock, 0, L.st>>>(L.m, L.ds, c, lrf_src);
-    else if (L.m.box)
-        k_lrf_accumulate_direct<false, true><<<grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin), 128, 0, L.st>>>(
-            L.m, L.ds, c, lrf_src);
-    else k_lrf_accumulate_direct<false, false><<<grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds, c, lrf_src);
+    }
+    dim3 g = grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin);
+    if (L.m.box) k_lrf_accumulate64<true><<<g, 128, 0, L.st>>>(L.m, L.ds, c, lrf_src);
+    else k_lrf_accumulate64<false><<<g, 128, 0, L.st>>>(L.m, L.ds, c, lrf_src);
     return 1;
 }
 

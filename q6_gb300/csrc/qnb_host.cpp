@@ -108,6 +108,7 @@ struct qnb_context {
         int* goff = nullptr;
         int* gatom = nullptr;
         int n = 0;
+        int tile_atoms = 0;   // most atoms of any kLrfTileGroups consecutive groups
     } lrft[2];
     // exclusion flags: the topology's, and all-clear for the box (excluded
     // atoms take part in every box list, in lrf_taylor and in temperature())
@@ -326,6 +327,7 @@ void use_lrf_tables(qnb_context* c, int tab) {
     c->m.nlrf_groups = T.n;
     c->m.lrf_gmeta = T.gmeta;
     c->m.lrf_goff = T.goff;
+    c->m.lrf_tile_atoms = T.tile_atoms;
     c->m.lrf_gatom = T.gatom;
     c->d_lrf_src = T.src;
 }
@@ -458,6 +460,7 @@ int build_model(qnb_context* c, const qnb_topology* t) {
         }
         auto& T = c->lrft[tab];
         T.n = (int)gmeta.size();
+        for (int g = 0; g < T.n; ++g) T.tile_atoms = std::max(T.tile_atoms, goff[std::min(T.n, g + kLrfTileGroups)] - goff[g]);
         TRY(c->upload(&T.src, lrf_src));
         TRY(c->upload(&T.gmeta, gmeta));
         TRY(c->upload(&T.goff, goff));
@@ -1018,8 +1021,6 @@ int alloc_state(qnb_context* c) {
         s.efix = c->efix_all + (size_t)kNumE * w;
         TRY(c->alloc(&s.lambda, (size_t)std::max(1, m.S)));
         TRY(c->alloc(&s.lrf, (size_t)std::max(1, m.ncgp) * kLrfLen));
-        if (c->mixed && c->use_lrf)
-            TRY(c->alloc(&s.lrf_part, (size_t)kLrfSplitMax * std::max(1, m.ncgp) * kLrfMoments));
         s.cnt = c->cnt_all + (size_t)C_NUM * w;
         TRY(c->alloc(&s.theta, (size_t)std::max(1, m.nwat)));
         TRY(c->alloc(&s.rkey, (size_t)std::max(1, m.nwat)));
@@ -1201,6 +1202,8 @@ int grow_lists(qnb_context* c, bool* grew, bool* do_qp, bool* do_qw) {
     return QNB_OK;
 }
 
+constexpr int64_t kLrfBehindRows = 16384;   // rows of all windows from which the LRF moments follow the row build
+
 int build_lists(qnb_context* c, const Cut& cut, int nw) {
     Launch L = nw == 1 ? c->one() : c->all();
     bool do_qp = !(c->qp_done && cut.rcq2 > c->rexcl_o2);   // src/nonbondene.f90:3678
@@ -1220,24 +1223,41 @@ int build_lists(qnb_context* c, const Cut& cut, int nw) {
             launch_pack(L);
             if (c->use_lrf) launch_group_centres(L), ++nl;
         });
-        // the LRF accumulation (needs the packed coordinates and the group
-        // centres only) runs on the second stream beside the list builds
-        if (c->use_lrf) {
-            CU(cudaEventRecord(c->ev_fork, c->stream));
-            CU(cudaStreamWaitEvent(c->stream2, c->ev_fork, 0));
-            Launch L2{L.m, L.s0, L.ds, L.nwin, c->stream2, L.tu};
-            timed_on(c, c->stream2, K_LRF_BUILD, [&] { nl += launch_lrf_accumulate(L2, cut, c->mixed, c->d_lrf_src); });
-            CU(cudaEventRecord(c->ev_join, c->stream2));
-        }
+        // The LRF accumulation (needs the packed coordinates and the group
+        // centres only) runs on the second stream beside the list builds; of
+        // a large batch, whose row build fills the device by itself, behind it
+        // instead.  Side by side they also share each SM's 256 KB: rows built
+        // while or after the accumulation holds 190 KB of it as shared memory
+        // have little L1 cache left.  51 windows of the 25 A sphere (87,000
+        // rows): 1,968 us side by side, 1,635 us one after the other; 16
+        // windows in a box (27,000): 1,000 and 888; one window (1,700): 139
+        // and 187.
+        const bool rows = c->mixed && (!c->m.box || c->m.box_rows);
+        const bool behind = rows && (int64_t)nw * (c->ncgp_solute + c->nwat) >= kLrfBehindRows;
+        auto lrf = [&]() -> int {
+            if (!c->use_lrf) return QNB_OK;
+            Launch L2 = L;
+            if (!behind) {
+                CU(cudaEventRecord(c->ev_fork, c->stream));
+                CU(cudaStreamWaitEvent(c->stream2, c->ev_fork, 0));
+                L2.st = c->stream2;
+            }
+            timed_on(c, L2.st, K_LRF_BUILD, [&] { nl += launch_lrf_accumulate(L2, cut, c->mixed, c->d_lrf_src); });
+            if (!behind) CU(cudaEventRecord(c->ev_join, c->stream2));
+            return QNB_OK;
+        };
+        if (!behind) TRY(lrf());
+        if (rows) timed(c, K_BUILD, [&] {
+            nl += launch_bin_cells(L, cut);
+            nl += launch_build_rows(L, cut);
+        });
+        if (behind) TRY(lrf());
         timed(c, K_BUILD, [&] {
             if (c->m.box) {
                 // the mixed form's box path builds the gather rows (switch
                 // atoms, minimum image); the Q lists keep the box builder
-                if (c->m.box_rows) nl += launch_build_rows(L, cut);
                 launch_build_box(L, cut, c->d_qnear, !c->m.box_rows), nl += c->m.box_rows ? 1 : 3;
-            } else if (c->mixed) {
-                nl += launch_build_rows(L, cut);
-            } else {
+            } else if (!c->mixed) {
                 launch_build_pp(L, cut), nl += 2;
                 launch_build_pw(L, cut), ++nl;
                 launch_build_ww(L, cut), ++nl;
@@ -1249,7 +1269,7 @@ int build_lists(qnb_context* c, const Cut& cut, int nw) {
             if (c->mixed && (do_qp || do_qw)) launch_clear_fq(L), ++nl;   // atoms may leave the Q lists
         });
         c->launches += nl;
-        if (c->use_lrf) CU(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+        if (c->use_lrf && !behind) CU(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
         TRY(check_launch());
         CU(cudaMemcpyAsync(c->counts.data(), c->cnt_all, sizeof(int) * C_NUM * nw, cudaMemcpyDeviceToHost,
                            c->stream));

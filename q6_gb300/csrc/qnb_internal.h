@@ -14,7 +14,8 @@ constexpr int kMaxStates = 8;   // FEP states
 constexpr int kMaxShell = 16;   // water polarisation shells
 constexpr int kLrfLen = 43;     // cgp_cent(3) phi0 phi1(3) phi2(9) phi3(27)
 constexpr int kLrfMoments = 24; // symmetric moments the LRF accumulation sums per target group
-constexpr int kLrfSplitMax = 8; // source ranges of the mixed form's LRF accumulation
+constexpr int kLrfTileGroups = 16;  // source groups it stages at a time
+constexpr int kLrfClusterMax = 4;   // blocks per cluster of the mixed form's LRF accumulation
 constexpr double kFix = 4294967296.0;   // 2^32: fixed-point quantum of forces/energies
 constexpr float kFixF = 4294967296.0f;
 
@@ -141,6 +142,7 @@ struct DevModel {
     const int* lrf_gmeta;       // [nlrf_groups]
     const int* lrf_goff;        // [nlrf_groups + 1]
     const int* lrf_gatom;       // [lrf_goff[nlrf_groups]]
+    int lrf_tile_atoms;         // most atoms of any kLrfTileGroups consecutive source groups
     // periodic box (qnb_set_box): rectangular box lengths, their inverses
     // and the Q-list switching atom (FEP file [PBC] switching_atom)
     int box;
@@ -185,7 +187,6 @@ struct DevState {
     unsigned long long* efix;  // [kNumE] fixed-point energies (mixed form)
     double* lambda;      // [S]
     double* lrf;         // [ncgp*43]
-    double* lrf_part;    // mixed form: [kLrfSplitMax][ncgp][kLrfMoments] LRF moments per source range
     int* cnt;            // [C_NUM] list sizes (device-maintained)
     int2* ww; int64_t cap_ww;      // water pairs (iw, jw), iw < jw
     int2* pw; int64_t cap_pw;      // (solute atom, water)
@@ -279,7 +280,8 @@ void launch_build_qp(const Launch& L, const uint8_t* qnear, double rcq2);
 void launch_build_qw(const Launch& L, const Cut& c);
 int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src);
 
-int launch_build_rows(const Launch& L, const Cut& c);
+int launch_bin_cells(const Launch& L, const Cut& c);
+int launch_build_rows(const Launch& L, const Cut& c);   // after launch_bin_cells
 // cells per box edge for the periodic row build (0: too few cells, the rows
 // take every candidate)
 int box_cells(const DevModel& m, const Cut& c, int* n);

@@ -13,6 +13,7 @@
 // is kept at the granularity the reference tests the cut-off at (charge-group
 // pairs, solute atom x water, water pairs) and expanded to atom pairs inside
 // the force kernels.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -48,6 +49,15 @@ __device__ __forceinline__ double dist2_exact(double ax, double ay, double az, d
 __device__ __noinline__ double dist2_exact_atoms(const double* __restrict__ x, int a, int b) {
     return dist2_exact(x[3 * a], x[3 * a + 1], x[3 * a + 2], x[3 * b], x[3 * b + 1], x[3 * b + 2]);
 }
+
+// asynchronous 16-byte global-to-shared copy of a lane (through L2)
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // warp-aggregated append: returns this lane's first slot (valid when n > 0)
 __device__ __forceinline__ int warp_append(int* counter, int n) {
@@ -701,39 +711,13 @@ __device__ __forceinline__ void lrf_expand(const double* m, double* L) {
     P[24] -= U[0]; P[25] -= U[1]; P[26] -= 3.0 * U[2];
 }
 
-// The mixed form's LRF sums with 20 moments: the sums m[10] and m[21..23] of
-// lrf_terms follow from the others, F0 = tr S2 / 3 (f1 r2 = 3 f0) and
+// The LRF sums with 20 moments (the mixed form, and the FP64 form's
+// switch-atom kernels): the sums m[10] and m[21..23] of lrf_terms follow from
+// the others, F0 = tr S2 / 3 (f1 r2 = 3 f0) and
 // U(c) = (S3(xxc) + S3(yyc) + S3(zzc)) / 5 (dr_x^2 + dr_y^2 + dr_z^2 = r2), so
 // they are formed in FP64 from the totals instead of summed per atom.
 //   n[0] phi0, n[1..3] phi1, n[4..9] S2, n[10..19] S3 (the order of lrf_terms)
 constexpr int kLrfMom20 = 20;
-__device__ __forceinline__ void lrf_terms20(float dx, float dy, float dz, float q, float* n) {
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float ri = rsqrtf(r2), ri2 = ri * ri;
-    const float qri = q * ri;
-    const float f0 = qri * ri2;
-    const float f1 = 3.f * f0 * ri2;
-    const float g = -5.f * f1 * ri2;   // 5 f2
-    n[0] += qri;                        // f0 r2
-    n[1] -= dx * f0;
-    n[2] -= dy * f0;
-    n[3] -= dz * f0;
-    const float ax = dx * f1, ay = dy * f1, az = dz * f1;
-    n[4] += ax * dx; n[5] += ax * dy; n[6] += ax * dz;
-    n[7] += ay * dy; n[8] += ay * dz; n[9] += az * dz;
-    const float gx = g * dx, gy = g * dy, gz = g * dz;
-    const float gxx = gx * dx, gyy = gy * dy, gzz = gz * dz, gxy = gx * dy;
-    n[10] += gxx * dx;   // xxx
-    n[11] += gxx * dy;   // xxy
-    n[12] += gxx * dz;   // xxz
-    n[13] += gyy * dx;   // xyy
-    n[14] += gxy * dz;   // xyz
-    n[15] += gzz * dx;   // xzz
-    n[16] += gyy * dy;   // yyy
-    n[17] += gyy * dz;   // yyz
-    n[18] += gzz * dy;   // yzz
-    n[19] += gzz * dz;   // zzz
-}
 // the 24 moments of lrf_expand from the 20 (FP64)
 __device__ __forceinline__ void lrf_moments24(const double* n, double* m) {
     for (int k = 0; k < 10; ++k) m[k] = n[k];
@@ -818,178 +802,6 @@ __device__ __forceinline__ float3 lrf_shift(const DevModel& m, float4 pb, float 
     return make_float3(m.boxlf[0] * roundf(tx), m.boxlf[1] * roundf(ty), m.boxlf[2] * roundf(tz));
 }
 
-// Mixed form, N-body layout: one thread per target group.  The blocks stage
-// the LRF source groups (the eligible atoms of each charge group, in group
-// order: lrf_gmeta / lrf_goff / lrf_gatom) in shared memory, kLrfGT groups
-// per tile, and every thread reads them as broadcasts.  The group-pair
-// classification runs once per (target, source group); the source group's
-// atoms then add their terms.  Each thread's 20 moment sums (lrf_terms20) run
-// in FP32 over at most kLrfFold source groups and are then folded into a
-// double-float accumulator with Knuth's TwoSum (s = a + b, bb = s - a,
-// e = (a - (s - bb)) + (b - bb)), so the FP32 rounding of the sums is kept
-// to short runs.  The source groups are split into nsplit ranges
-// (blockIdx.z, the split fixed by the topology) whose moments
-// k_lrf_combine adds in range order: each target's order of terms is fixed,
-// so its coefficients do not depend on the launch or the number of windows.
-constexpr int kLrfNB = 64;     // targets per block
-constexpr int kLrfGT = 64;     // source groups per staged tile
-constexpr int kLrfFold = 8;    // source groups per FP32 partial sum
-
-__device__ __forceinline__ void two_sum_fold(float& hi, float& lo, float& p) {
-    float s = __fadd_rn(hi, p);
-    float bb = __fsub_rn(s, hi);
-    float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(p, bb));
-    hi = s;
-    lo = __fadd_rn(lo, e);
-    p = 0.f;
-}
-
-// The 20 moments of lrf_terms20 in packed FP32x2 arithmetic: the source
-// atom's (x, y) and (z, q) arrive as register pairs from the staged float4,
-// and the 20 sums are held as 10 pairs, so 10 FFMA2 replace 20 FFMA.  Each
-// sum gets the same products in the same order as in lrf_terms20.  Slots
-// (lrf_slot):
-// (n1,n2) (n3,n0) (n4,n5) (n6,n9) (n7,n8) (n10,n11) (n12,n19) (n13,n16)
-// (n14,n17) (n15,n18).
-__host__ __device__ constexpr int lrf_slot(int k) {
-    constexpr int t[kLrfMom20] = {1, 2, 3, 0, 4, 5, 6, 9, 7, 8, 10, 11, 12, 19, 13, 16, 14, 17, 15, 18};
-    return t[k];
-}
-__device__ __forceinline__ void lrf_terms20x2(float4 xi, float2 oxy, float2 ozq, float2* n) {
-    const float2 dxy = __fadd2_rn(make_float2(xi.x, xi.y), oxy);   // (dx, dy)
-    const float2 dzq = __fadd2_rn(make_float2(xi.z, xi.w), ozq);   // (dz, q)
-    const float dx = dxy.x, dy = dxy.y, dz = dzq.x, q = dzq.y;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float ri = rsqrtf(r2), ri2 = ri * ri;
-    const float qri = q * ri;
-    const float f0 = qri * ri2;
-    const float f1 = 3.f * f0 * ri2;
-    const float g = -5.f * f1 * ri2;
-    n[0] = __ffma2_rn(dxy, make_float2(-f0, -f0), n[0]);                 // n1 -= dx f0, n2 -= dy f0
-    n[1] = __ffma2_rn(dzq, make_float2(-f0, ri), n[1]);                  // n3 -= dz f0, n0 += q ri
-    const float2 axy = __fmul2_rn(dxy, make_float2(f1, f1));             // (ax, ay)
-    const float az = dz * f1;
-    n[2] = __ffma2_rn(make_float2(axy.x, axy.x), dxy, n[2]);            // n4 += ax dx, n5 += ax dy
-    n[3] = __ffma2_rn(make_float2(axy.x, az), make_float2(dz, dz), n[3]);  // n6 += ax dz, n9 += az dz
-    n[4] = __ffma2_rn(make_float2(axy.y, axy.y), make_float2(dy, dz), n[4]);   // n7 += ay dy, n8 += ay dz
-    const float2 gxy = __fmul2_rn(dxy, make_float2(g, g));               // (gx, gy)
-    const float gz = g * dz;
-    const float2 gxxyy = __fmul2_rn(gxy, dxy);                           // (gxx, gyy)
-    const float gzz = gz * dz, gxy_ = gxy.x * dy;
-    n[5] = __ffma2_rn(make_float2(gxxyy.x, gxxyy.x), dxy, n[5]);         // n10 += gxx dx, n11 += gxx dy
-    n[6] = __ffma2_rn(make_float2(gxxyy.x, gzz), make_float2(dz, dz), n[6]);   // n12 += gxx dz, n19 += gzz dz
-    n[7] = __ffma2_rn(make_float2(gxxyy.y, gxxyy.y), dxy, n[7]);         // n13 += gyy dx, n16 += gyy dy
-    n[8] = __ffma2_rn(make_float2(gxy_, gxxyy.y), make_float2(dz, dz), n[8]);  // n14 += gxy dz, n17 += gyy dz
-    n[9] = __ffma2_rn(make_float2(gzz, gzz), dxy, n[9]);                 // n15 += gzz dx, n18 += gzz dy
-}
-template <bool BOX>
-__global__ void __launch_bounds__(kLrfNB, 10) k_lrf_nbody(DevModel m, const DevState* __restrict__ states, Cut c,
-                                                          int nsplit) {
-    const Band bpp = band(c.rcpp2, c.fpp), bpw = band(c.rcpw2, c.fpw), bww = band(c.rcww2, c.fww),
-               blrf = band(c.rlrf2, c.flrf);
-    __shared__ int s_meta[kLrfGT];
-    __shared__ int s_off[kLrfGT + 1];
-    __shared__ float4 s_xs[kLrfGT];
-    __shared__ float4 s_xi[kLrfGT * kMaxGroup];
-    const DevState& s = states[blockIdx.y];
-    const double* __restrict__ x = s.x;
-    const float4* __restrict__ xq = s.xq;
-    double* __restrict__ lrf = s.lrf;
-    const int g2 = blockIdx.x * kLrfNB + threadIdx.x;
-    int s2 = -1;
-    bool act = g2 < m.ncgp;
-    if (act) {
-        s2 = group_dist_atom(m, g2);
-        act = !m.excl[s2];
-    }
-    const bool sol2 = g2 < m.ncgp_solute;
-    const Band rc_s = sol2 ? bpp : bpw, rc_w = sol2 ? bpw : bww;
-    float ccx = 0.f, ccy = 0.f, ccz = 0.f;
-    float4 x2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (act) {
-        const double* L = lrf + (size_t)g2 * kLrfLen;
-        ccx = (float)(L[0] - m.xpcent[0]);
-        ccy = (float)(L[1] - m.xpcent[1]);
-        ccz = (float)(L[2] - m.xpcent[2]);
-        x2 = xq[s2];
-    }
-    constexpr int NS = kLrfMom20 / 2;   // packed slots (lrf_slot)
-    float2 part[NS], hi[NS], lo[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) part[k] = hi[k] = lo[k] = make_float2(0.f, 0.f);
-    const float2 oxy0 = make_float2(-ccx, -ccy), ozq0 = make_float2(-ccz, 0.f);
-    // this block's range of source groups (blockIdx.z of nsplit)
-    const int gbeg = (int)((int64_t)m.nlrf_groups * blockIdx.z / nsplit);
-    const int gend = (int)((int64_t)m.nlrf_groups * (blockIdx.z + 1) / nsplit);
-    for (int t0 = gbeg; t0 < gend; t0 += kLrfGT) {   // block-uniform
-        const int ng = min(kLrfGT, gend - t0);
-        const int a_base = m.lrf_goff[t0];
-        const int na = m.lrf_goff[t0 + ng] - a_base;   // <= kLrfGT * kMaxGroup
-        __syncthreads();   // the previous tile is consumed
-        for (int k = threadIdx.x; k < ng; k += kLrfNB) {
-            int meta = m.lrf_gmeta[t0 + k];
-            s_meta[k] = meta;
-            s_xs[k] = xq[meta & 0x3fffffff];
-            s_off[k] = m.lrf_goff[t0 + k] - a_base;
-        }
-        if (threadIdx.x == 0) s_off[ng] = na;
-        for (int k = threadIdx.x; k < na; k += kLrfNB) s_xi[k] = xq[m.lrf_gatom[a_base + k]];
-        __syncthreads();
-        if (!act) continue;
-        for (int gi = 0; gi < ng; ++gi) {
-            const int meta = s_meta[gi], s1 = meta & 0x3fffffff;
-            const Band& rc2 = (meta >> 30) ? rc_s : rc_w;
-            if (BOX) {
-                if (s1 != s2 && lrf_pair_box(m, x2, s_xs[gi], rc2, blrf, x, s2, s1)) {
-                    const float3 sh = lrf_shift(m, s_xs[gi], ccx, ccy, ccz, x, s1, lrf + (size_t)g2 * kLrfLen);
-                    const float2 oxy = make_float2(-(ccx + sh.x), -(ccy + sh.y)), ozq = make_float2(-(ccz + sh.z), 0.f);
-                    const int k1 = s_off[gi + 1];
-                    for (int k = s_off[gi]; k < k1; ++k) lrf_terms20x2(s_xi[k], oxy, ozq, part);
-                }
-            } else if (s1 != s2 && lrf_pair(r2_f(x2, s_xs[gi]), rc2, blrf, x, s2, s1)) {
-                const int k1 = s_off[gi + 1];
-                for (int k = s_off[gi]; k < k1; ++k) lrf_terms20x2(s_xi[k], oxy0, ozq0, part);
-            }
-            if ((gi + 1) % kLrfFold == 0 || gi == ng - 1) {
-#pragma unroll
-                for (int k = 0; k < NS; ++k) {
-                    two_sum_fold(hi[k].x, lo[k].x, part[k].x);
-                    two_sum_fold(hi[k].y, lo[k].y, part[k].y);
-                }
-            }
-        }
-    }
-    if (!act) return;
-    double tot[kLrfMom20];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        tot[lrf_slot(2 * k)] = (double)hi[k].x + (double)lo[k].x;
-        tot[lrf_slot(2 * k + 1)] = (double)hi[k].y + (double)lo[k].y;
-    }
-    double* out = s.lrf_part + ((size_t)blockIdx.z * m.ncgp + g2) * kLrfMom20;
-#pragma unroll
-    for (int k = 0; k < kLrfMom20; ++k) out[k] = tot[k];
-}
-
-// The source ranges' moments of each target summed in range order, then
-// expanded into the record.
-__global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, int nsplit) {
-    const DevState& s = states[blockIdx.y];
-    const int g2 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g2 >= m.ncgp || m.excl[group_dist_atom(m, g2)]) return;
-    double tot[kLrfMom20];
-#pragma unroll
-    for (int k = 0; k < kLrfMom20; ++k) tot[k] = 0.0;
-    for (int z = 0; z < nsplit; ++z) {
-        const double* p = s.lrf_part + ((size_t)z * m.ncgp + g2) * kLrfMom20;
-#pragma unroll
-        for (int k = 0; k < kLrfMom20; ++k) tot[k] += p[k];
-    }
-    double m24[kLrfMom];
-    lrf_moments24(tot, m24);
-    lrf_expand(m24, s.lrf + (size_t)g2 * kLrfLen + 3);
-}
-
 // The 20 moment sums of one source atom at d = (dx, dy, dz) from the target's
 // centre, in the scaled vector e = d / r^2 and w = q / r:
 //   n[0] w   n[1..3] -w e   n[4..9] w e e (xx xy xz yy yz zz)
@@ -1028,6 +840,314 @@ __device__ __forceinline__ void lrf_scale20(double* n) {
     for (int k = 4; k < 10; ++k) n[k] *= 3.0;
 #pragma unroll
     for (int k = 10; k < kLrfMom20; ++k) n[k] *= -15.0;
+}
+
+// Mixed form: one thread per PAIR of target groups, the two in the halves of
+// packed FP32x2 arithmetic, so every packed instruction advances both targets
+// and no half has to be rearranged (the 38 operations of lrf_terms_e take 44
+// issue slots for two targets; one target per thread with its sums paired up
+// took about 45 for one).  A packed instruction holds the FMA pipe for two
+// cycles, so the pipe's 38 operations per term bound the kernel.
+//
+// The block's kLrfWarps warps hold the same 64 targets (lane: targets l and
+// l + 32) and each sums a range of its own of the source groups (the eligible
+// atoms of each charge group, in group order: lrf_gmeta / lrf_goff /
+// lrf_gatom); the cluster's blocks split the source groups further, so a
+// single window of 1,713 groups has 864 warps.  A warp stages kLrfTile source
+// groups at a time by asynchronous copies while it evaluates the tile before;
+// its lanes read the atoms as broadcasts.  Per (target pair, source group)
+// the group-pair classification runs once; a target whose pair is not far
+// gets r^2 = infinity, so its terms are exact zeros at no cost.
+//
+// A tile's sums run in FP32 and are then folded into a double-float
+// accumulator (Knuth's TwoSum: s = a + b, bb = s - a,
+// e = (a - (s - bb)) + (b - bb)) kept in shared memory, so the FP32 rounding
+// is kept to short runs.  At the end the cluster's ranges are added in
+// double-float in range order through distributed shared memory, and each
+// block expands its share of the targets: no partial sums in global memory,
+// no second kernel.  Ranges and tiles are fixed by the topology alone, so a
+// window's coefficients do not depend on the launch or the number of windows.
+// Alone: 51 windows of the 25 A sphere 1.30 -> 1.06 ms, 8 of a 34 A sphere
+// 1.85 -> 1.28 ms, one of 25 A 140 -> 70 us; the FMA pipe's operations alone
+// would take half of that, the rest is their latency at four warps per
+// scheduler.  Records as far from FP64 as before (2e-6 of their scale).
+constexpr int kLrfWarps = 4;
+constexpr int kLrfTgt = 64;    // targets per cluster
+constexpr int kLrfTile = kLrfTileGroups;   // source groups per staged tile and FP32 partial sum
+
+struct LrfSmem {   // of one warp; the staged atoms follow the blocks' warps
+    float2 hi[kLrfMom20][kWarp], lo[kLrfMom20][kWarp];
+    float4 xs[2][kLrfTile];
+    int end[2][kLrfTile];   // last atom + 1 of the group in the tile | solute flag << 30
+};
+constexpr int kLrfTot = kLrfMom20 + 4;   // totals of a target: the 20 moments, F0, U(3)
+__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
+// (hi, lo) += (p, pl) in double-float
+__device__ __forceinline__ void df_add(float& hi, float& lo, float p, float pl) {
+    const float sum = __fadd_rn(hi, p), bb = __fsub_rn(sum, hi);
+    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(sum, bb)), __fsub_rn(p, bb));
+    hi = sum;
+    lo = __fadd_rn(lo, __fadd_rn(pl, e));
+}
+// coefficient c (0..39) of the record from a target's totals: phi0, phi1(a),
+// phi2(a, b) = S2(ab) - delta_ab F0, phi3(a, b, c) = S3(abc) - delta_ab U(c) -
+// delta_ac U(b) - delta_bc U(a)
+__device__ __forceinline__ double lrf_coef(const double* n, int c) {
+    if (c < 4) return n[c];
+    if (c < 13) {
+        const int a = (c - 4) / 3, b = (c - 4) % 3, lo = min(a, b), hi = max(a, b);
+        return n[4 + lo * (5 - lo) / 2 + hi] - (a == b ? n[kLrfMom20] : 0.0);
+    }
+    const int a = (c - 13) / 9, b = (c - 13) / 3 % 3, d = (c - 13) % 3;
+    // S3 index by how many of the three are y and z
+    const int nyc = (a == 1) + (b == 1) + (d == 1), nzc = (a == 2) + (b == 2) + (d == 2);
+    const int idx[4][4] = {{10, 12, 15, 19}, {11, 14, 18, 0}, {13, 17, 0, 0}, {16, 0, 0, 0}};   // [y][z]
+    const double* U = n + kLrfMom20 + 1;
+    double v = n[idx[nyc][nzc]];
+    if (a == b) v -= U[d];
+    if (a == d) v -= U[b];
+    if (b == d) v -= U[a];
+    return v;
+}
+#ifndef QNB_LRF_U
+#define QNB_LRF_U 3
+#endif
+// 1/sqrt on the SFU with subnormal inputs taken as zero (a squared distance
+// below 1e-38 A^2): without it the compiler brackets each use with the
+// scaling of subnormals
+__device__ __forceinline__ float rsqrt_ftz(float v) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }   // exact product
+
+// the FP64 decision of a target and source group whose FP32 distance is
+// inside a decision band (or, in a box, whose lattice index is near a half)
+template <bool BOX>
+__device__ __noinline__ bool lrf_far_exact(const DevModel& m, const Cut& c, const double* __restrict__ x, int st, int s1,
+                                           bool sol, bool ss) {
+    const double rc2 = sol && ss ? c.rcpp2 : (sol != ss ? c.rcpw2 : c.rcww2);
+    if (BOX) return lrf_pair_box_exact(m, x, st, s1, rc2, c.rlrf2);
+    const double r2 = dist2_exact_atoms(x, st, s1);
+    return r2 > rc2 && r2 <= c.rlrf2;
+}
+
+template <bool BOX>
+__global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, const DevState* __restrict__ states,
+                                                                    Cut c, int tile_atoms) {
+    extern __shared__ __align__(16) unsigned char lrf_smem[];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    LrfSmem* sm = reinterpret_cast<LrfSmem*>(lrf_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    LrfSmem& S = sm[warp];
+    float4* s_xi = reinterpret_cast<float4*>(sm + kLrfWarps) + (size_t)warp * 2 * tile_atoms;   // [2][tile_atoms]
+    const DevState& s = states[blockIdx.y];
+    const double* __restrict__ x = s.x;
+    const float4* __restrict__ xq = s.xq;
+    double* __restrict__ lrf = s.lrf;
+    // this lane's two targets, and the decision bands of its cut-offs against
+    // solute and water sources
+    int st[2];
+    bool act[2], sol[2];
+    float4 xt[2];
+    float cc[2][3];
+    CutBand bs[2], bw[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int g = blockIdx.x * kLrfTgt + h * kWarp + lane;
+        act[h] = g < m.ncgp;
+        st[h] = act[h] ? group_dist_atom(m, g) : 0;
+        if (act[h]) act[h] = !m.excl[st[h]];
+        sol[h] = g < m.ncgp_solute;
+        bs[h] = sol[h] ? c.fpp : c.fpw;
+        bw[h] = sol[h] ? c.fpw : c.fww;
+        if (!act[h]) bs[h].hi = bw[h].hi = bs[h].lo = bw[h].lo = INFINITY;   // never far
+        xt[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+        cc[h][0] = cc[h][1] = cc[h][2] = 0.f;
+        if (act[h]) {
+            const double* L = lrf + (size_t)g * kLrfLen;
+            xt[h] = xq[st[h]];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) cc[h][k] = (float)(L[k] - m.xpcent[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kLrfMom20; ++k) S.hi[k][lane] = S.lo[k][lane] = f2(0.f);
+    const float2 nx = make_float2(-cc[0][0], -cc[1][0]), ny = make_float2(-cc[0][1], -cc[1][1]),
+                 nz = make_float2(-cc[0][2], -cc[1][2]);
+    // this warp's range of source groups
+    const int z = blockIdx.z * kLrfWarps + warp, nz_all = gridDim.z * kLrfWarps;
+    const int gbeg = (int)((int64_t)m.nlrf_groups * z / nz_all), gend = (int)((int64_t)m.nlrf_groups * (z + 1) / nz_all);
+    // stages tile t0's atoms, switch atoms and group ends into buffer b
+    auto stage = [&](int t0, int b) {
+        const int ng = min(kLrfTile, gend - t0);
+        const int off = m.lrf_goff[t0 + min(lane, ng)], base = __shfl_sync(kFull, off, 0);
+        const int na = __shfl_sync(kFull, off, ng) - base;   // <= tile_atoms
+        const int end = __shfl_down_sync(kFull, off, 1) - base;
+        if (lane < ng) {
+            const int meta = m.lrf_gmeta[t0 + lane];
+            cp_async16(&S.xs[b][lane], xq + (meta & 0x3fffffff));
+            S.end[b][lane] = end | (meta & (1 << 30));
+        }
+        for (int u = lane; u < na; u += kWarp) cp_async16(s_xi + b * tile_atoms + u, xq + m.lrf_gatom[base + u]);
+    };
+    if (gbeg < gend) stage(gbeg, 0);
+    cp_async_commit();
+    int b = 0;
+    for (int t0 = gbeg; t0 < gend; t0 += kLrfTile, b ^= 1) {   // warp-uniform
+        if (t0 + kLrfTile < gend) stage(t0 + kLrfTile, b ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncwarp();
+        const int ng = min(kLrfTile, gend - t0);
+        const float4* xi = s_xi + b * tile_atoms;
+        float2 n[kLrfMom20];
+#pragma unroll
+        for (int k = 0; k < kLrfMom20; ++k) n[k] = f2(0.f);
+        for (int gi = 0, k1 = 0; gi < ng; ++gi) {
+            const int k0 = k1, e = S.end[b][gi];
+            const float4 xs = S.xs[b][gi];
+            const bool ss = (e >> 30) != 0;   // solute source
+            k1 = e & 0x3fffffff;
+            bool far[2], band[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float dx = xs.x - xt[h].x, dy = xs.y - xt[h].y, dz = xs.z - xt[h].z;
+                bool half = false;
+                if (BOX) {   // minimum image
+                    const float tx = dx * m.inv_boxlf[0], ty = dy * m.inv_boxlf[1], tz = dz * m.inv_boxlf[2];
+                    half = near_half(tx) || near_half(ty) || near_half(tz);
+                    dx = m.boxlf[0] * roundf(tx) - dx, dy = m.boxlf[1] * roundf(ty) - dy, dz = m.boxlf[2] * roundf(tz) - dz;
+                }
+                const float r2 = dx * dx + dy * dy + dz * dz;
+                const float lo = ss ? bs[h].lo : bw[h].lo, hi = ss ? bs[h].hi : bw[h].hi;
+                far[h] = r2 > hi && r2 < c.flrf.lo && !half;
+                band[h] = ((r2 >= lo && r2 <= c.flrf.hi) || half) && !far[h] && act[h];
+            }
+            if (band[0] || band[1]) {   // rare
+                const int s1 = m.lrf_gmeta[t0 + gi] & 0x3fffffff;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (band[h]) far[h] = lrf_far_exact<BOX>(m, c, x, st[h], s1, sol[h], ss);
+            }
+            if (!(far[0] || far[1])) continue;
+            const float2 far2 = make_float2(far[0] ? 0.f : INFINITY, far[1] ? 0.f : INFINITY);
+            float2 ox = nx, oy = ny, oz = nz;
+            if (BOX) {
+                float3 sh[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    sh[h] = far[h] ? lrf_shift(m, xs, cc[h][0], cc[h][1], cc[h][2], x, m.lrf_gmeta[t0 + gi] & 0x3fffffff,
+                                               lrf + (size_t)(blockIdx.x * kLrfTgt + h * kWarp + lane) * kLrfLen)
+                                   : make_float3(0.f, 0.f, 0.f);
+                ox = make_float2(-(cc[0][0] + sh[0].x), -(cc[1][0] + sh[1].x));
+                oy = make_float2(-(cc[0][1] + sh[0].y), -(cc[1][1] + sh[1].y));
+                oz = make_float2(-(cc[0][2] + sh[0].z), -(cc[1][2] + sh[1].z));
+            }
+            auto term = [&](const float4 a) {   // the terms of lrf_terms_e
+                const float2 dx = make_float2(a.x + ox.x, a.x + ox.y), dy = make_float2(a.y + oy.x, a.y + oy.y),
+                             dz = make_float2(a.z + oz.x, a.z + oz.y);
+                const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, far2)));
+                const float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y)), ri2 = __fmul2_rn(ri, ri);
+                const float2 w = make_float2(a.w * ri.x, a.w * ri.y);
+                const float2 ex = __fmul2_rn(dx, ri2), ey = __fmul2_rn(dy, ri2), ez = __fmul2_rn(dz, ri2);
+                const float2 ax = __fmul2_rn(w, ex), ay = __fmul2_rn(w, ey), az = __fmul2_rn(w, ez);
+                const float2 bxx = __fmul2_rn(ax, ex), byy = __fmul2_rn(ay, ey), bzz = __fmul2_rn(az, ez),
+                             bxy = __fmul2_rn(ax, ey);
+                // every sum takes its last product unrounded, although the
+                // next order needs it rounded as well
+                n[0] = make_float2(fmaf(a.w, ri.x, n[0].x), fmaf(a.w, ri.y, n[0].y));
+                n[1] = __ffma2_rn(w, ex, n[1]);   // negated in the total
+                n[2] = __ffma2_rn(w, ey, n[2]);
+                n[3] = __ffma2_rn(w, ez, n[3]);
+                n[4] = __ffma2_rn(ax, ex, n[4]);
+                n[5] = __ffma2_rn(ax, ey, n[5]);
+                n[6] = __ffma2_rn(ax, ez, n[6]);
+                n[7] = __ffma2_rn(ay, ey, n[7]);
+                n[8] = __ffma2_rn(ay, ez, n[8]);
+                n[9] = __ffma2_rn(az, ez, n[9]);
+                n[10] = __ffma2_rn(bxx, ex, n[10]);
+                n[11] = __ffma2_rn(bxx, ey, n[11]);
+                n[12] = __ffma2_rn(bxx, ez, n[12]);
+                n[13] = __ffma2_rn(byy, ex, n[13]);
+                n[14] = __ffma2_rn(bxy, ez, n[14]);
+                n[15] = __ffma2_rn(bzz, ex, n[15]);
+                n[16] = __ffma2_rn(byy, ey, n[16]);
+                n[17] = __ffma2_rn(byy, ez, n[17]);
+                n[18] = __ffma2_rn(bzz, ey, n[18]);
+                n[19] = __ffma2_rn(bzz, ez, n[19]);
+            };
+            // three atoms at a time (a water, most of a solute group): their
+            // dependent chains overlap
+            int k = k0;
+            for (; k + QNB_LRF_U <= k1; k += QNB_LRF_U) {
+#pragma unroll
+                for (int u = 0; u < QNB_LRF_U; ++u) term(xi[k + u]);
+            }
+            for (; k < k1; ++k) term(xi[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kLrfMom20; ++k) {   // TwoSum fold
+            const float2 hi = S.hi[k][lane], sum = __fadd2_rn(hi, n[k]), bb = fsub2(sum, hi);
+            const float2 e = __fadd2_rn(fsub2(hi, fsub2(sum, bb)), fsub2(n[k], bb));
+            S.hi[k][lane] = sum;
+            S.lo[k][lane] = __fadd2_rn(S.lo[k][lane], e);
+        }
+        __syncwarp();   // buffer b is refilled in the next iteration
+    }
+    cp_async_wait<0>();
+    // the block's warps in order, into warp 0's accumulators
+    __syncthreads();
+    for (int v = threadIdx.x; v < kLrfMom20 * kWarp; v += blockDim.x) {
+        float2 h = (&sm[0].hi[0][0])[v], l = (&sm[0].lo[0][0])[v];
+#pragma unroll
+        for (int w = 1; w < kLrfWarps; ++w) {
+            const float2 h2 = (&sm[w].hi[0][0])[v], l2 = (&sm[w].lo[0][0])[v];
+            df_add(h.x, l.x, h2.x, l2.x);
+            df_add(h.y, l.y, h2.y, l2.y);
+        }
+        (&sm[0].hi[0][0])[v] = h;
+        (&sm[0].lo[0][0])[v] = l;
+    }
+    cluster.sync();
+    // the other blocks' sums of this block's share of the targets, in rank
+    // order, all loads in flight together
+    double* tot = reinterpret_cast<double*>(sm + kLrfWarps);   // the staging space: [share][kLrfTot]
+    const int nb = gridDim.z, share = kLrfTgt / nb, tg0 = blockIdx.z * share;
+    for (int v = threadIdx.x; v < share * kLrfMom20; v += blockDim.x) {
+        const int t = tg0 + v / kLrfMom20, k = v % kLrfMom20, half = t / kWarp, l = t % kWarp;
+        float2 h[kLrfClusterMax], o[kLrfClusterMax];
+#pragma unroll
+        for (int r = 0; r < kLrfClusterMax; ++r)
+            if (r < nb) {
+                const LrfSmem* R = cluster.map_shared_rank(sm, r);
+                h[r] = R->hi[k][l], o[r] = R->lo[k][l];
+            }
+        float hi = 0.f, lo = 0.f;
+#pragma unroll
+        for (int r = 0; r < kLrfClusterMax; ++r)
+            if (r < nb) df_add(hi, lo, half ? h[r].y : h[r].x, half ? o[r].y : o[r].x);
+        const double d = (double)hi + (double)lo;
+        tot[(t - tg0) * kLrfTot + k] = k == 0 ? d : (k < 4 ? -d : (k < 10 ? 3.0 * d : -15.0 * d));
+    }
+    __syncthreads();
+    for (int v = threadIdx.x; v < share * 4; v += blockDim.x) {   // F0 and U(c) from the traces
+        const int q = v % 4;
+        double* n = tot + v / 4 * kLrfTot;
+        const int i0 = q == 0 ? 4 : 9 + q, i1 = q == 0 ? 7 : (q == 1 ? 13 : (q == 2 ? 16 : 17)),
+                  i2 = q == 0 ? 9 : (q == 1 ? 15 : (q == 2 ? 18 : 19));
+        n[kLrfMom20 + q] = (n[i0] + n[i1] + n[i2]) / (q == 0 ? 3.0 : 5.0);
+    }
+    __syncthreads();
+    // the 40 coefficients of a target by 40 threads (lrf_coef)
+    for (int v = threadIdx.x; v < share * 40; v += blockDim.x) {
+        const int t = v / 40, g = blockIdx.x * kLrfTgt + tg0 + t;
+        if (g < m.ncgp && !m.excl[group_dist_atom(m, g)])
+            lrf[(size_t)g * kLrfLen + 3 + v % 40] = lrf_coef(tot + t * kLrfTot, v % 40);
+    }
+    cluster.sync();   // no block leaves while another reads its shared memory
 }
 
 // FP64 form: one warp per target group reads the source atoms straight from
@@ -3081,13 +3201,6 @@ __device__ __forceinline__ TypeTab stage_types(const DevModel& m, float4* sh) {
 // chunk instead of once per loop iteration.  Row capacities are multiples of
 // 4 entries, so every row starts on a 16-byte boundary and a chunk rounded up
 // to whole 16-byte units stays inside its row.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 constexpr int kRowChunk = 128;   // entries per prefetched chunk
 
 // solute group rows: pp (partner atoms with exclusion / 1-4 kinds) and pw
@@ -3704,6 +3817,26 @@ void launch_build_qp(const Launch& L, const uint8_t* qnear, double rcq2) {
     if (L.m.ncgp_solute == 0 || L.m.nqat == 0) return;
     k_build_qp<<<dim3(1, L.nwin), 1024, 0, L.st>>>(L.m, L.ds, qnear, rcq2);
 }
+namespace {
+int launch_lrf_pairs(const Launch& L, const Cut& c, int nz, int tile_atoms, size_t smem) {
+    auto kern = L.m.box ? k_lrf_pairs<true> : k_lrf_pairs<false>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = nz;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((L.m.ncgp + kLrfTgt - 1) / kLrfTgt, L.nwin, nz);
+    cfg.blockDim = dim3(kLrfWarps * kWarp);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = L.st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, L.m, L.ds, c, tile_atoms);
+    return 1;
+}
+}  // namespace
+
 int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src) {
     if (L.m.any_atom && L.m.box) {
         k_lrf_accumulate_any_box<<<grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds, c);
@@ -3716,16 +3849,16 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
         return 1;
     }
     if (mixed) {
-        // source ranges of at least one staged tile each; the split depends on
-        // the topology only, so a window's coefficients are the same in a
-        // batch of any size (51 windows of a 1,400-source-group system:
-        // 8 ranges, about 9 waves of resident target threads)
-        const int nsplit = std::min(kLrfSplitMax, std::max(1, L.m.nlrf_groups / kLrfGT));
-        dim3 g((L.m.ncgp + kLrfNB - 1) / kLrfNB, L.nwin, nsplit);
-        if (L.m.box) k_lrf_nbody<true><<<g, kLrfNB, 0, L.st>>>(L.m, L.ds, c, nsplit);
-        else k_lrf_nbody<false><<<g, kLrfNB, 0, L.st>>>(L.m, L.ds, c, nsplit);
-        k_lrf_combine<<<dim3((L.m.ncgp + 127) / 128, L.nwin), 128, 0, L.st>>>(L.m, L.ds, nsplit);
-        return 2;
+        // blocks per cluster: ranges of at least one tile per warp, the split
+        // set by the topology only, so a window's coefficients are the same in
+        // a batch of any size.  At most 4: 8 sped up a single window (R25: 74
+        // -> 54 us) and slowed 51 windows (1,100 -> 1,240 us), 2 the reverse
+        // (130 and 1,085 us)
+        int nz = 1;
+        while (nz < kLrfClusterMax && L.m.nlrf_groups >= 2 * nz * kLrfWarps * kLrfTile) nz *= 2;
+        const int tile_atoms = std::max(96 / nz, (L.m.lrf_tile_atoms + 3) & ~3);   // 96 / nz: the totals' space
+        const size_t smem = kLrfWarps * (sizeof(LrfSmem) + 2 * tile_atoms * sizeof(float4));
+        return launch_lrf_pairs(L, c, nz, tile_atoms, smem);
     }
     dim3 g = grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin);
     if (L.m.box) k_lrf_accumulate64<true><<<g, 128, 0, L.st>>>(L.m, L.ds, c, lrf_src);
@@ -3748,27 +3881,26 @@ int box_cells(const DevModel& m, const Cut& c, int* n) {
     }
     return n[0] >= 5 && n[1] >= 5 && n[2] >= 5;
 }
+// the row build's cell grid (sphere with switch atoms; box with 5 cells per
+// edge); otherwise the rows take every candidate and nothing is launched
+int launch_bin_cells(const Launch& L, const Cut& c) {
+    if (L.m.ncgp_solute + L.m.nwat == 0 || (L.m.any_atom && !L.m.box)) return 0;
+    int n[3] = {0, 0, 0};
+    if (L.m.box && !box_cells(L.m, c, n)) return 0;
+    k_bin_cells<<<L.nwin, 1024, 0, L.st>>>(L.m, L.ds, L.m.box ? 0.f : (float)(1.0 / cell_edge(c)),
+                                           make_int3(n[0], n[1], n[2]));
+    return 1;
+}
 int launch_build_rows(const Launch& L, const Cut& c) {
     int nrows = L.m.ncgp_solute + L.m.nwat;
     if (nrows == 0) return 0;
     dim3 g = grid_for((int64_t)nrows * 32, 128, L.tu.v[T_BUILD], L.nwin);
-    if (L.m.box) {   // periodic box (switch atoms): minimum-image tests, wrapped stencil
-        int n[3];
-        if (!box_cells(L.m, c, n)) {   // fewer than 5 cells per edge: every unit is a candidate
-            k_build_rows<false, true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
-            return 1;
-        }
-        k_bin_cells<<<L.nwin, 1024, 0, L.st>>>(L.m, L.ds, 0.f, make_int3(n[0], n[1], n[2]));
-        k_build_rows<true, true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
-        return 2;
-    }
-    if (L.m.any_atom) {   // any-atom group tests: every group and water is a candidate
-        k_build_rows<false, false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
-        return 1;
-    }
-    k_bin_cells<<<L.nwin, 1024, 0, L.st>>>(L.m, L.ds, (float)(1.0 / cell_edge(c)), make_int3(0, 0, 0));
-    k_build_rows<true, false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
-    return 2;
+    int n[3];
+    if (L.m.box && box_cells(L.m, c, n)) k_build_rows<true, true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
+    else if (L.m.box) k_build_rows<false, true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);   // every unit is a candidate
+    else if (L.m.any_atom) k_build_rows<false, false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
+    else k_build_rows<true, false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
+    return 1;
 }
 int lj_smem(const DevModel& m) {
     return m.natyps <= kMaxTypesShared ? (int)(m.natyps * m.natyps * sizeof(float4)) : 0;

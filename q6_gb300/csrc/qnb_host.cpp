@@ -502,6 +502,14 @@ int build_model(qnb_context* c, const qnb_topology* t) {
         if (!gallq[g]) c->maxg = std::max(c->maxg, gslot[g + 1] - gslot[g]);
     }
     TRY(c->upload((uint8_t**)&m.gallq, gallq));
+    std::vector<int> gnq_off{0}, gnq_atom;
+    for (int g = 0; g < t->ncgp_solute; ++g) {
+        for (int a = gslot[g]; a < gslot[g + 1]; ++a)
+            if (iqatom[gatom[a]] < 0) gnq_atom.push_back(gatom[a]);
+        gnq_off.push_back((int)gnq_atom.size());
+    }
+    TRY(c->upload((int**)&m.gnq_off, gnq_off));
+    TRY(c->upload((int**)&m.gnq_atom, gnq_atom));
     // must agree with k_rows_solute's template choice (MAXG <= 8)
     m.type_in_entry = (c->maxg <= 8 && t->natyps <= 0xffff) ? 1 : 0;
     struct SG {
@@ -1242,7 +1250,7 @@ int build_lists(qnb_context* c, const Cut& cut, int nw) {
                 CU(cudaStreamWaitEvent(c->stream2, c->ev_fork, 0));
                 L2.st = c->stream2;
             }
-            timed_on(c, L2.st, K_LRF_BUILD, [&] { nl += launch_lrf_accumulate(L2, cut, c->mixed, c->d_lrf_src); });
+            timed_on(c, L2.st, K_LRF_BUILD, [&] { nl += launch_lrf_accumulate(L2, cut, c->mixed, c->d_lrf_src, c->md_ready); });
             if (!behind) CU(cudaEventRecord(c->ev_join, c->stream2));
             return QNB_OK;
         };
@@ -2559,6 +2567,9 @@ int qnb_md_init(qnb_context* c, const qnb_md_params* p, const double* mass, int3
     TRY(c->alloc(&c->md_rec, (size_t)kMdChunk * c->nwin * kMdRec));
     c->md_rec_steps = kMdChunk;
     CU(cudaMallocHost((void**)&c->h_md_rec, sizeof(double) * kMdChunk * c->nwin * kMdRec));
+    if (c->mixed && c->use_lrf)
+        for (int w = 0; w < c->nwin; ++w)
+            TRY(c->alloc(&c->st[w].lrf_part, (size_t)kLrfSplitMax * std::max(1, c->ncgp) * kLrfMoments));
     // restrain_solvent of an MD step reads the window's Tfree on the device
     for (int w = 0; w < c->nwin; ++w) c->st[w].md_tfree = &md.win[w].tfree;
     TRY(upload_states(c));

@@ -14,6 +14,7 @@ constexpr int kMaxStates = 8;   // FEP states
 constexpr int kMaxShell = 16;   // water polarisation shells
 constexpr int kLrfLen = 43;     // cgp_cent(3) phi0 phi1(3) phi2(9) phi3(27)
 constexpr int kLrfMoments = 24; // symmetric moments the LRF accumulation sums per target group
+constexpr int kLrfSplitMax = 8;     // source ranges of the mixed form's accumulation in MD contexts
 constexpr int kLrfTileGroups = 16;  // source groups it stages at a time
 constexpr int kLrfClusterMax = 4;   // blocks per cluster of the mixed form's LRF accumulation
 constexpr double kFix = 4294967296.0;   // 2^32: fixed-point quantum of forces/energies
@@ -132,6 +133,8 @@ struct DevModel {
     // rule: A = a_i a_j, B = b_i b_j)
     int geom;
     const ulonglong2* gtmask;           // [ncgp_solute] types 0-63 (x) and 64-127 (y)
+    const int* gnq_off;                 // [ncgp_solute+1] non-Q atoms of each solute group
+    const int* gnq_atom;
     const uint8_t* gallq;               // [ncgp_solute] 1: every atom of the group is a Q atom (no pair row)
     const float2* ljf1;                 // [natom]
     // LRF sources grouped by charge group (mixed form's accumulation):
@@ -187,6 +190,7 @@ struct DevState {
     unsigned long long* efix;  // [kNumE] fixed-point energies (mixed form)
     double* lambda;      // [S]
     double* lrf;         // [ncgp*43]
+    double* lrf_part;    // mixed form, MD contexts: [kLrfSplitMax][ncgp][kLrfMoments] LRF moments per source range
     int* cnt;            // [C_NUM] list sizes (device-maintained)
     int2* ww; int64_t cap_ww;      // water pairs (iw, jw), iw < jw
     int2* pw; int64_t cap_pw;      // (solute atom, water)
@@ -278,7 +282,8 @@ void launch_build_pw(const Launch& L, const Cut& c);
 void launch_build_pp(const Launch& L, const Cut& c);
 void launch_build_qp(const Launch& L, const uint8_t* qnear, double rcq2);
 void launch_build_qw(const Launch& L, const Cut& c);
-int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src);
+// keep_order: the mixed form's summation order of MD contexts (needs DevState::lrf_part)
+int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src, int keep_order);
 
 int launch_bin_cells(const Launch& L, const Cut& c);
 int launch_build_rows(const Launch& L, const Cut& c);   // after launch_bin_cells

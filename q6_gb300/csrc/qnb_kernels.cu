@@ -59,6 +59,17 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// 1/sqrt on the SFU with subnormal inputs taken as zero (a squared distance
+// below 1e-38 A^2): without it the compiler brackets each use with the
+// scaling of subnormals
+__device__ __forceinline__ float rsqrt_ftz(float v) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }   // exact product
+
 // warp-aggregated append: returns this lane's first slot (valid when n > 0)
 __device__ __forceinline__ int warp_append(int* counter, int n) {
     int lane = threadIdx.x & 31;
@@ -842,6 +853,183 @@ __device__ __forceinline__ void lrf_scale20(double* n) {
     for (int k = 10; k < kLrfMom20; ++k) n[k] *= -15.0;
 }
 
+// Mixed form of contexts with a running integrator (qnb_md_init): one thread
+// per target group, the summation that their trajectories were made with.  A
+// trajectory amplifies rounding -- watpol's order of two waters or a shell
+// boundary is crossed one step earlier or later -- so k_lrf_pairs, as near to
+// FP64 as this kernel, left a 25-step run by up to 1e-4 of the velocities in 2
+// of 14 systems; a list build every 25 steps gains too little there.  The blocks stage
+// the LRF source groups (the eligible atoms of each charge group, in group
+// order: lrf_gmeta / lrf_goff / lrf_gatom) in shared memory, kLrfGT groups
+// per tile, and every thread reads them as broadcasts.  The group-pair
+// classification runs once per (target, source group); the source group's
+// atoms then add their terms.  Each thread's 20 moment sums run
+// in FP32 over at most kLrfFold source groups and are then folded into a
+// double-float accumulator with Knuth's TwoSum (s = a + b, bb = s - a,
+// e = (a - (s - bb)) + (b - bb)), so the FP32 rounding of the sums is kept
+// to short runs.  The source groups are split into nsplit ranges
+// (blockIdx.z, the split fixed by the topology) whose moments
+// k_lrf_combine adds in range order: each target's order of terms is fixed,
+// so its coefficients do not depend on the launch or the number of windows.
+constexpr int kLrfNB = 64;     // targets per block
+constexpr int kLrfGT = 64;     // source groups per staged tile
+constexpr int kLrfFold = 8;    // source groups per FP32 partial sum
+
+__device__ __forceinline__ void two_sum_fold(float& hi, float& lo, float& p) {
+    float s = __fadd_rn(hi, p);
+    float bb = __fsub_rn(s, hi);
+    float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(p, bb));
+    hi = s;
+    lo = __fadd_rn(lo, e);
+    p = 0.f;
+}
+
+// Its 20 moments in packed FP32x2 arithmetic: the source
+// atom's (x, y) and (z, q) arrive as register pairs from the staged float4,
+// and the 20 sums are held as 10 pairs, so 10 FFMA2 replace 20 FFMA.  Each
+// sum gets the same products in the same order as in lrf_terms20.  Slots
+// (lrf_slot):
+// (n1,n2) (n3,n0) (n4,n5) (n6,n9) (n7,n8) (n10,n11) (n12,n19) (n13,n16)
+// (n14,n17) (n15,n18).
+__host__ __device__ constexpr int lrf_slot(int k) {
+    constexpr int t[kLrfMom20] = {1, 2, 3, 0, 4, 5, 6, 9, 7, 8, 10, 11, 12, 19, 13, 16, 14, 17, 15, 18};
+    return t[k];
+}
+__device__ __forceinline__ void lrf_terms20x2(float4 xi, float2 oxy, float2 ozq, float2* n) {
+    const float2 dxy = __fadd2_rn(make_float2(xi.x, xi.y), oxy);   // (dx, dy)
+    const float2 dzq = __fadd2_rn(make_float2(xi.z, xi.w), ozq);   // (dz, q)
+    const float dx = dxy.x, dy = dxy.y, dz = dzq.x, q = dzq.y;
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float ri = rsqrtf(r2), ri2 = ri * ri;
+    const float qri = q * ri;
+    const float f0 = qri * ri2;
+    const float f1 = 3.f * f0 * ri2;
+    const float g = -5.f * f1 * ri2;
+    n[0] = __ffma2_rn(dxy, make_float2(-f0, -f0), n[0]);                 // n1 -= dx f0, n2 -= dy f0
+    n[1] = __ffma2_rn(dzq, make_float2(-f0, ri), n[1]);                  // n3 -= dz f0, n0 += q ri
+    const float2 axy = __fmul2_rn(dxy, make_float2(f1, f1));             // (ax, ay)
+    const float az = dz * f1;
+    n[2] = __ffma2_rn(make_float2(axy.x, axy.x), dxy, n[2]);            // n4 += ax dx, n5 += ax dy
+    n[3] = __ffma2_rn(make_float2(axy.x, az), make_float2(dz, dz), n[3]);  // n6 += ax dz, n9 += az dz
+    n[4] = __ffma2_rn(make_float2(axy.y, axy.y), make_float2(dy, dz), n[4]);   // n7 += ay dy, n8 += ay dz
+    const float2 gxy = __fmul2_rn(dxy, make_float2(g, g));               // (gx, gy)
+    const float gz = g * dz;
+    const float2 gxxyy = __fmul2_rn(gxy, dxy);                           // (gxx, gyy)
+    const float gzz = gz * dz, gxy_ = gxy.x * dy;
+    n[5] = __ffma2_rn(make_float2(gxxyy.x, gxxyy.x), dxy, n[5]);         // n10 += gxx dx, n11 += gxx dy
+    n[6] = __ffma2_rn(make_float2(gxxyy.x, gzz), make_float2(dz, dz), n[6]);   // n12 += gxx dz, n19 += gzz dz
+    n[7] = __ffma2_rn(make_float2(gxxyy.y, gxxyy.y), dxy, n[7]);         // n13 += gyy dx, n16 += gyy dy
+    n[8] = __ffma2_rn(make_float2(gxy_, gxxyy.y), make_float2(dz, dz), n[8]);  // n14 += gxy dz, n17 += gyy dz
+    n[9] = __ffma2_rn(make_float2(gzz, gzz), dxy, n[9]);                 // n15 += gzz dx, n18 += gzz dy
+}
+template <bool BOX>
+__global__ void __launch_bounds__(kLrfNB, 10) k_lrf_nbody(DevModel m, const DevState* __restrict__ states, Cut c,
+                                                          int nsplit) {
+    const Band bpp = band(c.rcpp2, c.fpp), bpw = band(c.rcpw2, c.fpw), bww = band(c.rcww2, c.fww),
+               blrf = band(c.rlrf2, c.flrf);
+    __shared__ int s_meta[kLrfGT];
+    __shared__ int s_off[kLrfGT + 1];
+    __shared__ float4 s_xs[kLrfGT];
+    __shared__ float4 s_xi[kLrfGT * kMaxGroup];
+    const DevState& s = states[blockIdx.y];
+    const double* __restrict__ x = s.x;
+    const float4* __restrict__ xq = s.xq;
+    double* __restrict__ lrf = s.lrf;
+    const int g2 = blockIdx.x * kLrfNB + threadIdx.x;
+    int s2 = -1;
+    bool act = g2 < m.ncgp;
+    if (act) {
+        s2 = group_dist_atom(m, g2);
+        act = !m.excl[s2];
+    }
+    const bool sol2 = g2 < m.ncgp_solute;
+    const Band rc_s = sol2 ? bpp : bpw, rc_w = sol2 ? bpw : bww;
+    float ccx = 0.f, ccy = 0.f, ccz = 0.f;
+    float4 x2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (act) {
+        const double* L = lrf + (size_t)g2 * kLrfLen;
+        ccx = (float)(L[0] - m.xpcent[0]);
+        ccy = (float)(L[1] - m.xpcent[1]);
+        ccz = (float)(L[2] - m.xpcent[2]);
+        x2 = xq[s2];
+    }
+    constexpr int NS = kLrfMom20 / 2;   // packed slots (lrf_slot)
+    float2 part[NS], hi[NS], lo[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) part[k] = hi[k] = lo[k] = make_float2(0.f, 0.f);
+    const float2 oxy0 = make_float2(-ccx, -ccy), ozq0 = make_float2(-ccz, 0.f);
+    // this block's range of source groups (blockIdx.z of nsplit)
+    const int gbeg = (int)((int64_t)m.nlrf_groups * blockIdx.z / nsplit);
+    const int gend = (int)((int64_t)m.nlrf_groups * (blockIdx.z + 1) / nsplit);
+    for (int t0 = gbeg; t0 < gend; t0 += kLrfGT) {   // block-uniform
+        const int ng = min(kLrfGT, gend - t0);
+        const int a_base = m.lrf_goff[t0];
+        const int na = m.lrf_goff[t0 + ng] - a_base;   // <= kLrfGT * kMaxGroup
+        __syncthreads();   // the previous tile is consumed
+        for (int k = threadIdx.x; k < ng; k += kLrfNB) {
+            int meta = m.lrf_gmeta[t0 + k];
+            s_meta[k] = meta;
+            s_xs[k] = xq[meta & 0x3fffffff];
+            s_off[k] = m.lrf_goff[t0 + k] - a_base;
+        }
+        if (threadIdx.x == 0) s_off[ng] = na;
+        for (int k = threadIdx.x; k < na; k += kLrfNB) s_xi[k] = xq[m.lrf_gatom[a_base + k]];
+        __syncthreads();
+        if (!act) continue;
+        for (int gi = 0; gi < ng; ++gi) {
+            const int meta = s_meta[gi], s1 = meta & 0x3fffffff;
+            const Band& rc2 = (meta >> 30) ? rc_s : rc_w;
+            if (BOX) {
+                if (s1 != s2 && lrf_pair_box(m, x2, s_xs[gi], rc2, blrf, x, s2, s1)) {
+                    const float3 sh = lrf_shift(m, s_xs[gi], ccx, ccy, ccz, x, s1, lrf + (size_t)g2 * kLrfLen);
+                    const float2 oxy = make_float2(-(ccx + sh.x), -(ccy + sh.y)), ozq = make_float2(-(ccz + sh.z), 0.f);
+                    const int k1 = s_off[gi + 1];
+                    for (int k = s_off[gi]; k < k1; ++k) lrf_terms20x2(s_xi[k], oxy, ozq, part);
+                }
+            } else if (s1 != s2 && lrf_pair(r2_f(x2, s_xs[gi]), rc2, blrf, x, s2, s1)) {
+                const int k1 = s_off[gi + 1];
+                for (int k = s_off[gi]; k < k1; ++k) lrf_terms20x2(s_xi[k], oxy0, ozq0, part);
+            }
+            if ((gi + 1) % kLrfFold == 0 || gi == ng - 1) {
+#pragma unroll
+                for (int k = 0; k < NS; ++k) {
+                    two_sum_fold(hi[k].x, lo[k].x, part[k].x);
+                    two_sum_fold(hi[k].y, lo[k].y, part[k].y);
+                }
+            }
+        }
+    }
+    if (!act) return;
+    double tot[kLrfMom20];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        tot[lrf_slot(2 * k)] = (double)hi[k].x + (double)lo[k].x;
+        tot[lrf_slot(2 * k + 1)] = (double)hi[k].y + (double)lo[k].y;
+    }
+    double* out = s.lrf_part + ((size_t)blockIdx.z * m.ncgp + g2) * kLrfMom20;
+#pragma unroll
+    for (int k = 0; k < kLrfMom20; ++k) out[k] = tot[k];
+}
+
+// The source ranges' moments of each target summed in range order, then
+// expanded into the record.
+__global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, int nsplit) {
+    const DevState& s = states[blockIdx.y];
+    const int g2 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g2 >= m.ncgp || m.excl[group_dist_atom(m, g2)]) return;
+    double tot[kLrfMom20];
+#pragma unroll
+    for (int k = 0; k < kLrfMom20; ++k) tot[k] = 0.0;
+    for (int z = 0; z < nsplit; ++z) {
+        const double* p = s.lrf_part + ((size_t)z * m.ncgp + g2) * kLrfMom20;
+#pragma unroll
+        for (int k = 0; k < kLrfMom20; ++k) tot[k] += p[k];
+    }
+    double m24[kLrfMom];
+    lrf_moments24(tot, m24);
+    lrf_expand(m24, s.lrf + (size_t)g2 * kLrfLen + 3);
+}
+
 // Mixed form: one thread per PAIR of target groups, the two in the halves of
 // packed FP32x2 arithmetic, so every packed instruction advances both targets
 // and no half has to be rearranged (the 38 operations of lrf_terms_e take 44
@@ -881,7 +1069,6 @@ struct LrfSmem {   // of one warp; the staged atoms follow the blocks' warps
     int end[2][kLrfTile];   // last atom + 1 of the group in the tile | solute flag << 30
 };
 constexpr int kLrfTot = kLrfMom20 + 4;   // totals of a target: the 20 moments, F0, U(3)
-__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 // (hi, lo) += (p, pl) in double-float
 __device__ __forceinline__ void df_add(float& hi, float& lo, float p, float pl) {
     const float sum = __fadd_rn(hi, p), bb = __fsub_rn(sum, hi);
@@ -912,16 +1099,6 @@ __device__ __forceinline__ double lrf_coef(const double* n, int c) {
 #ifndef QNB_LRF_U
 #define QNB_LRF_U 3
 #endif
-// 1/sqrt on the SFU with subnormal inputs taken as zero (a squared distance
-// below 1e-38 A^2): without it the compiler brackets each use with the
-// scaling of subnormals
-__device__ __forceinline__ float rsqrt_ftz(float v) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }   // exact product
-
 // the FP64 decision of a target and source group whose FP32 distance is
 // inside a decision band (or, in a box, whose lattice index is near a half)
 template <bool BOX>
@@ -1391,7 +1568,7 @@ __device__ __forceinline__ PairF nbe_f(float4 a, float4 b, float A, float B, flo
     p.ty = b.y - a.y;
     p.tz = b.z - a.z;
     float rr = p.tx * p.tx + p.ty * p.ty + p.tz * p.tz;
-    float ri = rsqrtf(rr);
+    float ri = rsqrt_ftz(rr);
     float r2 = ri * ri;
     p.vel = el * ri;
     if (lj) {
@@ -3837,7 +4014,7 @@ int launch_lrf_pairs(const Launch& L, const Cut& c, int nz, int tile_atoms, size
 }
 }  // namespace
 
-int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src) {
+int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src, int keep_order) {
     if (L.m.any_atom && L.m.box) {
         k_lrf_accumulate_any_box<<<grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin), 128, 0, L.st>>>(L.m, L.ds, c);
         return 1;
@@ -3847,6 +4024,17 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
         if (mixed) k_lrf_accumulate_any<true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
         else k_lrf_accumulate_any<false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
         return 1;
+    }
+    if (mixed && keep_order) {
+        // source ranges of at least one staged tile each; the split depends on
+        // the topology only, so a window's coefficients are the same in a
+        // batch of any size
+        const int nsplit = std::min(kLrfSplitMax, std::max(1, L.m.nlrf_groups / kLrfGT));
+        dim3 g((L.m.ncgp + kLrfNB - 1) / kLrfNB, L.nwin, nsplit);
+        if (L.m.box) k_lrf_nbody<true><<<g, kLrfNB, 0, L.st>>>(L.m, L.ds, c, nsplit);
+        else k_lrf_nbody<false><<<g, kLrfNB, 0, L.st>>>(L.m, L.ds, c, nsplit);
+        k_lrf_combine<<<dim3((L.m.ncgp + 127) / 128, L.nwin), 128, 0, L.st>>>(L.m, L.ds, nsplit);
+        return 2;
     }
     if (mixed) {
         // blocks per cluster: ranges of at least one tile per warp, the split

@@ -3765,8 +3765,28 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
     }
 }
 
-// water rows: ww (waters, SPC fast path as nonbond_ww_spc) and wp (solute
-// groups) gradient of the water's atoms
+// Two Coulomb pairs in packed FP32x2 arithmetic, bit for bit pair_f's: t the
+// partners' positions minus the row atoms', el the charge products; returns the
+// energies, ndv = -dv.
+__device__ __forceinline__ float2 coul2(float2 tx, float2 ty, float2 tz, float2 el, float2& ndv) {
+    const float2 rr = __ffma2_rn(tz, tz, __ffma2_rn(tx, tx, __fmul2_rn(ty, ty)));   // (the order nvcc contracts nbe_f's sum in)
+    const float2 ri = make_float2(rsqrt_ftz(rr.x), rsqrt_ftz(rr.y));
+    const float2 vel = __fmul2_rn(el, ri);
+    ndv = __fmul2_rn(__fmul2_rn(ri, ri), vel);
+    return vel;
+}
+
+// Water rows: ww (waters, SPC fast path as nonbond_ww_spc) and wp (solute
+// groups): gradient of the water's atoms.  The row's issue slots and gathers
+// bound it.  SPC: a pair's nine terms are one LJ + Coulomb term and four packed
+// pairs of Coulomb terms (the partner's H against the row O; the row's H
+// against each partner atom), a solute atom's three one and a packed pair, each
+// sum in the order of the scalar terms, so the gradient is theirs bit for bit
+// (a trajectory amplifies rounding).  A lane takes a listed group's non-Q atoms
+// one after the other, the next one's data loaded ahead.  51 windows of the 25 A
+// sphere 110 -> 86 us, of the 15 A droplet 44 -> 36 us.  (Solute partners as a
+// list of atoms instead of groups measured 73 us, but sums them in another
+// order.)
 template <bool SPC, bool BOX>
 __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevState* __restrict__ states) {
     extern __shared__ float4 sh_lj[];   // natyps^2 type-pair table (dynamic: only its real size)
@@ -3777,14 +3797,11 @@ __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevStat
     TypeTab lj = stage_types(m, sh_lj);
     const float4* __restrict__ xq = s.xq;
     int lane = threadIdx.x & 31;
-    const int sa = m.sa;
-    // SPC rows: 3-atom molecules (the launcher's choice), so the row's atom
-    // arrays hold 3 entries and a partner's atoms are loaded one iteration
-    // ahead
+    const int sa = SPC ? 3 : m.sa;   // SPC rows: 3-atom molecules (the launcher's choice)
     constexpr int NA = SPC ? 3 : kMaxSolv;
     for (int w = warp_id_global(); w < m.nwat; w += warps_total()) {
-        int nww = s.cnt_ww[w], nwg = s.cnt_wg[w];   // an empty row still writes its zeros
-        int i0 = m.nat_solute + sa * w;
+        const int nww = s.cnt_ww[w], nwg = s.cnt_wg[w];   // an empty row still writes its zeros
+        const int i0 = m.nat_solute + sa * w;
         float4 xa[NA];
         float f[NA][3];
 #pragma unroll
@@ -3803,6 +3820,21 @@ __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevStat
         if (nchunk > 0) fetch_ww(0);
         for (int u = lane; u < (min(kRowChunk, nwg) + 3) >> 2; u += kWarp) cp_async16(&sh_wg[wib][4 * u], rg + 4 * u);
         cp_async_commit();
+        // SPC: the row's two H in packed pairs
+        const float2 hx = make_float2(xa[1].x, xa[2].x), hy = make_float2(xa[1].y, xa[2].y),
+                     hz = make_float2(xa[1].z, xa[2].z);
+        float2 ghx = make_float2(0.f, 0.f), ghy = ghx, ghz = ghx;
+        // the two H against one atom
+        auto h_pair = [&](const float4 xb, float2 el) -> float2 {
+            const float2 tx = make_float2(xb.x - hx.x, xb.x - hx.y), ty = make_float2(xb.y - hy.x, xb.y - hy.y),
+                         tz = make_float2(xb.z - hz.x, xb.z - hz.y);
+            float2 ndv;
+            const float2 vel = coul2(tx, ty, tz, el, ndv);
+            ghx = __ffma2_rn(tx, ndv, ghx);
+            ghy = __ffma2_rn(ty, ndv, ghy);
+            ghz = __ffma2_rn(tz, ndv, ghz);
+            return vel;
+        };
         for (int ch = 0; ch < nchunk; ++ch) {
           if (ch + 1 < nchunk) {
               fetch_ww(ch + 1);
@@ -3815,45 +3847,49 @@ __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevStat
           const int* buf = sh_ww[wib][ch & 1];
           const int n = min(kRowChunk, nww - ch * kRowChunk);
           if constexpr (SPC) {
-            float4 nx0 = make_float4(0.f, 0.f, 0.f, 0.f), nx1 = nx0, nx2 = nx0;
+            const float2 eoh = make_float2(m.wwEf[1], m.wwEf[2]), eho = make_float2(m.wwEf[kMaxSolv], m.wwEf[2 * kMaxSolv]),
+                         eh1 = make_float2(m.wwEf[kMaxSolv + 1], m.wwEf[2 * kMaxSolv + 1]),
+                         eh2 = make_float2(m.wwEf[kMaxSolv + 2], m.wwEf[2 * kMaxSolv + 2]);
+            float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0, n2 = n0;
             int nw2 = 0;
             if (lane < n) {
                 nw2 = buf[lane];
                 const int j = m.nat_solute + 3 * nw2;
-                nx0 = xq[j], nx1 = xq[j + 1], nx2 = xq[j + 2];
+                n0 = xq[j], n1 = xq[j + 1], n2 = xq[j + 2];
             }
             for (int k = lane; k < n; k += kWarp) {
-              const int w2 = nw2;
-              const float4 xp[3] = {nx0, nx1, nx2};
+              float4 x0 = n0, x1 = n1, x2 = n2;
+              const bool count = w < nw2;   // each molecule pair's energy once
               if (k + kWarp < n) {   // the next partner, one iteration ahead
                   nw2 = buf[k + kWarp];
                   const int j = m.nat_solute + 3 * nw2;
-                  nx0 = xq[j], nx1 = xq[j + 1], nx2 = xq[j + 2];
+                  n0 = xq[j], n1 = xq[j + 1], n2 = xq[j + 2];
               }
-              float pel = 0.f, pvdw = 0.f;
-#pragma unroll
-              for (int b = 0; b < 3; ++b) {
-                  float4 xb = xp[b];
-                  if (BOX) xb = at_image(m, xb, xa[0], xp[0]);
-#pragma unroll
-                  for (int a = 0; a < 3; ++a) {
-                      const int kk = a * kMaxSolv + b;
-                      const bool lj = a == 0 && b == 0;
-                      float vel, vdw;
-                      pair_f(xa[a], xb, m.wwAf[kk], m.wwBf[kk], m.wwEf[kk], lj, f[a][0], f[a][1], f[a][2], vel, vdw);
-                      pel += vel;
-                      if (lj) pvdw += vdw;
-                  }
+              if (BOX) {
+                  const float4 xr = x0;
+                  x0 = at_image(m, x0, xa[0], xr), x1 = at_image(m, x1, xa[0], xr), x2 = at_image(m, x2, xa[0], xr);
               }
-              if (w < w2) {   // each molecule pair's energy once
+              float vel, vdw;
+              pair_f(xa[0], x0, m.wwAf[0], m.wwBf[0], m.wwEf[0], true, f[0][0], f[0][1], f[0][2], vel, vdw);
+              const float2 tx = make_float2(x1.x - xa[0].x, x2.x - xa[0].x), ty = make_float2(x1.y - xa[0].y, x2.y - xa[0].y),
+                           tz = make_float2(x1.z - xa[0].z, x2.z - xa[0].z);
+              float2 ndv;
+              const float2 eo = coul2(tx, ty, tz, eoh, ndv);
+              f[0][0] = fmaf(tx.y, ndv.y, fmaf(tx.x, ndv.x, f[0][0]));
+              f[0][1] = fmaf(ty.y, ndv.y, fmaf(ty.x, ndv.x, f[0][1]));
+              f[0][2] = fmaf(tz.y, ndv.y, fmaf(tz.x, ndv.x, f[0][2]));
+              // the energies in the scalar terms' order, in which the charges'
+              // signs cancel early and the partial sums stay small
+              const float2 e0 = h_pair(x0, eho), e1 = h_pair(x1, eh1), e2 = h_pair(x2, eh2);
+              const float pel = vel + e0.x + e0.y + eo.x + e1.x + e1.y + eo.y + e2.x + e2.y;
+              if (count) {
                   rel += pel;
-                  rvdw += pvdw;
+                  rvdw += vdw;
               }
             }
           } else {
           for (int k = lane; k < n; k += kWarp) {
-            int w2 = buf[k];
-            int j0 = m.nat_solute + sa * w2;
+            const int w2 = buf[k], j0 = m.nat_solute + sa * w2;
             float pel = 0.f, pvdw = 0.f;
             const float4 xr = BOX ? xq[j0] : make_float4(0.f, 0.f, 0.f, 0.f);   // partner's first atom
 #pragma unroll
@@ -3883,15 +3919,31 @@ __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevStat
             cp_async_wait<0>();
             __syncwarp();
         }
+        // solute partners; the energy is counted in the solute rows
         for (int k = lane; k < nwg; k += kWarp) {
-            int g = k < kRowChunk ? sh_wg[wib][k] : rg[k];
+            const int g = k < kRowChunk ? sh_wg[wib][k] : rg[k];
             const float4 xr = BOX ? xq[m.gsw[g]] : make_float4(0.f, 0.f, 0.f, 0.f);   // group's switch atom
-            for (int bb = m.gslot[g]; bb < m.gslot[g + 1]; ++bb) {
-                int j = m.gatom[bb];
-                if (m.iqatom[j] >= 0) continue;
-                float4 xb = xq[j];
+            const int a1 = m.gnq_off[g + 1];
+            int b = m.gnq_off[g], nt = 0;
+            float4 nx = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto load = [&](int b) {
+                const int j = m.gnq_atom[b];
+                nx = xq[j];
+                nt = m.iac[j];
+            };
+            if (b < a1) load(b);
+            for (; b < a1; ++b) {
+                float4 xb = nx;
                 if (BOX) xb = at_image(m, xb, xa[0], xr);
-                int tj = m.iac[j];
+                const int tj = nt;
+                if (b + 1 < a1) load(b + 1);   // one atom ahead
+                if (SPC && m.wlj_mask == 1u) {   // O with LJ, two LJ-free H
+                    const float4 p = lj(tj, m.wtype[0]);
+                    float vel, vdw;
+                    pair_f(xa[0], xb, p.x, p.y, xb.w * m.wcrgf[0], true, f[0][0], f[0][1], f[0][2], vel, vdw);
+                    h_pair(xb, make_float2(xb.w * m.wcrgf[1], xb.w * m.wcrgf[2]));
+                    continue;
+                }
 #pragma unroll
                 for (int a = 0; a < NA; ++a) {
                     if (a >= sa) break;
@@ -3903,22 +3955,21 @@ __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevStat
             }
         }
         __syncwarp();   // sh_wg is refilled by the next row
-        // row gradient and energies stored as in k_rows_solute
-        float e0 = warp_sum(rel), e1 = warp_sum(rvdw);
-        if (lane == 0) {
-            if (e0 != 0.f) atomicAdd(s.efix + E_WW_EL, to_fix(e0));
-            if (e1 != 0.f) atomicAdd(s.efix + E_WW_VDW, to_fix(e1));
+        if constexpr (SPC) {
+            f[1][0] += ghx.x, f[1][1] += ghy.x, f[1][2] += ghz.x;   // (added to zeros unless the H have LJ)
+            f[2][0] += ghx.y, f[2][1] += ghy.y, f[2][2] += ghz.y;
         }
+        // row gradient and energies stored as in k_rows_solute: one transposed
+        // warp sum, lanes 2v and 2v + 1 end with value v
+        float g[16];
 #pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            if (a >= sa) break;
-            float v0 = warp_sum(f[a][0]), v1 = warp_sum(f[a][1]), v2 = warp_sum(f[a][2]);
-            if (lane == 0) {
-                float* fr = s.frow + 3 * (i0 + a);
-                fr[0] = v0;
-                fr[1] = v1;
-                fr[2] = v2;
-            }
+        for (int v = 0; v < 16; ++v) g[v] = v < 3 * NA ? f[v < 3 * NA ? v / 3 : 0][v % 3] : 0.f;
+        g[14] = rel, g[15] = rvdw;
+        const float v = reduce_scatter<16>(g, lane);
+        if (!(lane & 1)) {
+            const int c = lane >> 1;
+            if (c < 3 * sa) s.frow[3 * i0 + c] = v;
+            else if (c >= 14 && v != 0.f) atomicAdd(s.efix + (c == 14 ? E_WW_EL : E_WW_VDW), to_fix(v));
         }
     }
 }

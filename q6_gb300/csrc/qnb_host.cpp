@@ -1020,6 +1020,7 @@ int alloc_state(qnb_context* c) {
         s.x = c->x_all + n3 * w;
         s.d = c->d_all + n3 * w;
         TRY(c->alloc(&s.xq, (size_t)m.natom));
+        if (c->mixed) TRY(c->alloc(&s.xr, (size_t)m.natom));
         TRY(c->alloc(&s.frow, (size_t)3 * m.natom));
         CU(cudaMemset(s.frow, 0, sizeof(float) * 3 * m.natom));   // atoms outside every row stay 0
         TRY(c->alloc(&s.fq, (size_t)3 * m.natom));

@@ -183,6 +183,7 @@ struct DevState {
     const double* md_tfree;   // Tfree of the window's last MD temperature() (null before qnb_md_init)
     double* d;           // [natom*3] gradient accumulator (FP64 mode target)
     float4* xq;          // [natom] FP32 (x,y,z,charge) for the mixed form
+    float4* xr;          // [natom] FP32 position of each atom's unit reference atom (mixed form's box rows)
     float* frow;         // [natom*3] mixed form: row-kernel gradient of each atom's own row (FP32 warp sum)
     float* fq;           // [natom*3] mixed form: Q-environment gradient of each listed qp atom / qw water
     unsigned long long* fix;   // [natom*3] fixed-point gradient (mixed form)

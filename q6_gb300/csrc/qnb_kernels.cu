@@ -265,6 +265,11 @@ __global__ void k_pack(DevModel m, const DevState* __restrict__ states) {
     if (i >= m.natom) return;
     xq[i] = make_float4((float)(x[3 * i] - m.xpcent[0]), (float)(x[3 * i + 1] - m.xpcent[1]),
                         (float)(x[3 * i + 2] - m.xpcent[2]), (float)m.crg[i]);
+    if (m.box_rows) {   // each atom's unit reference atom (the row kernels' lattice shifts)
+        const int r = m.swat[i];
+        states[blockIdx.y].xr[i] = make_float4((float)(x[3 * r] - m.xpcent[0]), (float)(x[3 * r + 1] - m.xpcent[1]),
+                                               (float)(x[3 * r + 2] - m.xpcent[2]), 0.f);
+    }
 }
 
 __device__ __forceinline__ float r2_f(float4 a, float4 b) {
@@ -3387,38 +3392,56 @@ constexpr int kRowChunk = 128;   // entries per prefetched chunk
 // of all pp energies are halved instead of testing which side counts a pair.
 // Groups of at most 8 atoms carry the partner's LJ type in entry bits 16..31.
 //
-// Resident 128-thread blocks per SM asked of the register allocator: the
-// kernel waits mostly on its gathers, so occupancy pays more than the few
-// spilled registers (6 blocks = 80 registers for groups of up to 6 atoms).
+// All terms are packed (pair2), in the order of the scalar sums they replace,
+// and the row atoms' LJ factors and types are read from shared memory, so the
+// registers hold positions, charges and gradients only: 187 -> 163 us per
+// 51-window R25 step, 262 -> 178 us in the box (whose partners' reference
+// positions come from one array instead of two dependent loads).
 // Two row atoms against one partner in packed FP32x2 arithmetic (GB300's
-// FFMA2 / FMUL2 / FADD2; one rsqrt per atom on the SFU): the plain code-1
-// pair of the geometric rule, A = fa fj.x and B = fb fj.y.  The row kernels
-// are bound by the latency of each pair's dependent chain, and a packed
-// instruction advances two chains.  n* are the negated row positions, q the
-// row charges; adds the row atoms' gradient into g* and their energies into
-// pel / pvdw.
-__device__ __forceinline__ void pair2_plain(float2 nx, float2 ny, float2 nz, float2 q, float2 fa, float2 fb,
-                                            float2 bx, float2 by, float2 bz, float2 bq, float2 fjx, float2 fjy,
-                                            float2& gx, float2& gy, float2& gz, float2& pel, float2& pvdw) {
+// FFMA2 / FMUL2 / FADD2; one rsqrt per atom on the SFU): the row kernels are
+// bound by the latency of each pair's dependent chain and by issue slots, and a
+// packed instruction advances two chains.  n* are the negated row positions,
+// b* the partner's, el the charge products, A and B the pairs' LJ parameters;
+// adds the row atoms' gradient into g* and their LJ energies into pvdw, and
+// returns their Coulomb energies in vel.
+// PLAIN: the order in which the plain loop has always summed the squared
+// distance; otherwise pair_f's, whose terms these then are bit for bit.
+// dead: atoms whose pair is excluded (el, A and B zero), whose distance may be
+// zero as well.
+template <bool PLAIN>
+__device__ __forceinline__ void pair2(float2 nx, float2 ny, float2 nz, float2 bx, float2 by, float2 bz, float2 el,
+                                      float2 A, float2 B, float2& gx, float2& gy, float2& gz, float2& vel, float2& pvdw,
+                                      bool dead0 = false, bool dead1 = false) {
     const float2 tx = __fadd2_rn(bx, nx), ty = __fadd2_rn(by, ny), tz = __fadd2_rn(bz, nz);
-    float2 rr = __fmul2_rn(tx, tx);
-    rr = __ffma2_rn(ty, ty, rr);
+    float2 rr = PLAIN ? __ffma2_rn(ty, ty, __fmul2_rn(tx, tx)) : __ffma2_rn(tx, tx, __fmul2_rn(ty, ty));
     rr = __ffma2_rn(tz, tz, rr);
-    const float2 ri = make_float2(rsqrtf(rr.x), rsqrtf(rr.y));
+    if (!PLAIN) rr = make_float2(dead0 ? 1.f : rr.x, dead1 ? 1.f : rr.y);
+    const float2 ri = make_float2(rsqrt_ftz(rr.x), rsqrt_ftz(rr.y));
     const float2 r2 = __fmul2_rn(ri, ri);
-    const float2 vel = __fmul2_rn(__fmul2_rn(q, bq), ri);
+    vel = __fmul2_rn(el, ri);
     const float2 r6 = __fmul2_rn(__fmul2_rn(r2, r2), r2);
-    const float2 va = __fmul2_rn(__fmul2_rn(__fmul2_rn(fa, fjx), r6), r6);
-    const float2 vb = __fmul2_rn(__fmul2_rn(fb, fjy), r6);
+    const float2 va = __fmul2_rn(__fmul2_rn(A, r6), r6);
+    const float2 vb = __fmul2_rn(B, r6);
     // -dv = r2 (vel + 12 va - 6 vb); the gradient of the row atom is -t dv
-    float2 t = __ffma2_rn(make_float2(12.f, 12.f), va, vel);
-    t = __ffma2_rn(make_float2(-6.f, -6.f), vb, t);
+    float2 t = __ffma2_rn(f2(12.f), va, vel);
+    t = __ffma2_rn(f2(-6.f), vb, t);
     const float2 ndv = __fmul2_rn(r2, t);
     gx = __ffma2_rn(tx, ndv, gx);
     gy = __ffma2_rn(ty, ndv, gy);
     gz = __ffma2_rn(tz, ndv, gz);
-    pel = __fadd2_rn(pel, vel);
-    pvdw = __fadd2_rn(pvdw, __ffma2_rn(make_float2(-1.f, -1.f), vb, va));
+    pvdw = __fadd2_rn(pvdw, fsub2(va, vb));
+}
+// the Coulomb term alone, bit for bit pair2<false>'s with A = B = 0
+__device__ __forceinline__ void pair2_coul(float2 nx, float2 ny, float2 nz, float2 bx, float2 by, float2 bz, float2 el,
+                                           float2& gx, float2& gy, float2& gz, float2& vel) {
+    const float2 tx = __fadd2_rn(bx, nx), ty = __fadd2_rn(by, ny), tz = __fadd2_rn(bz, nz);
+    const float2 rr = __ffma2_rn(tz, tz, __ffma2_rn(tx, tx, __fmul2_rn(ty, ty)));
+    const float2 ri = make_float2(rsqrt_ftz(rr.x), rsqrt_ftz(rr.y));
+    vel = __fmul2_rn(el, ri);
+    const float2 ndv = __fmul2_rn(__fmul2_rn(ri, ri), vel);
+    gx = __ffma2_rn(tx, ndv, gx);
+    gy = __ffma2_rn(ty, ndv, gy);
+    gz = __ffma2_rn(tz, ndv, gz);
 }
 
 // periodic box: partner position p at the image of its unit's reference
@@ -3436,69 +3459,50 @@ __device__ __forceinline__ float4 at_image(const DevModel& m, float4 p, float4 r
 #ifndef QNB_ROWS_MIN_BLOCKS
 #define QNB_ROWS_MIN_BLOCKS 0   // 0: the per-size default below
 #endif
-// resident 128-thread blocks per SM the row kernel is compiled for: the
-// packed plain loop of the geometric rule holds twice the row-atom registers
-// and measured best at 5 (96 registers: 212 us per 51-window R25 step, 226 at
-// 6 blocks, where it spills inside the loop); the scalar loop at 6
-template <int MAXG, bool GEOM>
+// resident 128-thread blocks per SM the row kernel is compiled for, groups of
+// up to 6 atoms, 51 windows of the 25 A sphere: 4 blocks (128 registers) 161 us
+// alone, 5 (96) 163, 6 (80, spilling inside the loop) 193; the box's lattice
+// images hold more registers: 178, 223 and 245 us.  5 on the sphere, where the
+// step beside the other branches was the shorter (457 against 471 us a pass)
+template <int MAXG, bool BOX>
 constexpr int rows_min_blocks() {
-    return QNB_ROWS_MIN_BLOCKS ? QNB_ROWS_MIN_BLOCKS
-                               : (MAXG <= 6 ? (GEOM ? 5 : 6) : (MAXG <= 8 ? 4 : 1));
+    return QNB_ROWS_MIN_BLOCKS ? QNB_ROWS_MIN_BLOCKS : (MAXG <= 6 ? (BOX ? 4 : 5) : (MAXG <= 8 ? 4 : 1));
 }
 template <int MAXG, bool GEOM, bool BOX>
-__global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_solute(DevModel m, const DevState* __restrict__ states) {
+__global__ void __launch_bounds__(128, rows_min_blocks<MAXG, BOX>()) k_rows_solute(DevModel m, const DevState* __restrict__ states) {
     extern __shared__ float4 sh_lj[];   // natyps^2 type-pair table (dynamic: only its real size)
     __shared__ __align__(16) uint2 sh_pp[4][2][kRowChunk];   // per warp: double-buffered special pp entries
     __shared__ __align__(16) int sh_pf[4][2][kRowChunk];     // per warp: double-buffered plain pp entries
     __shared__ __align__(16) int sh_pw[4][kRowChunk];        // per warp: first chunk of pw entries
     constexpr bool kTypeInEntry = MAXG <= 8;
+    constexpr int NP = MAXG / 2;        // row atoms in pairs (2p, 2p + 1)
+    constexpr int kIter = kRowChunk / kWarp;   // warp iterations per chunk
+    struct alignas(16) RowAtoms {   // of a warp's row, by pairs of atoms (read 16 bytes at a time)
+        float pos[NP][4][2], fab[NP][2][2];
+        int ta[MAXG];
+    };
+    static_assert(sizeof(RowAtoms) % 16 == 0 && sizeof(float) * 8 % 16 == 0, "16-byte rows of pos and fab");
+    __shared__ RowAtoms sh_row[4];
     const DevState& s = states[blockIdx.y];
     const int wib = threadIdx.x >> 5;
     TypeTab lj = stage_types(m, sh_lj);
     const float4* __restrict__ xq = s.xq;
+    const float4* __restrict__ xr = s.xr;   // (box) each atom's unit reference atom
     // m.el14f, not (float)m.el14: under register pressure the compiler may
     // rematerialise a double-to-float conversion of the parameter inside the
     // pair loop, and that conversion runs on the narrow FP64 pipe
     const float el14 = m.el14f;
     int lane = threadIdx.x & 31;
     for (int g = warp_id_global(); g < m.ncgp_solute; g += warps_total()) {
-        int npp = s.cnt_gp[g], npw = s.cnt_gw[g];   // an empty row still writes its zeros
-        int a0 = m.gslot[g], n1 = m.gslot[g + 1] - a0;
+        const int npp = s.cnt_gp[g], npw = s.cnt_gw[g], npf = s.cnt_gf[g];   // an empty row still writes its zeros
+        const int a0 = m.gslot[g], n1 = m.gslot[g + 1] - a0;
         if (n1 > MAXG) {   // a Q-only group larger than the rows handle: empty row, zero gradient
             for (int a = lane; a < 3 * n1; a += kWarp) s.frow[3 * m.gatom[a0 + a / 3] + a % 3] = 0.f;
             continue;
         }
-        // periodic box: the row group's reference atom (its lattice shifts)
-        const float4 xsw = BOX ? xq[m.gsw[g]] : make_float4(0.f, 0.f, 0.f, 0.f);
-        int ta[MAXG];
-        float4 xa[MAXG];
-        bool qa[MAXG];
-        float f[MAXG][3];
-#pragma unroll
-        for (int a = 0; a < MAXG; ++a) {
-            f[a][0] = f[a][1] = f[a][2] = 0.f;
-            if (a < n1) {
-                int i = m.gatom[a0 + a];
-                ta[a] = m.iac[i];
-                xa[a] = xq[i];
-                qa[a] = m.iqatom[i] >= 0;
-            } else {
-                ta[a] = 0;
-                xa[a] = make_float4(0, 0, 0, 0);
-                qa[a] = true;
-            }
-        }
-        // per-row FP32 energy sums of this lane, converted to fixed point once
-        // per row (row contents do not depend on the grid, so neither do they)
-        float rpel = 0.f, rpvdw = 0.f, rwel = 0.f, rwvdw = 0.f;
-        // ---- solute partner atoms (nonbond_pp, src/nonbondene.f90:4694-4760):
-        // the special entries (kinds, any LJ code) first, then the water
-        // partners, then the plain solute partners (the hot loop, last, so the
-        // type indices are no longer live in it)
         const uint2* rp = s.row_gp + (size_t)g * s.cap_gp;
         const int* rf = s.row_gf + (size_t)g * s.cap_gf;
         const int* rw = s.row_gw + (size_t)g * s.cap_gw;
-        const int npf = s.cnt_gf[g];
         const int nchunk = (npp + kRowChunk - 1) / kRowChunk, nfchunk = (npf + kRowChunk - 1) / kRowChunk;
         auto fetch_pp = [&](int ch) {
             int e0 = ch * kRowChunk, units = (min(kRowChunk, npp - e0) + 1) >> 1;
@@ -3509,9 +3513,55 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
             for (int u = lane; u < units; u += kWarp) cp_async16(&sh_pf[wib][ch & 1][4 * u], rf + e0 + 4 * u);
         };
         if (nchunk > 0) fetch_pp(0);
-        if (nfchunk > 0) fetch_pf(0);
         for (int u = lane; u < (min(kRowChunk, npw) + 3) >> 2; u += kWarp) cp_async16(&sh_pw[wib][4 * u], rw + 4 * u);
+        if (nfchunk > 0) fetch_pf(0);
         cp_async_commit();
+        // periodic box: the row group's reference atom (its lattice shifts)
+        const float4 xsw = BOX ? xq[m.gsw[g]] : make_float4(0.f, 0.f, 0.f, 0.f);
+        // the row atoms, one per lane, into shared memory in pairs: negated
+        // positions and charges (kept in registers below), code-1 LJ factors
+        // and types (read back as broadcasts, which spares registers).  A Q
+        // atom gets zero charge and LJ parameters throughout, so its terms are
+        // exact zeros (its row gradient is discarded); so does an odd group's
+        // last pair's second atom, far away
+        RowAtoms& R = sh_row[wib];
+        bool dead = true;
+        if (lane < MAXG) {
+            float4 v = make_float4(1.0e4f, 1.0e4f, 1.0e4f, 0.f);
+            float2 f1 = f2(0.f);
+            int t = 0;
+            if (lane < n1) {
+                const int i = m.gatom[a0 + lane];
+                t = m.iac[i];
+                v = xq[i];
+                dead = m.iqatom[i] >= 0;
+                if (dead) v.w = 0.f;
+                else if (GEOM) f1 = m.ljf1[i];
+            }
+            R.pos[lane >> 1][0][lane & 1] = -v.x;
+            R.pos[lane >> 1][1][lane & 1] = -v.y;
+            R.pos[lane >> 1][2][lane & 1] = -v.z;
+            R.pos[lane >> 1][3][lane & 1] = v.w;
+            R.fab[lane >> 1][0][lane & 1] = f1.x;
+            R.fab[lane >> 1][1][lane & 1] = f1.y;
+            R.ta[lane] = t;
+        }
+        const unsigned off = __ballot_sync(kFull, dead);   // bit a: row atom a is a Q atom or absent
+        __syncwarp();
+        float2 nx[NP], ny[NP], nz[NP], q2[NP], gx[NP], gy[NP], gz[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const float4 u = *reinterpret_cast<const float4*>(R.pos[p][0]), v = *reinterpret_cast<const float4*>(R.pos[p][2]);
+            nx[p] = make_float2(u.x, u.y), ny[p] = make_float2(u.z, u.w);
+            nz[p] = make_float2(v.x, v.y), q2[p] = make_float2(v.z, v.w);
+            gx[p] = gy[p] = gz[p] = f2(0.f);
+        }
+        // per-row FP32 energy sums of this lane, converted to fixed point once
+        // per row (row contents do not depend on the grid, so neither do they)
+        float2 pel = f2(0.f), pvdw = f2(0.f), wel = f2(0.f), wvdw = f2(0.f);
+        // ---- solute partner atoms (nonbond_pp, src/nonbondene.f90:4694-4760):
+        // the special entries (kinds, any LJ code) first, then the water
+        // partners, then the plain solute partners (the hot loop)
         for (int ch = 0; ch < nchunk; ++ch) {
           if (ch + 1 < nchunk) {
               fetch_pp(ch + 1);
@@ -3523,27 +3573,46 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
           __syncwarp();
           const uint2* buf = sh_pp[wib][ch & 1];
           const int n = min(kRowChunk, npp - ch * kRowChunk);
+          float4 xn = make_float4(0.f, 0.f, 0.f, 0.f), rn = xn;
+          unsigned kn = 0;
+          int tn = 0;
+          auto load = [&](int k) {
+              const uint2 e = buf[k];
+              const int j = (int)(e.x & 0x0fffffffu);
+              xn = xq[j];
+              if (BOX) rn = xr[j];
+              tn = kTypeInEntry ? (int)(e.y >> 16) : m.iac[j];
+              kn = kTypeInEntry ? (e.y & 0xffffu) : e.y;
+          };
+          if (lane < n) load(lane);
           for (int k = lane; k < n; k += kWarp) {
-            uint2 e = buf[k];
-            int j = (int)(e.x & 0x0fffffffu);
-            float4 xb = xq[j];
-            if (BOX) xb = at_image(m, xb, xsw, xq[m.swat[j]]);
-            int tj = kTypeInEntry ? (int)(e.y >> 16) : m.iac[j];
-            const unsigned kinds = kTypeInEntry ? (e.y & 0xffffu) : e.y;
+            const float4 xb = BOX ? at_image(m, xn, xsw, rn) : xn;
+            const unsigned kinds = kn;
+            const int tj = tn;
+            if (k + kWarp < n) load(k + kWarp);   // one iteration ahead
 #pragma unroll
-            for (int a = 0; a < MAXG; ++a) {
-                if (qa[a]) continue;
-                unsigned kind = (kinds >> (2 * a)) & 3u;
-                if (kind == 1u) continue;
-                float4 p = lj(ta[a], tj);
-                bool is14 = kind == 3u;
-                float A = is14 ? p.z : p.x, B = is14 ? p.w : p.y;
-                float el = xa[a].w * xb.w;
-                if (is14) el *= el14;
-                float vel, vdw;
-                pair_f(xa[a], xb, A, B, el, true, f[a][0], f[a][1], f[a][2], vel, vdw);
-                rpel += vel;
-                rpvdw += vdw;
+            for (int p = 0; p < NP; ++p) {
+                if (2 * p >= n1) break;   // warp-uniform
+                float2 A, B, el = __fmul2_rn(q2[p], f2(xb.w));
+                bool ex[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int a = 2 * p + h;
+                    const unsigned kind = (kinds >> (2 * a)) & 3u;
+                    ex[h] = kind == 1u;
+                    const bool dead = ex[h] || ((off >> a) & 1u);
+                    const float4 t = lj(R.ta[a], tj);
+                    const float Av = dead ? 0.f : (kind == 3u ? t.z : t.x), Bv = dead ? 0.f : (kind == 3u ? t.w : t.y);
+                    float e = h ? el.y : el.x;
+                    if (kind == 3u) e *= el14;
+                    if (ex[h]) e = 0.f;
+                    if (h) A.y = Av, B.y = Bv, el.y = e;
+                    else A.x = Av, B.x = Bv, el.x = e;
+                }
+                float2 vel;
+                pair2<false>(nx[p], ny[p], nz[p], f2(xb.x), f2(xb.y), f2(xb.z), el, A, B, gx[p], gy[p], gz[p], vel, pvdw,
+                             ex[0], ex[1]);
+                pel = __fadd2_rn(pel, vel);
             }
           }
           __syncwarp();   // this buffer is refilled two chunks later
@@ -3552,6 +3621,20 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
             cp_async_wait<0>();
             __syncwarp();
         }
+        // the plain partners' first data, behind the water loop
+        float4 xbn = make_float4(0.f, 0.f, 0.f, 0.f), xrn = xbn;
+        float2 fjn = f2(0.f);
+        int tjn = 0;
+        auto load_pf = [&](int k) {   // entry k of the row, its chunk in shared memory
+            const int j = sh_pf[wib][(k / kRowChunk) & 1][k % kRowChunk];
+            xbn = xq[j];
+            if (BOX) xrn = xr[j];
+            if constexpr (GEOM) fjn = m.ljf1[j];
+            else tjn = m.iac[j];
+        };
+        if (lane < npf) load_pf(lane);
+        if (nfchunk > 1) fetch_pf(1);
+        cp_async_commit();
         // ---- water partners (nonbond_pw, src/nonbondene.f90:4856-4916); energy counted here
         if (m.sa == 3 && m.wlj_mask == 1u) {   // SPC: O with LJ, two LJ-free H; the molecule loaded at once
           const float qo = m.wcrgf[0], qh1 = m.wcrgf[1], qh2 = m.wcrgf[2];
@@ -3560,163 +3643,102 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
             int j0 = m.nat_solute + 3 * (k < kRowChunk ? sh_pw[wib][k] : rw[k]);
             float4 xo = xq[j0], xh1 = xq[j0 + 1], xh2 = xq[j0 + 2];
             if (BOX) {
-                const float4 xr = xo;
-                xo = at_image(m, xo, xsw, xr), xh1 = at_image(m, xh1, xsw, xr), xh2 = at_image(m, xh2, xsw, xr);
+                const float4 xw = xo;
+                xo = at_image(m, xo, xsw, xw), xh1 = at_image(m, xh1, xsw, xw), xh2 = at_image(m, xh2, xsw, xw);
             }
 #pragma unroll
-            for (int a = 0; a < MAXG; ++a) {
-                if (qa[a]) continue;
-                float4 p = lj(ta[a], to);
-                float v1, d1, v2, d2, v3, d3;
-                pair_f(xa[a], xo, p.x, p.y, xa[a].w * qo, true, f[a][0], f[a][1], f[a][2], v1, d1);
-                pair_f(xa[a], xh1, 0.f, 0.f, xa[a].w * qh1, false, f[a][0], f[a][1], f[a][2], v2, d2);
-                pair_f(xa[a], xh2, 0.f, 0.f, xa[a].w * qh2, false, f[a][0], f[a][1], f[a][2], v3, d3);
-                rwel += v1 + v2 + v3;
-                rwvdw += d1;
+            for (int p = 0; p < NP; ++p) {
+                if (2 * p >= n1) break;   // warp-uniform
+                const float4 t0 = lj(R.ta[2 * p], to), t1 = lj(R.ta[2 * p + 1], to);
+                const bool d0 = (off >> (2 * p)) & 1u, d1 = (off >> (2 * p + 1)) & 1u;
+                float2 v0, v1, v2;
+                pair2<false>(nx[p], ny[p], nz[p], f2(xo.x), f2(xo.y), f2(xo.z), __fmul2_rn(q2[p], f2(qo)),
+                             make_float2(d0 ? 0.f : t0.x, d1 ? 0.f : t1.x), make_float2(d0 ? 0.f : t0.y, d1 ? 0.f : t1.y),
+                             gx[p], gy[p], gz[p], v0, wvdw);
+                pair2_coul(nx[p], ny[p], nz[p], f2(xh1.x), f2(xh1.y), f2(xh1.z), __fmul2_rn(q2[p], f2(qh1)), gx[p], gy[p],
+                           gz[p], v1);
+                pair2_coul(nx[p], ny[p], nz[p], f2(xh2.x), f2(xh2.y), f2(xh2.z), __fmul2_rn(q2[p], f2(qh2)), gx[p], gy[p],
+                           gz[p], v2);
+                wel = __fadd2_rn(wel, __fadd2_rn(__fadd2_rn(v0, v1), v2));   // the molecule's charges cancel first
             }
           }
         } else {
         for (int k = lane; k < npw; k += kWarp) {
             int j0 = m.nat_solute + m.sa * (k < kRowChunk ? sh_pw[wib][k] : rw[k]);
-            const float4 xr = BOX ? xq[j0] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 xw = BOX ? xq[j0] : make_float4(0.f, 0.f, 0.f, 0.f);
             for (int b = 0; b < m.sa; ++b) {
                 float4 xb = xq[j0 + b];
-                if (BOX) xb = at_image(m, xb, xsw, xr);
-                int tw = m.wtype[b];
-                if ((m.wlj_mask >> b) & 1u) {
-#pragma unroll
-                    for (int a = 0; a < MAXG; ++a) {
-                        if (qa[a]) continue;
-                        float4 p = lj(ta[a], tw);
-                        float vel, vdw;
-                        pair_f(xa[a], xb, p.x, p.y, xa[a].w * m.wcrgf[b], true, f[a][0], f[a][1], f[a][2], vel, vdw);
-                        rwel += vel;
-                        rwvdw += vdw;
-                    }
-                } else {   // A = B = 0 with every solute type: the Coulomb term alone, bit for bit
-#pragma unroll
-                    for (int a = 0; a < MAXG; ++a) {
-                        if (qa[a]) continue;
-                        float vel, vdw;
-                        pair_f(xa[a], xb, 0.f, 0.f, xa[a].w * m.wcrgf[b], false, f[a][0], f[a][1], f[a][2], vel, vdw);
-                        rwel += vel;
-                    }
-                }
-            }
-        }
-        }
-        // plain partners: LJ code 1 with every row atom, no excluded or 1-4
-        // pair; with the geometric rule A and B are the products of the atoms'
-        // FP32 code-1 factors (the type table holds the same products)
-        {
-          // with the geometric rule a Q row atom gets zero charge and LJ
-          // factors here, so its terms are exact zeros (its row gradient is
-          // discarded) and the loop needs no per-atom test
-          float fa[MAXG], fb[MAXG];
-#pragma unroll
-          for (int a = 0; a < MAXG; ++a) {
-              float2 f1 = (GEOM && a < n1 && !qa[a]) ? m.ljf1[m.gatom[a0 + a]] : make_float2(0.f, 0.f);
-              fa[a] = f1.x;
-              fb[a] = f1.y;
-              if (GEOM && qa[a]) xa[a].w = 0.f;
-          }
-          for (int ch = 0; ch < nfchunk; ++ch) {
-            if (ch + 1 < nfchunk) {   // chunk 0 came with the first group
-                fetch_pf(ch + 1);
-                cp_async_commit();
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncwarp();
-            const int* buf = sh_pf[wib][ch & 1];
-            const int n = min(kRowChunk, npf - ch * kRowChunk);
-            // the next entry's partner data is loaded one iteration ahead
-            float4 xbn = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 fjn = make_float2(0.f, 0.f);
-            int tjn = 0;
-            if (lane < n) {
-                const int j = buf[lane];
-                xbn = xq[j];
-                if (BOX) xbn = at_image(m, xbn, xsw, xq[m.swat[j]]);
-                if constexpr (GEOM) fjn = m.ljf1[j];
-                else tjn = m.iac[j];
-            }
-            if constexpr (GEOM) {
-              // row atoms in pairs (2p, 2p + 1); an odd group's last pair has a
-              // dummy atom far away with zero charge and factors
-              constexpr int NP = MAXG / 2;
-              float2 nx[NP], ny[NP], nz[NP], q2[NP], fa2[NP], fb2[NP], gx[NP], gy[NP], gz[NP];
-              float2 pel = make_float2(0.f, 0.f), pvdw = make_float2(0.f, 0.f);
-#pragma unroll
-              for (int p = 0; p < NP; ++p) {
-                  const int a = 2 * p, b = 2 * p + 1;
-                  const bool hb = b < n1;
-                  nx[p] = make_float2(-xa[a].x, hb ? -xa[b].x : -1.0e4f);
-                  ny[p] = make_float2(-xa[a].y, hb ? -xa[b].y : -1.0e4f);
-                  nz[p] = make_float2(-xa[a].z, hb ? -xa[b].z : -1.0e4f);
-                  q2[p] = make_float2(xa[a].w, hb ? xa[b].w : 0.f);
-                  fa2[p] = make_float2(fa[a], hb ? fa[b] : 0.f);
-                  fb2[p] = make_float2(fb[a], hb ? fb[b] : 0.f);
-                  gx[p] = make_float2(f[a][0], f[b][0]);   // the accumulators move into the pairs
-                  gy[p] = make_float2(f[a][1], f[b][1]);
-                  gz[p] = make_float2(f[a][2], f[b][2]);
-              }
-              for (int k = lane; k < n; k += kWarp) {
-                const float4 xb = xbn;
-                const float2 fj = fjn;
-                if (k + kWarp < n) {
-                    const int jn = buf[k + kWarp];
-                    xbn = xq[jn];
-                    if (BOX) xbn = at_image(m, xbn, xsw, xq[m.swat[jn]]);
-                    fjn = m.ljf1[jn];
-                }
-                const float2 bx = make_float2(xb.x, xb.x), by = make_float2(xb.y, xb.y),
-                             bz = make_float2(xb.z, xb.z), bq = make_float2(xb.w, xb.w),
-                             fjx = make_float2(fj.x, fj.x), fjy = make_float2(fj.y, fj.y);
+                if (BOX) xb = at_image(m, xb, xsw, xw);
+                const int tw = m.wtype[b];
+                const bool ljw = (m.wlj_mask >> b) & 1u;
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
                     if (2 * p >= n1) break;   // warp-uniform
-                    pair2_plain(nx[p], ny[p], nz[p], q2[p], fa2[p], fb2[p], bx, by, bz, bq, fjx, fjy, gx[p], gy[p],
-                                gz[p], pel, pvdw);
+                    const float2 el = __fmul2_rn(q2[p], f2(m.wcrgf[b]));
+                    float2 vel;
+                    if (ljw) {
+                        const float4 t0 = lj(R.ta[2 * p], tw), t1 = lj(R.ta[2 * p + 1], tw);
+                        const bool d0 = (off >> (2 * p)) & 1u, d1 = (off >> (2 * p + 1)) & 1u;
+                        pair2<false>(nx[p], ny[p], nz[p], f2(xb.x), f2(xb.y), f2(xb.z), el,
+                                     make_float2(d0 ? 0.f : t0.x, d1 ? 0.f : t1.x),
+                                     make_float2(d0 ? 0.f : t0.y, d1 ? 0.f : t1.y), gx[p], gy[p], gz[p], vel, wvdw);
+                    } else {   // A = B = 0 with every solute type: the Coulomb term alone, bit for bit
+                        pair2_coul(nx[p], ny[p], nz[p], f2(xb.x), f2(xb.y), f2(xb.z), el, gx[p], gy[p], gz[p], vel);
+                    }
+                    wel = __fadd2_rn(wel, vel);
                 }
-              }
+            }
+        }
+        }
+        const float rwel = wel.x + wel.y, rwvdw = wvdw.x + wvdw.y;
+        // plain partners: LJ code 1 with every row atom, no excluded or 1-4
+        // pair; with the geometric rule A and B are the products of the atoms'
+        // FP32 code-1 factors (the type table holds the same products).  The
+        // next entry's partner data is loaded one iteration ahead, across the
+        // prefetched chunks
+        {
+          const int niter = (npf + kWarp - 1) / kWarp;
+          for (int it = 0; it < niter; ++it) {
+            const int k = it * kWarp + lane;
+            const float4 xb = BOX ? at_image(m, xbn, xsw, xrn) : xbn;
+            const float2 fj = fjn;
+            const int tj = tjn;
+            if (it % kIter == kIter - 1 && it + 1 < niter) {   // the next chunk, fetched a chunk ago
+                cp_async_wait<0>();
+                __syncwarp();
+            }
+            if (k + kWarp < npf) load_pf(k + kWarp);
+            if (it % kIter == kIter - 1) {   // this chunk is consumed
+                __syncwarp();
+                if (it / kIter + 2 < nfchunk) fetch_pf(it / kIter + 2);
+                cp_async_commit();
+            }
+            if (k < npf) {
+              const float2 bx = f2(xb.x), by = f2(xb.y), bz = f2(xb.z), bq = f2(xb.w);
 #pragma unroll
               for (int p = 0; p < NP; ++p) {
-                  f[2 * p][0] = gx[p].x;
-                  f[2 * p][1] = gy[p].x;
-                  f[2 * p][2] = gz[p].x;
-                  f[2 * p + 1][0] = gx[p].y;
-                  f[2 * p + 1][1] = gy[p].y;
-                  f[2 * p + 1][2] = gz[p].y;
-              }
-              rpel += pel.x + pel.y;
-              rpvdw += pvdw.x + pvdw.y;
-            } else {
-              for (int k = lane; k < n; k += kWarp) {
-                const float4 xb = xbn;
-                const int tj = tjn;
-                if (k + kWarp < n) {
-                    const int jn = buf[k + kWarp];
-                    tjn = m.iac[jn];
-                    xbn = xq[jn];
-                    if (BOX) xbn = at_image(m, xbn, xsw, xq[m.swat[jn]]);
+                if (2 * p >= n1) break;   // warp-uniform
+                float2 vel;
+                if constexpr (GEOM) {
+                    const float4 fab = *reinterpret_cast<const float4*>(R.fab[p][0]);
+                    pair2<true>(nx[p], ny[p], nz[p], bx, by, bz, __fmul2_rn(q2[p], bq),
+                                __fmul2_rn(make_float2(fab.x, fab.y), f2(fj.x)),
+                                __fmul2_rn(make_float2(fab.z, fab.w), f2(fj.y)), gx[p], gy[p], gz[p], vel, pvdw);
+                } else {
+                    const float4 t0 = lj(R.ta[2 * p], tj), t1 = lj(R.ta[2 * p + 1], tj);
+                    const bool d0 = (off >> (2 * p)) & 1u, d1 = (off >> (2 * p + 1)) & 1u;
+                    pair2<false>(nx[p], ny[p], nz[p], bx, by, bz, __fmul2_rn(q2[p], bq),
+                                 make_float2(d0 ? 0.f : t0.x, d1 ? 0.f : t1.x), make_float2(d0 ? 0.f : t0.y, d1 ? 0.f : t1.y),
+                                 gx[p], gy[p], gz[p], vel, pvdw);
                 }
-#pragma unroll
-                for (int a = 0; a < MAXG; ++a) {
-                    if (qa[a]) continue;   // warp-uniform
-                    float4 p = lj(ta[a], tj);
-                    float vel, vdw;
-                    pair_f(xa[a], xb, p.x, p.y, xa[a].w * xb.w, true, f[a][0], f[a][1], f[a][2], vel, vdw);
-                    rpel += vel;
-                    rpvdw += vdw;
-                }
+                pel = __fadd2_rn(pel, vel);
               }
             }
-            __syncwarp();   // this buffer is refilled two chunks later
           }
+          cp_async_wait<0>();
         }
-        __syncwarp();   // sh_pw is refilled by the next row
+        __syncwarp();   // the staging buffers are refilled by the next row
+        const float rpel = pel.x + pel.y, rpvdw = pvdw.x + pvdw.y;
         // The row owns its atoms' pp and pw gradient and its energies: FP32
         // warp sums in a fixed shuffle order, stored without atomics
         // (k_apply_fixed converts each atom's sum once to 64-bit fixed point
@@ -3729,8 +3751,10 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
             float gv[32];
 #pragma unroll
             for (int a = 0; a < 8; ++a) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) gv[3 * a + c] = a < MAXG ? f[a < MAXG ? a : 0][c] : 0.f;
+                const int p = a < MAXG ? a / 2 : 0;
+                gv[3 * a] = a < MAXG ? (a % 2 ? gx[p].y : gx[p].x) : 0.f;
+                gv[3 * a + 1] = a < MAXG ? (a % 2 ? gy[p].y : gy[p].x) : 0.f;
+                gv[3 * a + 2] = a < MAXG ? (a % 2 ? gz[p].y : gz[p].x) : 0.f;
             }
             gv[24] = 0.5f * rpel, gv[25] = 0.5f * rpvdw, gv[26] = rwel, gv[27] = rwvdw;
             gv[28] = gv[29] = gv[30] = gv[31] = 0.f;
@@ -3752,13 +3776,15 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, GEOM>()) k_rows_sol
 #pragma unroll
             for (int a = 0; a < MAXG; ++a) {
                 if (a >= n1) break;   // warp-uniform
-                float v0 = warp_sum(f[a][0]), v1 = warp_sum(f[a][1]), v2 = warp_sum(f[a][2]);
+                const int p = a / 2;
+                const float v0 = warp_sum(a % 2 ? gx[p].y : gx[p].x), v1 = warp_sum(a % 2 ? gy[p].y : gy[p].x),
+                            v2 = warp_sum(a % 2 ? gz[p].y : gz[p].x);
                 if (lane == 0) {
-                    int i = m.gatom[a0 + a];
-                    float* fr = s.frow + 3 * i;
-                    fr[0] = qa[a] ? 0.f : v0;
-                    fr[1] = qa[a] ? 0.f : v1;
-                    fr[2] = qa[a] ? 0.f : v2;
+                    const bool q = (off >> a) & 1u;
+                    float* fr = s.frow + 3 * m.gatom[a0 + a];
+                    fr[0] = q ? 0.f : v0;
+                    fr[1] = q ? 0.f : v1;
+                    fr[2] = q ? 0.f : v2;
                 }
             }
         }

@@ -2346,7 +2346,11 @@ __global__ void __launch_bounds__(256) k_qq(DevModel m, const DevState* __restri
     }
 }
 
-// lrf_taylor, src/nonbondene.f90:507-571 (FP64 in both forms)
+// lrf_taylor, src/nonbondene.f90:507-571 (FP64 in both forms).  The FP64 pipe
+// bounds it; phi2 and phi3 are symmetric (lrf_expand), so their 6 and 10
+// distinct coefficients against the products of dr take 20 loads per atom
+// where the full sums took 43, and fewer operations (51 windows of the 25 A
+// sphere 49.0 -> 46.3 us).
 template <bool MIX>
 __global__ void __launch_bounds__(256) k_lrf_taylor(DevModel m, const DevState* __restrict__ states, const int* __restrict__ iwhich) {
     const DevState& s = states[blockIdx.y];
@@ -2355,25 +2359,23 @@ __global__ void __launch_bounds__(256) k_lrf_taylor(DevModel m, const DevState* 
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.natom; i += gridDim.x * blockDim.x) {
         if (m.excl[i] || m.iqatom[i] >= 0 || iwhich[i] < 0) continue;   // (an atom in no group: no record)
         const double* L = s.lrf + (size_t)iwhich[i] * kLrfLen;
-        double dx = L[0] - s.x[3 * i], dy = L[1] - s.x[3 * i + 1], dz = L[2] - s.x[3 * i + 2];
-        const double* p1 = L + 4;
+        const double dx = L[0] - s.x[3 * i], dy = L[1] - s.x[3 * i + 1], dz = L[2] - s.x[3 * i + 2];
         const double* p2 = L + 7;    // p2[3a + c]
-        const double* p3 = L + 16;   // p3[3m + c]
-        double t0 = dx * p2[0] + dy * p2[1] + dz * p2[2];
-        double t1 = dx * p2[3] + dy * p2[4] + dz * p2[5];
-        double t2 = dx * p2[6] + dy * p2[7] + dz * p2[8];
-        double V = L[3] + (dx * p1[0] + dy * p1[1] + dz * p1[2]) + 0.5 * (dx * t0 + dy * t1 + dz * t2);
+        const double* p3 = L + 16;   // p3[9a + 3b + c]
+        const double xy2 = p2[1], xz2 = p2[2], yz2 = p2[5];
+        // phi2 dr
+        const double t0 = dx * p2[0] + dy * xy2 + dz * xz2;
+        const double t1 = dx * xy2 + dy * p2[4] + dz * yz2;
+        const double t2 = dx * xz2 + dy * yz2 + dz * p2[8];
+        const double V = L[3] + (dx * L[4] + dy * L[5] + dz * L[6]) + 0.5 * (dx * t0 + dy * t1 + dz * t2);
         elrf.add(0.5 * m.crg[i] * V);
-        double df[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const double* q = p3 + 9 * a;
-            double u0 = dx * q[0] + dy * q[1] + dz * q[2];
-            double u1 = dx * q[3] + dy * q[4] + dz * q[5];
-            double u2 = dx * q[6] + dy * q[7] + dz * q[8];
-            df[a] = p1[a] + (dx * p2[3 * a] + dy * p2[3 * a + 1] + dz * p2[3 * a + 2]) +
-                    0.5 * (dx * u0 + dy * u1 + dz * u2);
-        }
+        // 0.5 dr phi3 dr
+        const double hxx = 0.5 * dx * dx, hyy = 0.5 * dy * dy, hzz = 0.5 * dz * dz, xy = dx * dy, xz = dx * dz, yz = dy * dz;
+        const double xxy = p3[1], xxz = p3[2], xyy = p3[4], xyz = p3[5], xzz = p3[8], yyz = p3[14], yzz = p3[17];
+        const double df[3] = {
+            L[4] + t0 + (p3[0] * hxx + xxy * xy + xxz * xz + xyy * hyy + xyz * yz + xzz * hzz),
+            L[5] + t1 + (xxy * hxx + xyy * xy + xyz * xz + p3[13] * hyy + yyz * yz + yzz * hzz),
+            L[6] + t2 + (xxz * hxx + xyz * xy + xzz * xz + yyz * hyy + yzz * yz + p3[26] * hzz)};
         double q = m.crg[i];
         if constexpr (!MIX) acc.grad(i, -df[0] * q, -df[1] * q, -df[2] * q);
         else acc.gradd(i, -df[0] * q, -df[1] * q, -df[2] * q);

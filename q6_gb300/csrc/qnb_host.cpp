@@ -144,6 +144,7 @@ struct qnb_context {
         int64_t nlaunch = 0;
         std::vector<Pending> prof;   // profiled graphs: the event pairs their nodes record
     } gslot[2][2];                   // [watpol update step][profiled]
+    GraphSlot gslot_host[2];         // [watpol update step]: qnb_pot_energy_step with its host transfers
     bool capturing = false;          // timed() is recording into a graph capture
     std::vector<Pending> cap_pending;
     bool qenv_pending = false;     // mixed form: fq not yet added into d
@@ -1569,6 +1570,8 @@ int qnb_destroy(qnb_context* c) {
                 cudaEventDestroy(p.b);
             }
         }
+    for (auto& g : c->gslot_host)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->h_e) cudaFreeHost(c->h_e);
     if (c->h_adj) cudaFreeHost(c->h_adj);
@@ -1958,10 +1961,9 @@ int capture_graph(cudaStream_t st, cudaGraphExec_t* exec, F&& f) {
 // pairs are queued for collect_profile, which must run (qnb_profile_collect)
 // before the next replay re-records them -- run_compute collects first if the
 // caller did not.
-int run_compute(qnb_context* c, double Tfree, int istep) {
-    if (!c->use_graphs) return enqueue_compute(c, Tfree, istep);
-    const int prof = c->profiling ? 1 : 0;
-    auto& g = c->gslot[watpol_update_step(c, istep) ? 1 : 0][prof];
+template <typename F>
+int replay(qnb_context* c, qnb_context::GraphSlot& g, double Tfree, F&& enqueue) {
+    const bool prof = c->profiling;
     for (auto& p : c->pending)
         if (p.owned) {   // an earlier replay's times were not collected yet
             collect_profile(c);
@@ -1978,7 +1980,7 @@ int run_compute(qnb_context* c, double Tfree, int istep) {
         int64_t l0 = c->launches;
         c->capturing = true;
         c->cap_pending.clear();
-        int rc = capture_graph(c->stream, &g.exec, [&] { return enqueue_compute(c, Tfree, istep); });
+        int rc = capture_graph(c->stream, &g.exec, enqueue);
         c->capturing = false;
         g.prof.swap(c->cap_pending);
         if (rc) {
@@ -1999,6 +2001,26 @@ int run_compute(qnb_context* c, double Tfree, int istep) {
     c->launches += g.nlaunch;
     if (prof) c->pending.insert(c->pending.end(), g.prof.begin(), g.prof.end());
     return QNB_OK;
+}
+int run_compute(qnb_context* c, double Tfree, int istep) {
+    if (!c->use_graphs) return enqueue_compute(c, Tfree, istep);
+    return replay(c, c->gslot[watpol_update_step(c, istep) ? 1 : 0][c->profiling ? 1 : 0], Tfree,
+                  [&] { return enqueue_compute(c, Tfree, istep); });
+}
+// The evaluation of a single-window context between its host transfers: x
+// from h_stage, the gradient (cleared on the device) into h_stage, the energies
+// into h_e, all in one graph.
+int run_host_step(qnb_context* c, double Tfree, int istep) {
+    const int n = 3 * c->natom;
+    auto f = [&]() -> int {
+        launch_host_in(c->h_stage, c->st[0].x, n, c->stream);
+        TRY(enqueue_compute(c, Tfree, istep));
+        launch_host_out(c->st[0].d, c->h_stage, n, c->e_all, c->h_e, 2 * kNumE * c->nwin, c->stream);
+        c->launches += 2;
+        return check_launch();
+    };
+    if (!c->use_graphs || c->profiling) return f();
+    return replay(c, c->gslot_host[watpol_update_step(c, istep) ? 1 : 0], Tfree, f);
 }
 
 // adds the energies of every window, as read into e, into E / EQ / Erst
@@ -2061,13 +2083,9 @@ int qnb_pot_energy_step(qnb_context* c, const double* x, double* d, double Tfree
     if (c->nwin != 1) return fail(QNB_ERR_ARG, "single-window contexts only (batches: qnb_compute_dev)");
     CU(cudaSetDevice(c->device));
     if (!c->lists_built) return fail(QNB_ERR_STATE, "pair lists not built");
-    TRY(stage_x(c, x));
-    TRY(run_compute(c, Tfree, istep));   // gradient applied into window 0's FP64 accumulator
     const size_t n = 3 * (size_t)c->natom;
-    // stream order: the coordinate copy out of h_stage precedes this copy into it
-    CU(cudaMemcpyAsync(c->h_stage, c->st[0].d, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemsetAsync(c->st[0].d, 0, n * sizeof(double), c->stream));
-    TRY(enqueue_energies(c, 1));
+    memcpy(c->h_stage, x, n * sizeof(double));
+    TRY(run_host_step(c, Tfree, istep));
     CU(cudaStreamSynchronize(c->stream));
     for (size_t k = 0; k < n; ++k) d[k] += c->h_stage[k];
     const long long* fx = (const long long*)(c->h_e + (size_t)kNumE * c->nwin);

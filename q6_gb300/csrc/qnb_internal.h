@@ -275,6 +275,9 @@ struct Launch {
     const Tune& tu;
 };
 
+void launch_host_in(const double* h, double* x, int n, cudaStream_t st);
+// d to h, d cleared; e to he
+void launch_host_out(double* d, double* h, int n, const double* e, double* he, int ne, cudaStream_t st);
 void launch_pack(const Launch& L);
 void launch_reset_counts(const Launch& L, unsigned keep_mask);
 void launch_group_centres(const Launch& L);

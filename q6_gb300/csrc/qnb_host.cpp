@@ -117,7 +117,6 @@ struct qnb_context {
     uint8_t* d_qnear = nullptr;
     int* d_wsw = nullptr;
     uint8_t* d_heavy_solv = nullptr;
-    double* d_shell_tsum = nullptr;
     std::vector<void*> allocs;
     bool lists_built = false, qp_done = false, qw_done = false;
     bool diag_valid = false;       // mixed form: half lists for inspection built from x_build
@@ -1039,7 +1038,9 @@ int alloc_state(qnb_context* c) {
         TRY(c->alloc(&s.rank, (size_t)std::max(1, m.nwat)));
         TRY(c->alloc(&s.n_insh, (size_t)kMaxShell));
         TRY(c->alloc(&s.wstate, (size_t)3 * kMaxShell));
-        TRY(c->alloc(&s.shell_tsum, (size_t)kMaxShell));
+        TRY(c->alloc(&s.wp_count, (size_t)kMaxShell + 1));
+        CU(cudaMemset(s.n_insh, 0, sizeof(int) * kMaxShell));
+        CU(cudaMemset(s.wp_count, 0, sizeof(int) * (kMaxShell + 1)));
         TRY(c->alloc(&s.theta_sorted, (size_t)kMaxShell * std::max(1, m.nwat)));
         s.adj = c->adj_all + (size_t)3 * std::max(1, m.nqat * m.S) * w;
         TRY(c->alloc(&s.shell_list, (size_t)kMaxShell * std::max(1, m.nwat)));
@@ -1908,10 +1909,9 @@ int enqueue_compute(qnb_context* c, double Tfree, int istep) {
             c->launches++;
         }
         if (c->have_solv) {
-            timed_on(c, B.st, K_RESTRAIN, [&] { launch_restrain_solvent(B, c->solv, Tfree, c->mixed, c->d_wsw, c->d_heavy_solv); });
-            c->launches++;
             int nl = 0;
-            timed_on(c, B.st, K_WATPOL, [&] { nl = launch_watpol(B, c->solv, istep, 1, c->mixed); });
+            timed_on(c, B.st, K_RESTRAIN, [&] { nl += launch_boundary_theta(B, c->solv, Tfree, istep, c->mixed, c->d_wsw, c->d_heavy_solv); });
+            timed_on(c, B.st, K_WATPOL, [&] { nl += launch_boundary_watpol(B, c->solv, c->mixed); });
             c->launches += nl;
         }
         return check_launch();

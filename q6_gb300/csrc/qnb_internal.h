@@ -225,10 +225,10 @@ struct DevState {
     double* wvec;        // [nwat][8] unit dipole / radial vectors and lengths of the last md call
     int* shell;          // [nwat] shell or -1
     int* rank;           // [nwat]
-    int* n_insh;         // [kMaxShell]
+    int* n_insh;         // [kMaxShell] waters per shell of the last md call
+    int* wp_count;       // [kMaxShell+1] this call's counts, and its finished blocks; zero between calls
     int* shell_list;     // [kMaxShell][nwat] waters per shell
     double* wstate;      // [3*kMaxShell]: theta_corr, avtheta, avn_insh
-    double* shell_tsum;  // [kMaxShell] per-step sum of theta per shell (in sorted order)
     double* theta_sorted;   // [kMaxShell][nwat] the shell's thetas by rank
 };
 
@@ -324,6 +324,11 @@ struct SolventDev {
 void launch_restrain_solvent(const Launch& L, const SolventDev& p, double Tfree, int mixed, const int* wsw,
                              const uint8_t* heavy_solv);
 int launch_watpol(const Launch& L, const SolventDev& p, int istep, int md, int mixed);
+// the step's boundary terms in two launches: the radial restraint with watpol's
+// angles (and its theta_corr update, at an update step), then the rest of watpol
+int launch_boundary_theta(const Launch& L, const SolventDev& p, double Tfree, int istep, int mixed, const int* wsw,
+                          const uint8_t* heavy_solv);
+int launch_boundary_watpol(const Launch& L, const SolventDev& p, int mixed);
 
 void launch_q_adjoint(const Launch& L);
 

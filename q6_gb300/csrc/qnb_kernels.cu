@@ -2411,72 +2411,81 @@ __global__ void k_apply_fixed(int n, const DevState* __restrict__ states, int ro
 // Spherical-boundary solvent terms (FP64 in both forms)
 // =============================================================================
 
-// restrain_solvent, src/nonbondene.f90:6466-6544
+// restrain_solvent, src/nonbondene.f90:6466-6544, of water w
+template <bool MIX>
+__device__ __forceinline__ void restrain_water(const DevModel& m, const DevState& s, const SolventDev& p, double shift, float r0f,
+                                               const int* __restrict__ wsw, const uint8_t* __restrict__ heavy_solv, int w,
+                                               const Acc<MIX>& acc, ESum<MIX>& er) {
+    int isw = wsw[w];
+    if (m.excl[isw]) return;
+    int first = m.nat_solute + m.sa * w;
+    for (int is = 0; is < m.sa; ++is) {
+        int i, idist;
+        if (m.sa == 3) {
+            if (is > 0) break;
+            i = idist = isw;
+        } else {
+            if (!heavy_solv[is]) continue;
+            idist = first;
+            i = first + is;
+        }
+        if constexpr (MIX) {   // FP32 arithmetic; the two branches meet with equal value and slope at db = 0
+            float4 xa = s.xq[idist];
+            float ux = xa.x + m.wcoff[0], uy = xa.y + m.wcoff[1], uz = xa.z + m.wcoff[2];
+            float bf = sqrtf(ux * ux + uy * uy + uz * uz);
+            float dbf = bf - r0f;
+            float ef, dvf;
+            if (dbf > 0.f) {
+                ef = 0.5f * p.fk_wspheref * (dbf * dbf) - p.Dwmzf;
+                dvf = p.fk_wspheref * dbf / bf;
+            } else if (bf > 0.f) {
+                float fexp = expf(p.awmzf * dbf);
+                ef = p.Dwmzf * (fexp * fexp - 2.f * fexp);
+                dvf = -2.f * p.Dwmzf * p.awmzf * (fexp - fexp * fexp) / bf;
+            } else {
+                ef = 0.f;
+                dvf = 0.f;
+            }
+            acc.grad_alu(i, ux * dvf, uy * dvf, uz * dvf);
+            er.add_alu(ef);
+            continue;
+        }
+        double vx = s.x[3 * idist] - m.xwcent[0], vy = s.x[3 * idist + 1] - m.xwcent[1],
+               vz = s.x[3 * idist + 2] - m.xwcent[2];
+        double b = sqrt(vx * vx + vy * vy + vz * vz);
+        double db = b - (p.rwat - shift);
+        double erst, dv;
+        if (db > 0.0) {
+            erst = 0.5 * p.fk_wsphere * (db * db) - p.Dwmz;
+            dv = p.fk_wsphere * db / b;
+        } else if (b > 0.0) {
+            double fexp = exp(p.awmz * db);
+            erst = p.Dwmz * (fexp * fexp - 2.0 * fexp);
+            dv = -2.0 * p.Dwmz * p.awmz * (fexp - fexp * fexp) / b;
+        } else {
+            erst = 0.0;
+            dv = 0.0;
+        }
+        if constexpr (!MIX) acc.grad(i, vx * dv, vy * dv, vz * dv);
+        else acc.gradd(i, vx * dv, vy * dv, vz * dv);
+        er.add(erst);
+    }
+}
+// the radial restraint's shift; tdev: from the window's Tfree of its last MD
+// temperature(), as the host computes it
+__device__ __forceinline__ double restrain_shift(const DevState& s, const SolventDev& p, double shift, int tdev) {
+    return !tdev ? shift : ((p.fk_wsphere != 0.0) ? sqrt(p.boltz * *s.md_tfree / p.fk_wsphere) : 0.0);
+}
 template <bool MIX>
 __global__ void k_restrain_solvent(DevModel m, const DevState* __restrict__ states, SolventDev p, double shift,
                                    const int* __restrict__ wsw, const uint8_t* __restrict__ heavy_solv, int tdev) {
     const DevState& s = states[blockIdx.y];
-    if (tdev)   // the window's Tfree from its last MD temperature(), as the host computes the shift
-        shift = (p.fk_wsphere != 0.0) ? sqrt(p.boltz * *s.md_tfree / p.fk_wsphere) : 0.0;
+    shift = restrain_shift(s, p, shift, tdev);
     Acc<MIX> acc = make_acc<MIX>(s);
     ESum<MIX> er;
     const float r0f = (float)(p.rwat - shift);
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < m.nwat; w += gridDim.x * blockDim.x) {
-        int isw = wsw[w];
-        if (m.excl[isw]) continue;
-        int first = m.nat_solute + m.sa * w;
-        for (int is = 0; is < m.sa; ++is) {
-            int i, idist;
-            if (m.sa == 3) {
-                if (is > 0) break;
-                i = idist = isw;
-            } else {
-                if (!heavy_solv[is]) continue;
-                idist = first;
-                i = first + is;
-            }
-            if constexpr (MIX) {   // FP32 arithmetic; the two branches meet with equal value and slope at db = 0
-                float4 xa = s.xq[idist];
-                float ux = xa.x + m.wcoff[0], uy = xa.y + m.wcoff[1], uz = xa.z + m.wcoff[2];
-                float bf = sqrtf(ux * ux + uy * uy + uz * uz);
-                float dbf = bf - r0f;
-                float ef, dvf;
-                if (dbf > 0.f) {
-                    ef = 0.5f * p.fk_wspheref * (dbf * dbf) - p.Dwmzf;
-                    dvf = p.fk_wspheref * dbf / bf;
-                } else if (bf > 0.f) {
-                    float fexp = expf(p.awmzf * dbf);
-                    ef = p.Dwmzf * (fexp * fexp - 2.f * fexp);
-                    dvf = -2.f * p.Dwmzf * p.awmzf * (fexp - fexp * fexp) / bf;
-                } else {
-                    ef = 0.f;
-                    dvf = 0.f;
-                }
-                acc.grad_alu(i, ux * dvf, uy * dvf, uz * dvf);
-                er.add_alu(ef);
-                continue;
-            }
-            double vx = s.x[3 * idist] - m.xwcent[0], vy = s.x[3 * idist + 1] - m.xwcent[1],
-                   vz = s.x[3 * idist + 2] - m.xwcent[2];
-            double b = sqrt(vx * vx + vy * vy + vz * vz);
-            double db = b - (p.rwat - shift);
-            double erst, dv;
-            if (db > 0.0) {
-                erst = 0.5 * p.fk_wsphere * (db * db) - p.Dwmz;
-                dv = p.fk_wsphere * db / b;
-            } else if (b > 0.0) {
-                double fexp = exp(p.awmz * db);
-                erst = p.Dwmz * (fexp * fexp - 2.0 * fexp);
-                dv = -2.0 * p.Dwmz * p.awmz * (fexp - fexp * fexp) / b;
-            } else {
-                erst = 0.0;
-                dv = 0.0;
-            }
-            if constexpr (!MIX) acc.grad(i, vx * dv, vy * dv, vz * dv);
-            else acc.gradd(i, vx * dv, vy * dv, vz * dv);
-            er.add(erst);
-        }
-    }
+    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < m.nwat; w += gridDim.x * blockDim.x)
+        restrain_water<MIX>(m, s, p, shift, r0f, wsw, heavy_solv, w, acc, er);
     er.flush(acc, E_RST_RAD);
 }
 
@@ -2549,10 +2558,7 @@ __device__ __forceinline__ int watpol_shell(const SolventDev& p, double rcd) {
 // water is decided exactly: the FP32 distance decides away from the shell
 // radii, the FP64 distance within 2e-4 of one.
 template <bool MIX>
-__global__ void k_watpol_theta(DevModel m, const DevState* __restrict__ states, SolventDev p) {
-    const DevState& s = states[blockIdx.y];
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= m.nwat) return;
+__device__ __forceinline__ void watpol_theta(const DevModel& m, const DevState& s, const SolventDev& p, int w) {
     s.shell[w] = -1;
     s.theta[w] = 0.0;
     s.rkey[w] = 0.0;
@@ -2608,29 +2614,158 @@ __global__ void k_watpol_theta(DevModel m, const DevState* __restrict__ states, 
     int is = watpol_shell(p, rcd);
     if (is >= 0) {
         s.shell[w] = is;
-        int k = atomicAdd(s.n_insh + is, 1);
+        int k = atomicAdd(s.wp_count + is, 1);
         s.shell_list[(size_t)is * m.nwat + k] = w;
     }
 }
+// theta and shell of every water, with RST the radial restraint in the same
+// pass.  FP64 operations per water: blocks of one warp spread over the SMs.
+template <bool MIX, bool RST>
+__global__ void __launch_bounds__(32) k_watpol_theta(DevModel m, const DevState* __restrict__ states, SolventDev p, double shift,
+                                                     const int* __restrict__ wsw, const uint8_t* __restrict__ heavy_solv,
+                                                     int tdev) {
+    const DevState& s = states[blockIdx.y];
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w < m.nwat) watpol_theta<MIX>(m, s, p, w);
+    if constexpr (RST) {
+        shift = restrain_shift(s, p, shift, tdev);
+        Acc<MIX> acc = make_acc<MIX>(s);
+        ESum<MIX> er;
+        if (w < m.nwat) restrain_water<MIX>(m, s, p, shift, (float)(p.rwat - shift), wsw, heavy_solv, w, acc, er);
+        er.flush(acc, E_RST_RAD);
+    }
+}
 
-// stable selection order of src/nonbondene.f90:6612-6628: rank = number of
-// waters of the same shell with a smaller key, ties broken by water index
-// (the reference scans the shell in water order and keeps the first minimum).
+// theta_corr update every itdis steps, src/nonbondene.f90:6630-6645
+__global__ void k_watpol_update(SolventDev p, const DevState* __restrict__ states) {
+    double* wstate = states[blockIdx.y].wstate;
+    int is = threadIdx.x;
+    if (is >= p.nshell) return;
+    double* tc = wstate;
+    double* av = wstate + kMaxShell;
+    double* an = wstate + 2 * kMaxShell;
+    av[is] = av[is] / p.itdis;
+    an[is] = an[is] / p.itdis;
+    tc[is] = tc[is] + av[is] - acos(p.cstb[is]);
+    av[is] = 0.0;
+    an[is] = 0.0;
+}
+
+// energy and gradient of water w, the il-th of n in shell sh,
+// src/nonbondene.f90:6646-6742.  STORED: the vectors and theta of this call's
+// k_watpol_theta are current (md); otherwise they are recomputed from the
+// coordinates, as the reference does in every call.
+template <bool MIX, bool STORED>
+__device__ __forceinline__ void watpol_force(const DevModel& m, const DevState& s, const SolventDev& p, int w, int sh, int n,
+                                             int il, const Acc<MIX>& acc, ESum<MIX>& ep) {
+    const double pi = 3.14159265358979323846;
+    if constexpr (MIX) {
+        if (m.sa == 3) {   // FP32 arithmetic (the theta kernel's FP32 vectors when STORED)
+            const float pif = 3.14159265f;
+            float arg = 1.f + (1.f - 2.f * (float)il) / (float)n;
+            float t0 = acosf(arg);
+            t0 = t0 - 3.f * sinf(t0) * p.cstbf[sh] / 2.f;
+            t0 = fminf(fmaxf(t0, 0.f), pif);
+            float th = (float)s.theta[w];
+            float dth = th - t0 + (float)s.wstate[sh];
+            ep.add_alu(0.5f * p.fkwpolf * dth * dth);
+            float dv = p.fkwpolf * dth;
+            float rmx, rmy, rmz, rm, rcx, rcy, rcz, rc;
+            if constexpr (STORED) {
+                const double* v = s.wvec + 8 * (size_t)w;
+                rmx = (float)v[0]; rmy = (float)v[1]; rmz = (float)v[2]; rm = (float)v[3];
+                rcx = (float)v[4]; rcy = (float)v[5]; rcz = (float)v[6]; rc = (float)v[7];
+            } else {
+                water_vectors_f(m, s.xq, w, rmx, rmy, rmz, rm, rcx, rcy, rcz, rc);
+            }
+            float scp = fminf(1.f, fmaxf(-1.f, rmx * rcx + rmy * rcy + rmz * rcz));
+            float f0 = STORED ? sinf(th) : sinf(acosf(scp));
+            if (fabsf(f0) < 1.0e-10f) f0 = 1.0e-10f;
+            f0 = dv * (-1.f / f0);
+            float f3x = (rcx - rmx * scp) / rm, f3y = (rcy - rmy * scp) / rm, f3z = (rcz - rmz * scp) / rm;
+            float f2x = (rmx - rcx * scp) / rc, f2y = (rmy - rcy * scp) / rc, f2z = (rmz - rcz * scp) / rc;
+            int i = m.nat_solute + 3 * w;
+            acc.grad_alu(i, (-2.f * f3x + f2x) * f0, (-2.f * f3y + f2y) * f0, (-2.f * f3z + f2z) * f0);
+            acc.grad_alu(i + 1, f3x * f0, f3y * f0, f3z * f0);
+            acc.grad_alu(i + 2, f3x * f0, f3y * f0, f3z * f0);
+            return;
+        }
+    }
+    double arg = 1.0 + (1.0 - 2.0 * (double)il) / (double)n;
+    double t0 = acos(arg);
+    t0 = t0 - 3.0 * sin(t0) * p.cstb[sh] / 2.0;
+    if (t0 < 0.0) t0 = 0.0;
+    if (t0 > pi) t0 = pi;
+    double th = s.theta[w];
+    double dth = th - t0 + s.wstate[sh];
+    ep.add(0.5 * p.fkwpol * dth * dth);
+    double dv = p.fkwpol * dth;
+    double rmx, rmy, rmz, rm, rcx, rcy, rcz, rc, f0;
+    if constexpr (STORED) {
+        const double* v = s.wvec + 8 * (size_t)w;
+        rmx = v[0]; rmy = v[1]; rmz = v[2]; rm = v[3];
+        rcx = v[4]; rcy = v[5]; rcz = v[6]; rc = v[7];
+    } else {
+        water_vectors(m, s.x, w, rmx, rmy, rmz, rm, rcx, rcy, rcz, rc);
+    }
+    double scp = rmx * rcx + rmy * rcy + rmz * rcz;
+    scp = fmin(1.0, fmax(-1.0, scp));
+    // theta = acos(scp) of this same scp when STORED
+    f0 = STORED ? sin(th) : sin(acos(scp));
+    if (fabs(f0) < 1.0e-10) f0 = 1.0e-10;
+    f0 = dv * (-1.0 / f0);
+    double f1x = (rcx - rmx * scp) * -2.0 / rm, f1y = (rcy - rmy * scp) * -2.0 / rm,
+           f1z = (rcz - rmz * scp) * -2.0 / rm;
+    double f3x = (rcx - rmx * scp) / rm, f3y = (rcy - rmy * scp) / rm, f3z = (rcz - rmz * scp) / rm;
+    double f2x = (rmx - rcx * scp) / rc, f2y = (rmy - rcy * scp) / rc, f2z = (rmz - rcz * scp) / rc;
+    int i = m.nat_solute + m.sa * w;
+    if constexpr (!MIX) acc.grad(i, (f1x + f2x) * f0, (f1y + f2y) * f0, (f1z + f2z) * f0);
+    else acc.gradd(i, (f1x + f2x) * f0, (f1y + f2y) * f0, (f1z + f2z) * f0);
+    for (int k = 1; k < m.sa; ++k) {
+        if constexpr (!MIX) acc.grad(i + k, f3x * f0, f3y * f0, f3z * f0);
+        else acc.gradd(i + k, f3x * f0, f3y * f0, f3z * f0);
+    }
+}
+// a call without md: shells and ranks of the last call with it
+template <bool MIX>
+__global__ void k_watpol_force(DevModel m, const DevState* __restrict__ states, SolventDev p) {
+    const DevState& s = states[blockIdx.y];
+    Acc<MIX> acc = make_acc<MIX>(s);
+    ESum<MIX> ep;
+    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < m.nwat; w += gridDim.x * blockDim.x) {
+        const int sh = s.shell[w];
+        if (sh >= 0) watpol_force<MIX, false>(m, s, p, w, sh, s.n_insh[sh], s.rank[w] + 1, acc, ep);
+    }
+    ep.flush(acc, E_RST_POL);
+}
+
+// The selection order, the forces and the running averages of an md call.
+// Stable selection order of src/nonbondene.f90:6612-6628: rank = number of
+// waters of the same shell with a smaller key, ties broken by water index (the
+// reference scans the shell in water order and keeps the first minimum).
 // kRankParts blocks per shell: each stages the whole shell's keys in shared
-// memory and ranks its share of the waters, one warp per water with the
-// lanes splitting the comparisons.
+// memory, ranks its share of the waters, one warp per water with the lanes
+// splitting the comparisons, and then takes its waters' forces, one thread
+// each.  The window's last block to finish sums each shell's thetas by rank
+// (one warp per shell, a fixed order, whatever order the shell list was filled
+// in; 6652-6666, 6738-6741) into the running averages and hands the counts
+// over.  As five kernels (reset, rank, force, average and the radial restraint
+// beside theta) the boundary branch was the longest of a small system's step.
 constexpr int kRankBlock = 256;
-constexpr int kRankParts = 4;
-__global__ void __launch_bounds__(kRankBlock) k_watpol_rank(DevModel m, const DevState* __restrict__ states) {
+constexpr int kRankParts = 8;
+template <bool MIX>
+__global__ void __launch_bounds__(kRankBlock) k_watpol_rank_force(DevModel m, const DevState* __restrict__ states, SolventDev p) {
     const DevState& s = states[blockIdx.y];
     // the keys (theta, or 1 - cos theta in the mixed form) are >= 0, so the
     // bit patterns of the doubles order like the values;
     // integer compares keep the sort off the (narrow) FP64 pipe
     __shared__ long long th[1024];
     __shared__ int ww[1024];
-    const int sh = blockIdx.x / kRankParts, part = blockIdx.x % kRankParts, n = s.n_insh[sh];
+    __shared__ bool last;
+    const int sh = blockIdx.x / kRankParts, part = blockIdx.x % kRankParts, n = s.wp_count[sh];
     const int* L = s.shell_list + (size_t)sh * m.nwat;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int nw = kRankBlock / kWarp;
     for (int base = 0; base < n; base += 1024) {
         int cn = min(1024, n - base);
         __syncthreads();
@@ -2658,143 +2793,45 @@ __global__ void __launch_bounds__(kRankBlock) k_watpol_rank(DevModel m, const De
             }
         }
     }
-}
-
-__global__ void k_watpol_reset(const DevState* __restrict__ states) {
-    const DevState& s = states[blockIdx.x];
-    if (threadIdx.x < kMaxShell) {
-        s.n_insh[threadIdx.x] = 0;
-        s.shell_tsum[threadIdx.x] = 0.0;
-    }
-}
-
-// theta_corr update every itdis steps, src/nonbondene.f90:6630-6645
-__global__ void k_watpol_update(SolventDev p, const DevState* __restrict__ states) {
-    double* wstate = states[blockIdx.y].wstate;
-    int is = threadIdx.x;
-    if (is >= p.nshell) return;
-    double* tc = wstate;
-    double* av = wstate + kMaxShell;
-    double* an = wstate + 2 * kMaxShell;
-    av[is] = av[is] / p.itdis;
-    an[is] = an[is] / p.itdis;
-    tc[is] = tc[is] + av[is] - acos(p.cstb[is]);
-    av[is] = 0.0;
-    an[is] = 0.0;
-}
-
-// energy and gradient, src/nonbondene.f90:6646-6742.  STORED: the vectors and
-// theta of this call's k_watpol_theta are current (md); otherwise they are
-// recomputed from the coordinates, as the reference does in every call.
-template <bool MIX, bool STORED>
-__global__ void k_watpol_force(DevModel m, const DevState* __restrict__ states, SolventDev p) {
-    const DevState& s = states[blockIdx.y];
+    __syncthreads();   // the block's ranks
     Acc<MIX> acc = make_acc<MIX>(s);
     ESum<MIX> ep;
-    const double pi = 3.14159265358979323846;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < m.nwat; w += gridDim.x * blockDim.x) {
-        int sh = s.shell[w];
-        if (sh < 0) continue;
-        int n = s.n_insh[sh];
-        int il = s.rank[w] + 1;
-        if constexpr (MIX) {
-            if (m.sa == 3) {   // FP32 arithmetic (the theta kernel's FP32 vectors when STORED)
-                const float pif = 3.14159265f;
-                float arg = 1.f + (1.f - 2.f * (float)il) / (float)n;
-                float t0 = acosf(arg);
-                t0 = t0 - 3.f * sinf(t0) * p.cstbf[sh] / 2.f;
-                t0 = fminf(fmaxf(t0, 0.f), pif);
-                float th = (float)s.theta[w];
-                float dth = th - t0 + (float)s.wstate[sh];
-                ep.add_alu(0.5f * p.fkwpolf * dth * dth);
-                float dv = p.fkwpolf * dth;
-                float rmx, rmy, rmz, rm, rcx, rcy, rcz, rc;
-                if constexpr (STORED) {
-                    const double* v = s.wvec + 8 * (size_t)w;
-                    rmx = (float)v[0]; rmy = (float)v[1]; rmz = (float)v[2]; rm = (float)v[3];
-                    rcx = (float)v[4]; rcy = (float)v[5]; rcz = (float)v[6]; rc = (float)v[7];
-                } else {
-                    water_vectors_f(m, s.xq, w, rmx, rmy, rmz, rm, rcx, rcy, rcz, rc);
-                }
-                float scp = fminf(1.f, fmaxf(-1.f, rmx * rcx + rmy * rcy + rmz * rcz));
-                float f0 = STORED ? sinf(th) : sinf(acosf(scp));
-                if (fabsf(f0) < 1.0e-10f) f0 = 1.0e-10f;
-                f0 = dv * (-1.f / f0);
-                float f3x = (rcx - rmx * scp) / rm, f3y = (rcy - rmy * scp) / rm, f3z = (rcz - rmz * scp) / rm;
-                float f2x = (rmx - rcx * scp) / rc, f2y = (rmy - rcy * scp) / rc, f2z = (rmz - rcz * scp) / rc;
-                int i = m.nat_solute + 3 * w;
-                acc.grad_alu(i, (-2.f * f3x + f2x) * f0, (-2.f * f3y + f2y) * f0, (-2.f * f3z + f2z) * f0);
-                acc.grad_alu(i + 1, f3x * f0, f3y * f0, f3z * f0);
-                acc.grad_alu(i + 2, f3x * f0, f3y * f0, f3z * f0);
-                continue;
-            }
+    double* sorted = s.theta_sorted + (size_t)sh * m.nwat;
+    for (int t = threadIdx.x;; t += kRankBlock) {   // the block's waters in the order of its warps' rounds
+        const int k = part * nw + t % nw + t / nw * (kRankParts * nw);
+        if (k >= n) {
+            if (part * nw + t / nw * (kRankParts * nw) >= n) break;   // the whole round is past the shell
+            continue;
         }
-        double arg = 1.0 + (1.0 - 2.0 * (double)il) / (double)n;
-        double t0 = acos(arg);
-        t0 = t0 - 3.0 * sin(t0) * p.cstb[sh] / 2.0;
-        if (t0 < 0.0) t0 = 0.0;
-        if (t0 > pi) t0 = pi;
-        double th = s.theta[w];
-        double dth = th - t0 + s.wstate[sh];
-        ep.add(0.5 * p.fkwpol * dth * dth);
-        double dv = p.fkwpol * dth;
-        double rmx, rmy, rmz, rm, rcx, rcy, rcz, rc, f0;
-        if constexpr (STORED) {
-            const double* v = s.wvec + 8 * (size_t)w;
-            rmx = v[0]; rmy = v[1]; rmz = v[2]; rm = v[3];
-            rcx = v[4]; rcy = v[5]; rcz = v[6]; rc = v[7];
-        } else {
-            water_vectors(m, s.x, w, rmx, rmy, rmz, rm, rcx, rcy, rcz, rc);
-        }
-        double scp = rmx * rcx + rmy * rcy + rmz * rcz;
-        scp = fmin(1.0, fmax(-1.0, scp));
-        // theta = acos(scp) of this same scp when STORED
-        f0 = STORED ? sin(th) : sin(acos(scp));
-        if (fabs(f0) < 1.0e-10) f0 = 1.0e-10;
-        f0 = dv * (-1.0 / f0);
-        double f1x = (rcx - rmx * scp) * -2.0 / rm, f1y = (rcy - rmy * scp) * -2.0 / rm,
-               f1z = (rcz - rmz * scp) * -2.0 / rm;
-        double f3x = (rcx - rmx * scp) / rm, f3y = (rcy - rmy * scp) / rm, f3z = (rcz - rmz * scp) / rm;
-        double f2x = (rmx - rcx * scp) / rc, f2y = (rmy - rcy * scp) / rc, f2z = (rmz - rcz * scp) / rc;
-        int i = m.nat_solute + m.sa * w;
-        if constexpr (!MIX) acc.grad(i, (f1x + f2x) * f0, (f1y + f2y) * f0, (f1z + f2z) * f0);
-        else acc.gradd(i, (f1x + f2x) * f0, (f1y + f2y) * f0, (f1z + f2z) * f0);
-        for (int k = 1; k < m.sa; ++k) {
-            if constexpr (!MIX) acc.grad(i + k, f3x * f0, f3y * f0, f3z * f0);
-            else acc.gradd(i + k, f3x * f0, f3y * f0, f3z * f0);
-        }
+        const int w = L[k], r = s.rank[w];
+        sorted[r] = s.theta[w];
+        watpol_force<MIX, true>(m, s, p, w, sh, n, r + 1, acc, ep);
     }
+    __syncwarp();
     ep.flush(acc, E_RST_POL);
-}
-
-// running averages (md only), src/nonbondene.f90:6738-6741
-// running averages (md only), src/nonbondene.f90:6738-6741.  The shell's
-// theta sum (6652-6666) is taken over the thetas placed at their ranks, by one
-// warp per shell in a fixed order: deterministic whatever order the shell
-// list was filled in.
-__global__ void __launch_bounds__(512) k_watpol_average(DevModel m, SolventDev p, const DevState* __restrict__ states) {
-    const DevState& s = states[blockIdx.y];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int sh = 0; sh < p.nshell; ++sh) {
-        const int n = s.n_insh[sh];
-        const int* L = s.shell_list + (size_t)sh * m.nwat;
-        double* sorted = s.theta_sorted + (size_t)sh * m.nwat;
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            int w = L[k];
-            sorted[s.rank[w]] = s.theta[w];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(s.wp_count + kMaxShell, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int q = warp; q < p.nshell; q += nw) {
+        const int nq = s.wp_count[q];
+        const double* sq = s.theta_sorted + (size_t)q * m.nwat;
+        double t = 0.0;
+        for (int k = lane; k < nq; k += kWarp) t += __ldcg(sq + k);
+        t = warp_sum(t);
+        if (lane == 0 && nq > 0) {
+            s.wstate[kMaxShell + q] += t / (double)nq;
+            s.wstate[2 * kMaxShell + q] += (double)nq;
         }
     }
     __syncthreads();
-    for (int sh = warp; sh < p.nshell; sh += nw) {
-        const int n = s.n_insh[sh];
-        const double* sorted = s.theta_sorted + (size_t)sh * m.nwat;
-        double t = 0.0;
-        for (int k = lane; k < n; k += kWarp) t += sorted[k];
-        t = warp_sum(t);
-        if (lane == 0 && n > 0) {
-            s.wstate[kMaxShell + sh] += t / (double)n;
-            s.wstate[2 * kMaxShell + sh] += (double)n;
-        }
+    // the shells' counts for calls without md; the working counts and the
+    // block count start the next call at zero
+    if (threadIdx.x <= kMaxShell) {
+        if (threadIdx.x < kMaxShell) s.n_insh[threadIdx.x] = s.wp_count[threadIdx.x];
+        s.wp_count[threadIdx.x] = 0;
     }
 }
 
@@ -5323,44 +5360,57 @@ void launch_restraints(const Launch& L, const RestrDev& r, int mixed) {
     if (mixed) k_restraints<true><<<g, kRestrBlock, 0, L.st>>>(L.m, L.ds, r);
     else k_restraints<false><<<g, kRestrBlock, 0, L.st>>>(L.m, L.ds, r);
 }
+static double host_shift(const SolventDev& p, double Tfree) {
+    return Tfree >= 0.0 && p.fk_wsphere != 0.0 ? sqrt(p.boltz * Tfree / p.fk_wsphere) : 0.0;
+}
 void launch_restrain_solvent(const Launch& L, const SolventDev& p, double Tfree, int mixed, const int* wsw,
                              const uint8_t* heavy_solv) {
     if (L.m.nwat == 0) return;
     const int tdev = Tfree < 0.0;
-    double shift = (!tdev && p.fk_wsphere != 0.0) ? sqrt(p.boltz * Tfree / p.fk_wsphere) : 0.0;
     dim3 g = grid_for(L.m.nwat, 32, 16, L.nwin);
-    if (mixed) k_restrain_solvent<true><<<g, 32, 0, L.st>>>(L.m, L.ds, p, shift, wsw, heavy_solv, tdev);
-    else k_restrain_solvent<false><<<g, 32, 0, L.st>>>(L.m, L.ds, p, shift, wsw, heavy_solv, tdev);
+    if (mixed) k_restrain_solvent<true><<<g, 32, 0, L.st>>>(L.m, L.ds, p, host_shift(p, Tfree), wsw, heavy_solv, tdev);
+    else k_restrain_solvent<false><<<g, 32, 0, L.st>>>(L.m, L.ds, p, host_shift(p, Tfree), wsw, heavy_solv, tdev);
 }
-// returns the number of launches
+static bool watpol_on(const Launch& L, const SolventDev& p) { return L.m.nwat > 0 && p.wpol && p.nshell > 0; }
+static int launch_watpol_rest(const Launch& L, const SolventDev& p, int mixed) {
+    dim3 g(p.nshell * kRankParts, L.nwin);
+    if (mixed) k_watpol_rank_force<true><<<g, kRankBlock, 0, L.st>>>(L.m, L.ds, p);
+    else k_watpol_rank_force<false><<<g, kRankBlock, 0, L.st>>>(L.m, L.ds, p);
+    return 1;
+}
+static int launch_watpol_update(const Launch& L, const SolventDev& p, int istep) {
+    if (istep <= 0 || istep % (int)llround(p.itdis) != 0) return 0;
+    k_watpol_update<<<dim3(1, L.nwin), kMaxShell, 0, L.st>>>(p, L.ds);   // of the averages up to the last call
+    return 1;
+}
 int launch_watpol(const Launch& L, const SolventDev& p, int istep, int md, int mixed) {
-    if (L.m.nwat == 0 || !p.wpol || p.nshell <= 0) return 0;
-    int nl = 0;
+    if (!watpol_on(L, p)) return 0;
     dim3 gw((L.m.nwat + 31) / 32, L.nwin);   // FP64 math per water: 32-thread blocks
-    if (md) {
-        k_watpol_reset<<<L.nwin, kMaxShell, 0, L.st>>>(L.ds);
-        if (mixed) k_watpol_theta<true><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
-        else k_watpol_theta<false><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
-        k_watpol_rank<<<dim3(p.nshell * kRankParts, L.nwin), kRankBlock, 0, L.st>>>(L.m, L.ds);
-        nl += 3;
+    if (!md) {
+        if (mixed) k_watpol_force<true><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
+        else k_watpol_force<false><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
+        return 1;
     }
-    if (istep > 0 && md && (istep % (int)llround(p.itdis)) == 0) {
-        k_watpol_update<<<dim3(1, L.nwin), kMaxShell, 0, L.st>>>(p, L.ds);
-        ++nl;
+    int nl = launch_watpol_update(L, p, istep);
+    if (mixed) k_watpol_theta<true, false><<<gw, 32, 0, L.st>>>(L.m, L.ds, p, 0.0, nullptr, nullptr, 0);
+    else k_watpol_theta<false, false><<<gw, 32, 0, L.st>>>(L.m, L.ds, p, 0.0, nullptr, nullptr, 0);
+    return nl + 1 + launch_watpol_rest(L, p, mixed);
+}
+int launch_boundary_theta(const Launch& L, const SolventDev& p, double Tfree, int istep, int mixed, const int* wsw,
+                          const uint8_t* heavy_solv) {
+    if (!watpol_on(L, p)) {
+        launch_restrain_solvent(L, p, Tfree, mixed, wsw, heavy_solv);
+        return 1;
     }
-    if (md) {
-        if (mixed) k_watpol_force<true, true><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
-        else k_watpol_force<false, true><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
-    } else {
-        if (mixed) k_watpol_force<true, false><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
-        else k_watpol_force<false, false><<<gw, 32, 0, L.st>>>(L.m, L.ds, p);
-    }
-    ++nl;
-    if (md) {
-        k_watpol_average<<<dim3(1, L.nwin), 512, 0, L.st>>>(L.m, p, L.ds);
-        ++nl;
-    }
-    return nl;
+    dim3 gw((L.m.nwat + 31) / 32, L.nwin);
+    const int nl = launch_watpol_update(L, p, istep), tdev = Tfree < 0.0;
+    const double sh = host_shift(p, Tfree);
+    if (mixed) k_watpol_theta<true, true><<<gw, 32, 0, L.st>>>(L.m, L.ds, p, sh, wsw, heavy_solv, tdev);
+    else k_watpol_theta<false, true><<<gw, 32, 0, L.st>>>(L.m, L.ds, p, sh, wsw, heavy_solv, tdev);
+    return nl + 1;
+}
+int launch_boundary_watpol(const Launch& L, const SolventDev& p, int mixed) {
+    return watpol_on(L, p) ? launch_watpol_rest(L, p, mixed) : 0;
 }
 
 void launch_q_adjoint(const Launch& L) {

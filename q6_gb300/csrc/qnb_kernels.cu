@@ -1812,12 +1812,26 @@ constexpr int kQRed = 5;   // Q atoms per transposed reduction (15 of its 16 val
 // water's first atom (qw) or against the first atom of the solute atom's
 // group within Rcq of qswitch (qp, nbqp_cgp; iwhich, rq2); the pair vector
 // is shift - (x_q - x_j).
+//
+// Latency bounds it: a warp meets its Q atoms one after the other.  The blocks
+// are small, so that one window's few warps spread over the SMs (256-thread
+// blocks put the 32 warps of 1,020 waters on four); the water parameters are
+// staged in shared memory, and a solute atom's are loaded a Q atom ahead.
+// With both, 51 windows of 446 waters and 6 Q atoms take 12 us for the waters
+// and 10 us for the solute (22 and 16 in 256-thread blocks that read the
+// parameters from global memory), event overhead of about 5 us included.
+constexpr int kQLaneBlock = 64;
 template <bool SPC, bool WATER, int SMAX, bool BOX = false>
-__global__ void __launch_bounds__(kQBlock) k_qenv_lanes(DevModel m, const DevState* __restrict__ states,
-                                                        const int* __restrict__ iwhich = nullptr, float rq2 = 0.f) {
+__global__ void __launch_bounds__(kQLaneBlock) k_qenv_lanes(DevModel m, const DevState* __restrict__ states,
+                                                            const int* __restrict__ iwhich = nullptr, float rq2 = 0.f) {
+    extern __shared__ float4 sh_par[];   // WATER: m.qw_tabf
     const DevState& s = states[blockIdx.y];
     __shared__ unsigned long long red[3 * kMaxQ];
     __shared__ float4 sq[kMaxQ];
+    if (WATER) {
+        const float4* t = reinterpret_cast<const float4*>(m.qw_tabf);
+        for (int k = threadIdx.x; k < m.nqat * m.sa * m.S; k += blockDim.x) sh_par[k] = t[k];
+    }
     for (int k = threadIdx.x; k < 3 * m.nqat; k += blockDim.x) red[k] = 0ull;
     for (int k = threadIdx.x; k < m.nqat; k += blockDim.x) sq[k] = s.xq[m.iqseq[k]];
     __syncthreads();
@@ -1864,6 +1878,14 @@ __global__ void __launch_bounds__(kQBlock) k_qenv_lanes(DevModel m, const DevSta
         float pel[SMAX], pvdw[SMAX];
 #pragma unroll
         for (int st = 0; st < SMAX; ++st) pel[st] = pvdw[st] = 0.f;
+        QParF nxt[SMAX];   // (solute atoms) the next Q atom's parameters
+        auto load_par = [&](int iq) {
+            const QParF* P = m.qp_tabft + ((size_t)iq * m.nat_solute + j0) * S;
+#pragma unroll
+            for (int st = 0; st < SMAX; ++st)
+                if (st < S) nxt[st] = P[st];
+        };
+        if (!WATER) load_par(0);   // (an idle lane's j0 is atom 0)
         // Q atoms in blocks of kQRed: their 3 kQRed gradient components are
         // summed over the warp in one transposed butterfly (reduce_scatter)
         for (int q0 = 0; q0 < nq; q0 += kQRed) {
@@ -1876,6 +1898,12 @@ __global__ void __launch_bounds__(kQBlock) k_qenv_lanes(DevModel m, const DevSta
                 if (iq >= nq) break;   // warp-uniform
                 const float4 xi = sq[iq];
                 float gx = 0.f, gy = 0.f, gz = 0.f;
+                QParF par[SMAX];
+                if (!WATER) {
+#pragma unroll
+                    for (int st = 0; st < SMAX; ++st) par[st] = nxt[st];
+                    if (iq + 1 < nq) load_par(iq + 1);
+                }
                 if (act) {
 #pragma unroll
                     for (int a = 0; a < NA; ++a) {
@@ -1888,8 +1916,7 @@ __global__ void __launch_bounds__(kQBlock) k_qenv_lanes(DevModel m, const DevSta
                             tx = xj[a].x - xi.x, ty = xj[a].y - xi.y, tz = xj[a].z - xi.z;
                         }
                         float r = rsqrtf(tx * tx + ty * ty + tz * tz), r2 = r * r;
-                        const QParF* P = WATER ? m.qw_tabf + (iq * m.sa + a) * S
-                                               : m.qp_tabft + ((size_t)iq * m.nat_solute + j0) * S;
+                        const QParF* P = WATER ? reinterpret_cast<const QParF*>(sh_par) + (iq * m.sa + a) * S : par;
                         float dvs = QPairF<SMAX>::run(P, lam, S, lj, r2, r, pel, pvdw);
                         gx -= tx * dvs; gy -= ty * dvs; gz -= tz * dvs;
                         gj[a][0] += tx * dvs; gj[a][1] += ty * dvs; gj[a][2] += tz * dvs;
@@ -4280,9 +4307,10 @@ void launch_qenv(const Launch& L, int mixed, int per_sm, const int* iwhich, doub
     if (units == 0 || L.m.nqat == 0) return;
     const bool spc = L.m.spc != 0, s4 = L.m.S <= 4, box = iwhich != nullptr;
     if (mixed) {
-        dim3 g = grid_for((int64_t)(WATER ? L.s0.cap_qw : L.s0.cap_qp) * 32, kQBlock, per_sm, L.nwin);
+        dim3 g = grid_for(units, kQLaneBlock, per_sm * (kQBlock / kQLaneBlock), L.nwin);
         const float rq2 = (float)rcq2;
-#define QT(SPC, SM, BX) k_qenv_lanes<SPC, WATER, SM, BX><<<g, kQBlock, 0, L.st>>>(L.m, L.ds, iwhich, rq2)
+        const int sm = WATER ? L.m.nqat * L.m.sa * L.m.S * (int)sizeof(QParF) : 0;   // at most 64 x 4 x 8: 32 KB
+#define QT(SPC, SM, BX) k_qenv_lanes<SPC, WATER, SM, BX><<<g, kQLaneBlock, sm, L.st>>>(L.m, L.ds, iwhich, rq2)
 #define QS(SPC, SM) do { if (box) QT(SPC, SM, true); else QT(SPC, SM, false); } while (0)
         if (spc) { if (s4) QS(true, 4); else QS(true, kMaxStates); }
         else { if (s4) QS(false, 4); else QS(false, kMaxStates); }

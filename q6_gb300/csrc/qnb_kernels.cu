@@ -1043,11 +1043,12 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
 // cycles, so the pipe's 38 operations per term bound the kernel.
 //
 // The block's kLrfWarps warps hold the same 64 targets (lane: targets l and
-// l + 32) and each sums a range of its own of the source groups (the eligible
-// atoms of each charge group, in group order: lrf_gmeta / lrf_goff /
-// lrf_gatom); the cluster's blocks split the source groups further, so a
-// single window of 1,713 groups has 864 warps.  A warp stages kLrfTile source
-// groups at a time by asynchronous copies while it evaluates the tile before;
+// l + 32) and the cluster's warps take the tiles of kLrfTile source groups in
+// turn (the eligible atoms of each charge group, in group order: lrf_gmeta /
+// lrf_goff / lrf_gatom), so a single window of 1,713 groups has 864 warps.  In
+// turn, not a range for each: a range of neighbouring groups is near some of
+// the targets, and its warp was done long before the others.  A warp stages
+// its next tile by asynchronous copies while it evaluates the tile before;
 // its lanes read the atoms as broadcasts.  Per (target pair, source group)
 // the group-pair classification runs once; a target whose pair is not far
 // gets r^2 = infinity, so its terms are exact zeros at no cost.
@@ -1055,15 +1056,17 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
 // A tile's sums run in FP32 and are then folded into a double-float
 // accumulator (Knuth's TwoSum: s = a + b, bb = s - a,
 // e = (a - (s - bb)) + (b - bb)) kept in shared memory, so the FP32 rounding
-// is kept to short runs.  At the end the cluster's ranges are added in
-// double-float in range order through distributed shared memory, and each
+// is kept to short runs.  At the end the warps' sums are added in
+// double-float in warp order through distributed shared memory, and each
 // block expands its share of the targets: no partial sums in global memory,
-// no second kernel.  Ranges and tiles are fixed by the topology alone, so a
+// no second kernel.  The tiles are fixed by the topology alone, so a
 // window's coefficients do not depend on the launch or the number of windows.
-// Alone: 51 windows of the 25 A sphere 1.30 -> 1.06 ms, 8 of a 34 A sphere
-// 1.85 -> 1.28 ms, one of 25 A 140 -> 70 us; the FMA pipe's operations alone
-// would take half of that, the rest is their latency at four warps per
-// scheduler.  Records as far from FP64 as before (2e-6 of their scale).
+// Alone: 51 windows of the 25 A sphere 1.30 -> 0.95 ms, 8 of a 34 A sphere
+// 1.85 -> 1.18 ms, one of 25 A 140 -> 62 us (with a range of neighbouring
+// groups per warp: 1.06 and 1.28 ms, 70 us; tiles in turn, their indices read
+// only when they are staged: 0.97, 1.20, 64).  The FMA pipe is busy 54 % of
+// the time, the rest is latency at four warps per scheduler.  Records as far
+// from FP64 as before (2e-6 of their scale).
 constexpr int kLrfWarps = 4;
 constexpr int kLrfTgt = 64;    // targets per cluster
 constexpr int kLrfTile = kLrfTileGroups;   // source groups per staged tile and FP32 partial sum
@@ -1101,9 +1104,7 @@ __device__ __forceinline__ double lrf_coef(const double* n, int c) {
     if (b == d) v -= U[a];
     return v;
 }
-#ifndef QNB_LRF_U
-#define QNB_LRF_U 3
-#endif
+constexpr int kLrfAtoms = 3;   // source atoms evaluated together
 // the FP64 decision of a target and source group whose FP32 distance is
 // inside a decision band (or, in a box, whose lattice index is near a half)
 template <bool BOX>
@@ -1159,27 +1160,37 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
     for (int k = 0; k < kLrfMom20; ++k) S.hi[k][lane] = S.lo[k][lane] = f2(0.f);
     const float2 nx = make_float2(-cc[0][0], -cc[1][0]), ny = make_float2(-cc[0][1], -cc[1][1]),
                  nz = make_float2(-cc[0][2], -cc[1][2]);
-    // this warp's range of source groups
-    const int z = blockIdx.z * kLrfWarps + warp, nz_all = gridDim.z * kLrfWarps;
-    const int gbeg = (int)((int64_t)m.nlrf_groups * z / nz_all), gend = (int)((int64_t)m.nlrf_groups * (z + 1) / nz_all);
-    // stages tile t0's atoms, switch atoms and group ends into buffer b
-    auto stage = [&](int t0, int b) {
+    // this warp's tiles of source groups: one of every step / kLrfTile
+    const int gbeg = (blockIdx.z * kLrfWarps + warp) * kLrfTile, step = gridDim.z * kLrfWarps * kLrfTile;
+    const int gend = m.nlrf_groups;
+    // a tile's group offsets and switch atoms (lanes), read a tile before its
+    // atoms are staged
+    int off = 0, meta = 0;
+    auto look = [&](int t0) {
         const int ng = min(kLrfTile, gend - t0);
-        const int off = m.lrf_goff[t0 + min(lane, ng)], base = __shfl_sync(kFull, off, 0);
+        if (ng <= 0) return;
+        off = m.lrf_goff[t0 + min(lane, ng)];
+        if (lane < ng) meta = m.lrf_gmeta[t0 + lane];
+    };
+    // stages that tile's atoms, switch atoms and group ends into buffer b
+    auto stage = [&](int t0, int b) {
+        const int ng = min(kLrfTile, gend - t0), base = __shfl_sync(kFull, off, 0);
         const int na = __shfl_sync(kFull, off, ng) - base;   // <= tile_atoms
         const int end = __shfl_down_sync(kFull, off, 1) - base;
         if (lane < ng) {
-            const int meta = m.lrf_gmeta[t0 + lane];
             cp_async16(&S.xs[b][lane], xq + (meta & 0x3fffffff));
             S.end[b][lane] = end | (meta & (1 << 30));
         }
         for (int u = lane; u < na; u += kWarp) cp_async16(s_xi + b * tile_atoms + u, xq + m.lrf_gatom[base + u]);
     };
+    look(gbeg);
     if (gbeg < gend) stage(gbeg, 0);
+    look(gbeg + step);
     cp_async_commit();
     int b = 0;
-    for (int t0 = gbeg; t0 < gend; t0 += kLrfTile, b ^= 1) {   // warp-uniform
-        if (t0 + kLrfTile < gend) stage(t0 + kLrfTile, b ^ 1);
+    for (int t0 = gbeg; t0 < gend; t0 += step, b ^= 1) {   // warp-uniform
+        if (t0 + step < gend) stage(t0 + step, b ^ 1);
+        look(t0 + 2 * step);
         cp_async_commit();
         cp_async_wait<1>();
         __syncwarp();
@@ -1264,9 +1275,9 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
             // three atoms at a time (a water, most of a solute group): their
             // dependent chains overlap
             int k = k0;
-            for (; k + QNB_LRF_U <= k1; k += QNB_LRF_U) {
+            for (; k + kLrfAtoms <= k1; k += kLrfAtoms) {
 #pragma unroll
-                for (int u = 0; u < QNB_LRF_U; ++u) term(xi[k + u]);
+                for (int u = 0; u < kLrfAtoms; ++u) term(xi[k + u]);
             }
             for (; k < k1; ++k) term(xi[k]);
         }

@@ -503,13 +503,18 @@ int build_model(qnb_context* c, const qnb_topology* t) {
     }
     TRY(c->upload((uint8_t**)&m.gallq, gallq));
     std::vector<int> gnq_off{0}, gnq_atom;
+    std::vector<int2> gnq_rec;
     for (int g = 0; g < t->ncgp_solute; ++g) {
         for (int a = gslot[g]; a < gslot[g + 1]; ++a)
-            if (iqatom[gatom[a]] < 0) gnq_atom.push_back(gatom[a]);
+            if (iqatom[gatom[a]] < 0) {
+                gnq_atom.push_back(gatom[a]);
+                gnq_rec.push_back(make_int2(gatom[a], (iac[gatom[a]] & 0xffff) | (a - gslot[g]) << 16));
+            }
         gnq_off.push_back((int)gnq_atom.size());
     }
     TRY(c->upload((int**)&m.gnq_off, gnq_off));
     TRY(c->upload((int**)&m.gnq_atom, gnq_atom));
+    TRY(c->upload((int2**)&m.gnq_rec, gnq_rec));
     // must agree with k_rows_solute's template choice (MAXG <= 8)
     m.type_in_entry = (c->maxg <= 8 && t->natyps <= 0xffff) ? 1 : 0;
     struct SG {

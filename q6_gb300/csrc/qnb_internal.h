@@ -135,6 +135,7 @@ struct DevModel {
     const ulonglong2* gtmask;           // [ncgp_solute] types 0-63 (x) and 64-127 (y)
     const int* gnq_off;                 // [ncgp_solute+1] non-Q atoms of each solute group
     const int* gnq_atom;
+    const int2* gnq_rec;                // the same: atom, its type (16 bits) and its place in the group << 16
     const uint8_t* gallq;               // [ncgp_solute] 1: every atom of the group is a Q atom (no pair row)
     const float2* ljf1;                 // [natom]
     // LRF sources grouped by charge group (mixed form's accumulation):

@@ -2961,9 +2961,8 @@ __device__ __forceinline__ bool within_box(const DevModel& m, float4 pa, float4 
 // partner atom j needs the general pair path against some row atom (its LJ
 // code with a row atom's type is not 1); the row mask covers 128 types, and
 // with more every partner takes the general path
-__device__ __forceinline__ bool type_special(const DevModel& m, ulonglong2 tmask, int j) {
+__device__ __forceinline__ bool type_special(const DevModel& m, ulonglong2 tmask, int t) {
     if (m.natyps > 128) return true;
-    const int t = m.iac[j];
     return t < 64 ? ((tmask.x >> t) & 1ull) : ((tmask.y >> (t - 64)) & 1ull);
 }
 
@@ -3169,15 +3168,28 @@ __device__ __forceinline__ int run_item(const Runs& R, int t) {
 // tests); otherwise every group and water is a candidate (any-atom tests).
 // The inside tests are the same in both: the FP32 distance of the packed
 // positions, the FP64 distance within the decision band.
+//
+// A solute row's candidates are tested 32 at a time and the selected groups
+// (a quarter of the stencil's) gathered in shared memory; their atoms are
+// classified and written when 32 are together, so that the loops over a
+// group's atoms run with every lane.  Latency bounds the kernel, so the atoms'
+// types come with their numbers in one record and eight blocks share an SM
+// (64 registers).  The whole row build, binning and centres included: 51
+// windows of the 25 A sphere 563 -> 321 us (338 at seven blocks), 8 of a 34 A
+// sphere 258 -> 216 us, one of 25 A 128 -> 77 us, against each lane looping
+// over its candidate's atoms.
+constexpr int kRowWarps = 4;
 template <bool CELLS, bool BOX>
-__global__ void k_build_rows(DevModel m, const DevState* __restrict__ states, Cut c) {
+__global__ void __launch_bounds__(kRowWarps * kWarp, 8) k_build_rows(DevModel m, const DevState* __restrict__ states, Cut c) {
     constexpr int NSEG = CELLS && BOX ? 2 : 1;   // a periodic stencil's wrapped x-runs come second
     const Band bpp = band(c.rcpp2, c.fpp), bpw = band(c.rcpw2, c.fpw), bww = band(c.rcww2, c.fww);
+    __shared__ int sh_in[kRowWarps][2 * kWarp];   // a warp's selected groups not written yet
     const DevState& s = states[blockIdx.y];
     const double* __restrict__ x = s.x;
     const float4* __restrict__ xq = s.xq;
     int nrows = m.ncgp_solute + m.nwat;
     int lane = threadIdx.x & 31;
+    int* in = sh_in[threadIdx.x / kWarp];
     CellGrid G;
     if (CELLS) G = *s.grid;
     for (int r = warp_id_global(); r < nrows; r += warps_total()) {
@@ -3196,6 +3208,66 @@ __global__ void k_build_rows(DevModel m, const DevState* __restrict__ states, Cu
                 // a row with more than 32 falls back to the binary search)
                 const int sl0 = m.sgl_off[g], nsl = m.sgl_off[g + 1] - sl0;
                 const int2 my_sg = lane < nsl ? m.sgl_ent[sl0 + lane] : make_int2(-1, -1);
+                // writes the entries of the first n (<= 32) selected groups, one
+                // group per lane
+                auto write = [&](int n) {
+                    int g2 = -1, q0 = 0, n2 = 0, ns = 0, sgi = -1;
+                    unsigned special = 0;   // of the group's atoms outside the Q region
+                    if (lane < n) {
+                        g2 = in[lane];
+                        q0 = m.gnq_off[g2];
+                        n2 = m.gnq_off[g2 + 1] - q0;
+                    }
+                    if (nsl <= kWarp) {
+                        for (int c = 0; c < nsl; ++c) {   // warp-uniform
+                            const int eg = __shfl_sync(kFull, my_sg.x, c), es = __shfl_sync(kFull, my_sg.y, c);
+                            if (eg == g2) sgi = es;
+                        }
+                    } else if (lane < n) {
+                        sgi = sg_find(m, g <= g2 ? (long long)g * m.ncgp_solute + g2 : (long long)g2 * m.ncgp_solute + g);
+                    }
+                    // the general path: the group itself, group pairs with
+                    // excluded / 1-4 atom pairs, and partner types with LJ
+                    // code 2 against a row atom; plain code-1 partners otherwise
+                    if (g2 == g || sgi >= 0) {
+                        special = (1u << n2) - 1u;
+                    } else {
+                        for (int b = 0; b < n2; ++b)
+                            if (type_special(m, tmask, m.gnq_rec[q0 + b].y & 0xffff)) special |= 1u << b;
+                    }
+                    ns = __popc(special);
+                    const int nf = n2 - ns;
+                    // row-local offsets of both lists: one inclusive warp scan of the
+                    // packed counts (at most 15 * 32 per warp)
+                    int incl = ns | (nf << 16);
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        int v = __shfl_up_sync(kFull, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    const int total = __shfl_sync(kFull, incl, 31);
+                    int ps = npp + (incl & 0xffff) - ns, pf = npf + (incl >> 16) - nf;
+                    const unsigned flags = (g < g2 ? 1u : 0u) | (g == g2 ? 2u : 0u);
+                    for (int k = 0; k < n2; ++k) {
+                        const int2 rec = m.gnq_rec[q0 + k];
+                        const int j = rec.x, b = rec.y >> 16;   // atom, its place in the group
+                        if (!((special >> k) & 1u)) {
+                            if (pf < s.cap_gf) rf[pf] = j;
+                            ++pf;
+                            continue;
+                        }
+                        // 2-bit kind per row atom against partner atom b (the
+                        // host's table of the group pair; none: every kind 0)
+                        unsigned mask = g == g2 ? 1u << (2 * b) : 0u;   // the atom itself
+                        if (sgi >= 0) mask = m.sgm[m.sgm_off[sgi] + (g <= g2 ? b : n1 + b)];
+                        if (m.type_in_entry) mask |= (unsigned)(rec.y & 0xffff) << 16;
+                        if (ps < s.cap_gp) rp[ps] = make_uint2((unsigned)j | (flags << 28), mask);
+                        ++ps;
+                    }
+                    npp += total & 0xffff;
+                    npf += total >> 16;
+                };
+                int nin = 0;
                 for (int seg = 0; seg < NSEG; ++seg) {
                 if (CELLS) R = stencil_runs<BOX>(s.cend_s, G, cs, seg);
                 const int ncand = CELLS ? R.total : m.ncgp_solute;
@@ -3203,7 +3275,7 @@ __global__ void k_build_rows(DevModel m, const DevState* __restrict__ states, Cu
                     const int t = j0 + lane;
                     const int bi = CELLS ? run_item(R, t) : 0;
                     bool ok = false;
-                    int g2 = -1, b0 = 0, n2 = 0, ns = 0, nf = 0, sgi = -1;
+                    int g2 = t;
                     if (t < ncand) {
                         if (CELLS) {
                             float4 it = s.bin_s[bi];
@@ -3211,73 +3283,25 @@ __global__ void k_build_rows(DevModel m, const DevState* __restrict__ states, Cu
                             ok = g2 == g || (BOX ? within_box(m, xs, it, bpp, x, is, m.gsw[g2])
                                                  : within(r2_f(xs, it), bpp, x, is, m.gsw[g2]));
                         } else if (BOX) {
-                            g2 = t;
                             ok = g2 == g || within_box(m, xs, xq[m.gsw[g2]], bpp, x, is, m.gsw[g2]);
                         } else {
-                            g2 = t;
                             if (!m.excl[m.gsw[g2]]) ok = g2 == g || gg_inside(m, x, xq, g, g2, bpp);
                         }
                     }
-                    if (nsl <= kWarp) {
-                        for (int c = 0; c < nsl; ++c) {   // warp-uniform
-                            const int eg = __shfl_sync(kFull, my_sg.x, c), es = __shfl_sync(kFull, my_sg.y, c);
-                            if (eg == g2) sgi = es;
-                        }
+                    nin = row_append(in, 2 * kWarp, nin, ok, g2);
+                    __syncwarp();
+                    if (nin >= kWarp) {   // warp-uniform
+                        write(kWarp);
+                        nin -= kWarp;
+                        const int rest = in[kWarp + lane];
+                        __syncwarp();
+                        in[lane] = rest;
+                        __syncwarp();
                     }
-                    if (t < ncand) {
-                        if (ok) {
-                            b0 = m.gslot[g2];
-                            n2 = m.gslot[g2 + 1] - b0;
-                            if (nsl > kWarp)
-                                sgi = sg_find(m, g <= g2 ? (long long)g * m.ncgp_solute + g2
-                                                         : (long long)g2 * m.ncgp_solute + g);
-                            // the general path: the group itself, group pairs with
-                            // excluded / 1-4 atom pairs, and partner types with LJ
-                            // code 2 against a row atom; plain code-1 partners otherwise
-                            const bool all_special = g2 == g || sgi >= 0;
-                            for (int b = 0; b < n2; ++b) {
-                                int j = m.gatom[b0 + b];
-                                if (m.iqatom[j] >= 0) continue;
-                                if (all_special || type_special(m, tmask, j)) ++ns;
-                                else ++nf;
-                            }
-                        }
-                    }
-                    // row-local offsets of both lists: one inclusive warp scan of the
-                    // packed counts (each below 2^15 per lane, at most 15 * 32 per warp)
-                    int incl = ns | (nf << 16);
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        int v = __shfl_up_sync(kFull, incl, o);
-                        if (lane >= o) incl += v;
-                    }
-                    int total = __shfl_sync(kFull, incl, 31);
-                    if (ns + nf > 0) {
-                        int ps = npp + (incl & 0xffff) - ns, pf = npf + (incl >> 16) - nf;
-                        const bool lower = g <= g2;
-                        const bool all_special = g2 == g || sgi >= 0;
-                        unsigned flags = (g < g2 ? 1u : 0u) | (g == g2 ? 2u : 0u);
-                        for (int b = 0; b < n2; ++b) {
-                            int j = m.gatom[b0 + b];
-                            if (m.iqatom[j] >= 0) continue;
-                            if (!all_special && !type_special(m, tmask, j)) {
-                                if (pf < s.cap_gf) rf[pf] = j;
-                                ++pf;
-                                continue;
-                            }
-                            // 2-bit kind per row atom against partner atom b (the
-                            // host's table of the group pair; none: every kind 0)
-                            unsigned mask = g == g2 ? 1u << (2 * b) : 0u;   // the atom itself
-                            if (sgi >= 0) mask = m.sgm[m.sgm_off[sgi] + (lower ? b : n1 + b)];
-                            if (m.type_in_entry) mask |= (unsigned)m.iac[j] << 16;
-                            if (ps < s.cap_gp) rp[ps] = make_uint2((unsigned)j | (flags << 28), mask);
-                            ++ps;
-                        }
-                    }
-                    npp += total & 0xffff;
-                    npf += total >> 16;
                 }
                 }
+                write(nin);
+                __syncwarp();
                 int* rw = s.row_gw + (size_t)g * s.cap_gw;
                 for (int seg = 0; seg < NSEG; ++seg) {
                 if (CELLS) R = stencil_runs<BOX>(s.cend_w, G, cs, seg);
@@ -4258,12 +4282,12 @@ int launch_bin_cells(const Launch& L, const Cut& c) {
 int launch_build_rows(const Launch& L, const Cut& c) {
     int nrows = L.m.ncgp_solute + L.m.nwat;
     if (nrows == 0) return 0;
-    dim3 g = grid_for((int64_t)nrows * 32, 128, L.tu.v[T_BUILD], L.nwin);
+    dim3 g = grid_for((int64_t)nrows * 32, kRowWarps * kWarp, L.tu.v[T_BUILD], L.nwin);
     int n[3];
-    if (L.m.box && box_cells(L.m, c, n)) k_build_rows<true, true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
-    else if (L.m.box) k_build_rows<false, true><<<g, 128, 0, L.st>>>(L.m, L.ds, c);   // every unit is a candidate
-    else if (L.m.any_atom) k_build_rows<false, false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
-    else k_build_rows<true, false><<<g, 128, 0, L.st>>>(L.m, L.ds, c);
+    if (L.m.box && box_cells(L.m, c, n)) k_build_rows<true, true><<<g, kRowWarps * kWarp, 0, L.st>>>(L.m, L.ds, c);
+    else if (L.m.box) k_build_rows<false, true><<<g, kRowWarps * kWarp, 0, L.st>>>(L.m, L.ds, c);   // every unit is a candidate
+    else if (L.m.any_atom) k_build_rows<false, false><<<g, kRowWarps * kWarp, 0, L.st>>>(L.m, L.ds, c);
+    else k_build_rows<true, false><<<g, kRowWarps * kWarp, 0, L.st>>>(L.m, L.ds, c);
     return 1;
 }
 int lj_smem(const DevModel& m) {

@@ -1735,7 +1735,7 @@ __device__ __forceinline__ void nbe_qx_f(float r2, float r, float r6_hc, float A
 }
 
 constexpr int kMaxQ = 64;
-constexpr int kQBlock = 256;   // threads per block of the Q kernels
+constexpr int kQBlock = 256;   // threads per block of the adjoint kernel; the Q grids' blocks per SM count this size
 
 // Per-lane Q-atom x environment-atom interaction for all states (soft-core
 // LJ + Coulomb when lj, Coulomb only otherwise): returns the lambda-weighted

@@ -4250,9 +4250,9 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
     if (mixed) {
         // blocks per cluster: ranges of at least one tile per warp, the split
         // set by the topology only, so a window's coefficients are the same in
-        // a batch of any size.  At most 4: 8 sped up a single window (R25: 74
-        // -> 54 us) and slowed 51 windows (1,100 -> 1,240 us), 2 the reverse
-        // (130 and 1,085 us)
+        // a batch of any size.  At most 4: 8 sped up a single window (R25: 63
+        // -> 54 us) and slowed 51 windows (953 -> 1,191 us); 2, measured when
+        // each warp summed one range, the reverse (74 -> 130, 1,100 -> 1,085)
         int nz = 1;
         while (nz < kLrfClusterMax && L.m.nlrf_groups >= 2 * nz * kLrfWarps * kLrfTile) nz *= 2;
         const int tile_atoms = std::max(96 / nz, (L.m.lrf_tile_atoms + 3) & ~3);   // 96 / nz: the totals' space

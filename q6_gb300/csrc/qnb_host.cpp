@@ -1551,6 +1551,7 @@ int qnb_create_batch(const qnb_topology* t, const qnb_options* opt, int32_t nwin
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess)
         rc = fail(QNB_ERR_CUDA, "stream creation failed");
+    if (!rc && (e = kernels_init()) != cudaSuccess) rc = fail(QNB_ERR_CUDA, "kernel attributes: %s", cudaGetErrorString(e));
     if (!rc) rc = build_model(c, t);
     if (!rc) rc = alloc_state(c);
     if (rc) {

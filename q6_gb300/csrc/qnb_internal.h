@@ -276,6 +276,7 @@ struct Launch {
     const Tune& tu;
 };
 
+cudaError_t kernels_init();   // per-device kernel attributes, set when a context is created
 void launch_host_in(const double* h, double* x, int n, cudaStream_t st);
 // d to h, d cleared; e to he
 void launch_host_out(double* d, double* h, int n, const double* e, double* he, int ne, cudaStream_t st);

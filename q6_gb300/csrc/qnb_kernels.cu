@@ -4206,9 +4206,11 @@ void launch_build_qp(const Launch& L, const uint8_t* qnear, double rcq2) {
     k_build_qp<<<dim3(1, L.nwin), 1024, 0, L.st>>>(L.m, L.ds, qnear, rcq2);
 }
 namespace {
-int launch_lrf_pairs(const Launch& L, const Cut& c, int nz, int tile_atoms, size_t smem) {
+size_t lrf_pairs_smem(int tile_atoms) {
+    return kLrfWarps * (sizeof(LrfSmem) + 2 * tile_atoms * sizeof(float4));
+}
+int launch_lrf_pairs(const Launch& L, const Cut& c, int nz, int tile_atoms) {
     auto kern = L.m.box ? k_lrf_pairs<true> : k_lrf_pairs<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = at.val.clusterDim.y = 1;
@@ -4216,7 +4218,7 @@ int launch_lrf_pairs(const Launch& L, const Cut& c, int nz, int tile_atoms, size
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((L.m.ncgp + kLrfTgt - 1) / kLrfTgt, L.nwin, nz);
     cfg.blockDim = dim3(kLrfWarps * kWarp);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = lrf_pairs_smem(tile_atoms);
     cfg.stream = L.st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
@@ -4224,6 +4226,19 @@ int launch_lrf_pairs(const Launch& L, const Cut& c, int nz, int tile_atoms, size
     return 1;
 }
 }  // namespace
+
+// The shared memory that k_lrf_pairs may ask for is a property of the function
+// on a device, common to all contexts and threads: it is set to the largest
+// that any topology needs (a tile of groups of kMaxGroup atoms), always the
+// same value, never to one context's own.
+cudaError_t kernels_init() {
+    constexpr int kTileAtomsMax = kLrfTileGroups * kMaxGroup;
+    static_assert(kMaxGroup >= kMaxSolv && kTileAtomsMax % 4 == 0 && kTileAtomsMax >= 96, "launch_lrf_accumulate's tiles");
+    const int smem = (int)lrf_pairs_smem(kTileAtomsMax);
+    cudaError_t e = cudaFuncSetAttribute(k_lrf_pairs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_lrf_pairs<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e;
+}
 
 int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* lrf_src, int keep_order) {
     if (L.m.any_atom && L.m.box) {
@@ -4256,8 +4271,7 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
         int nz = 1;
         while (nz < kLrfClusterMax && L.m.nlrf_groups >= 2 * nz * kLrfWarps * kLrfTile) nz *= 2;
         const int tile_atoms = std::max(96 / nz, (L.m.lrf_tile_atoms + 3) & ~3);   // 96 / nz: the totals' space
-        const size_t smem = kLrfWarps * (sizeof(LrfSmem) + 2 * tile_atoms * sizeof(float4));
-        return launch_lrf_pairs(L, c, nz, tile_atoms, smem);
+        return launch_lrf_pairs(L, c, nz, tile_atoms);
     }
     dim3 g = grid_for((int64_t)L.m.ncgp * 32, 128, 16, L.nwin);
     if (L.m.box) k_lrf_accumulate64<true><<<g, 128, 0, L.st>>>(L.m, L.ds, c, lrf_src);

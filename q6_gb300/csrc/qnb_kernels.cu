@@ -67,6 +67,17 @@ __device__ __forceinline__ float rsqrt_ftz(float v) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
+// 1/r and 1/r^2 in FP64 from the squared distance.  The square of the
+// reciprocal square root alone has 2.2 times the rounding error of a quotient
+// (0.95 against 0.42 x 2^-53, root mean square); one Newton step (two
+// multiply-adds) brings it to the quotient's.  Outside the normal numbers the
+// step would make a NaN of the square's 0 or infinity; the test is an integer's,
+// off the FP64 pipe.
+__device__ __forceinline__ void inv_dist(double d2, double& r, double& r2) {
+    r = rsqrt(d2);
+    const double h = r * r, h1 = fma(h, fma(-d2, h, 1.0), h);
+    r2 = (unsigned)__double2hiint(d2) - 0x00100000u < 0x7fe00000u ? h1 : h;
+}
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }   // exact product
 
@@ -830,37 +841,44 @@ __device__ __forceinline__ float3 lrf_shift(const DevModel& m, float4 pb, float 
 }
 
 // The 20 moment sums of one source atom at d = (dx, dy, dz) from the target's
-// centre, in the scaled vector e = d / r^2 and w = q / r:
-//   n[0] w   n[1..3] -w e   n[4..9] w e e (xx xy xz yy yz zz)
-//   n[10..19] w e e e (xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz)
-// w e e = q d d / r^5 and w e e e = q d d d / r^7, so S2 = 3 n and S3 = -15 n
-// (lrf_scale20).  The products of one order are the factors of the next, so a
-// term takes 38 operations and a reciprocal square root.
-__device__ __forceinline__ void lrf_terms_e(double dx, double dy, double dz, double q, double* n) {
-    const double ri = rsqrt(dx * dx + dy * dy + dz * dz), ri2 = ri * ri, w = q * ri;
-    const double ex = dx * ri2, ey = dy * ri2, ez = dz * ri2;
-    const double ax = w * ex, ay = w * ey, az = w * ez;
-    const double bxx = ax * ex, byy = ay * ey, bzz = az * ez, bxy = ax * ey;
+// centre, in FP64:
+//   n[0] q/r   n[1..3] -q d/r^3   n[4..9] q d d/r^5 (xx xy xz yy yz zz)
+//   n[10..19] q d d d/r^7 (xxx xxy xxz xyy xyz xzz yyy yyz yzz zzz)
+// so S2 = 3 n and S3 = -15 n (lrf_scale20).  q/r^3 is formed from the
+// reciprocal square root ri and corrected once for ri's own rounding and that
+// of its square (residuals e of 1 - r^2 ri^2), so that it is as near as
+// q/(r^2 sqrt(r^2)) by division: of single terms the coefficients of order 0
+// to 3 are off by 0.60, 0.49, 1.19 and 3.8 x 2^-53 of q/r^(k+1) (root mean
+// square), with divisions by 0.85, 0.49, 1.17 and 4.0, and with the powers of
+// d/r^2 on q ri, ten operations fewer, by 0.60, 0.87, 2.2 and 6.8.
+__device__ __forceinline__ void lrf_terms64(double dx, double dy, double dz, double q, double* n) {
+    const double d2 = dx * dx + dy * dy + dz * dz, ri = rsqrt(d2), h = ri * ri;
+    const double e2 = fma(-d2, h, 1.0), e = fma(-d2, fma(ri, ri, -h), e2);
+    const double w = q * ri, p = w * h, ri2 = fma(h, e2, h);
+    const double f0 = fma(p, fma(0.5, e, e2), p), f1 = f0 * ri2, f2 = f1 * ri2;
+    const double ax = dx * f1, ay = dy * f1, az = dz * f1;
+    const double gx = dx * f2, gy = dy * f2, gz = dz * f2;
+    const double gxx = gx * dx, gyy = gy * dy, gzz = gz * dz, gxy = gx * dy;
     n[0] += w;
-    n[1] -= ax;
-    n[2] -= ay;
-    n[3] -= az;
-    n[4] += bxx;
-    n[5] += bxy;
-    n[6] += ax * ez;
-    n[7] += byy;
-    n[8] += ay * ez;
-    n[9] += bzz;
-    n[10] += bxx * ex;
-    n[11] += bxx * ey;
-    n[12] += bxx * ez;
-    n[13] += byy * ex;
-    n[14] += bxy * ez;
-    n[15] += bzz * ex;
-    n[16] += byy * ey;
-    n[17] += byy * ez;
-    n[18] += bzz * ey;
-    n[19] += bzz * ez;
+    n[1] -= dx * f0;
+    n[2] -= dy * f0;
+    n[3] -= dz * f0;
+    n[4] += ax * dx;
+    n[5] += ax * dy;
+    n[6] += ax * dz;
+    n[7] += ay * dy;
+    n[8] += ay * dz;
+    n[9] += az * dz;
+    n[10] += gxx * dx;
+    n[11] += gxx * dy;
+    n[12] += gxx * dz;
+    n[13] += gyy * dx;
+    n[14] += gxy * dz;
+    n[15] += gzz * dx;
+    n[16] += gyy * dy;
+    n[17] += gyy * dz;
+    n[18] += gzz * dy;
+    n[19] += gzz * dz;
 }
 __device__ __forceinline__ void lrf_scale20(double* n) {
 #pragma unroll
@@ -1048,7 +1066,7 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
 
 // Mixed form: one thread per PAIR of target groups, the two in the halves of
 // packed FP32x2 arithmetic, so every packed instruction advances both targets
-// and no half has to be rearranged (the 38 operations of lrf_terms_e take 44
+// and no half has to be rearranged (the 38 operations of a term take 44
 // issue slots for two targets; one target per thread with its sums paired up
 // took about 45 for one).  A packed instruction holds the FMA pipe for two
 // cycles, so the pipe's 38 operations per term bound the kernel.
@@ -1250,7 +1268,10 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
                 oy = make_float2(-(cc[0][1] + sh[0].y), -(cc[1][1] + sh[1].y));
                 oz = make_float2(-(cc[0][2] + sh[0].z), -(cc[1][2] + sh[1].z));
             }
-            auto term = [&](const float4 a) {   // the terms of lrf_terms_e
+            // The 20 moment sums in the scaled vector e = d / r^2 and w = q / r:
+            // w, w e, w e e and w e e e, the products of one order the factors
+            // of the next (S2 = 3 n and S3 = -15 n, as in lrf_terms64)
+            auto term = [&](const float4 a) {
                 const float2 dx = make_float2(a.x + ox.x, a.x + ox.y), dy = make_float2(a.y + oy.x, a.y + oy.y),
                              dz = make_float2(a.z + oz.x, a.z + oz.y);
                 const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, far2)));
@@ -1396,7 +1417,7 @@ __global__ void __launch_bounds__(128) k_lrf_accumulate64(DevModel m, const DevS
             }
             double dx = x[3 * i] - cx, dy = x[3 * i + 1] - cy, dz = x[3 * i + 2] - cz;
             if constexpr (BOX) dx -= sx, dy -= sy, dz -= sz;
-            lrf_terms_e(dx, dy, dz, m.crg[i], mom);
+            lrf_terms64(dx, dy, dz, m.crg[i], mom);
         }
         __syncwarp();
 #pragma unroll
@@ -1559,7 +1580,7 @@ __global__ void __launch_bounds__(128) k_lrf_accumulate_any_box(DevModel m, cons
 // form's kernels are bound by the FP64 pipe (84 % busy at two lanes per clock
 // and SM), where the reference's division and square root of the quotient
 // were 15 of a pair's 37 operations (16 windows of the 25 A sphere: pp 774 ->
-// 661 us, ww 269 -> 185, pw 212 -> 165).  Both orders are within a few ulp.
+// 661 us, ww 269 -> 185, pw 212 -> 165).  See inv_dist for its rounding.
 struct PairD {
     double tx, ty, tz, dv, vel, vdw;
 };
@@ -1572,7 +1593,8 @@ __device__ __forceinline__ PairD nbe_d(const double (&xi)[3], const double (&xj)
     p.tx = xj[0] - xi[0];
     p.ty = xj[1] - xi[1];
     p.tz = xj[2] - xi[2];
-    const double r = rsqrt(p.tx * p.tx + p.ty * p.ty + p.tz * p.tz), r2 = r * r;
+    double r, r2;
+    inv_dist(p.tx * p.tx + p.ty * p.ty + p.tz * p.tz, r, r2);
     p.vel = el * r;
     if (lj) {
         double r6 = r2 * r2 * r2;
@@ -2049,7 +2071,9 @@ __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __re
                     } else {
                         tx = xj[a][0] - xi[0], ty = xj[a][1] - xi[1], tz = xj[a][2] - xi[2];
                     }
-                    const double d2 = tx * tx + ty * ty + tz * tz, r = rsqrt(d2);
+                    const double d2 = tx * tx + ty * ty + tz * tz;
+                    double r, r2;
+                    inv_dist(d2, r, r2);
                     const QPar* P = WATER ? m.qw_tab + (size_t)(iq * m.sa + a) * S
                                           : m.qp_tab + ((size_t)j0 * nq + iq) * S;
                     double sum = 0.0;   // -dv / r2
@@ -2080,7 +2104,7 @@ __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __re
                             eel[st].add(vel);
                         }
                     }
-                    const double dvs = -(r * r) * sum;
+                    const double dvs = -r2 * sum;
                     gx -= tx * dvs; gy -= ty * dvs; gz -= tz * dvs;
                     gj[a][0] += tx * dvs; gj[a][1] += ty * dvs; gj[a][2] += tz * dvs;
                 }

@@ -1082,13 +1082,13 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
 // the group-pair classification runs once; a target whose pair is not far
 // gets r^2 = infinity, so its terms are exact zeros at no cost.
 //
-// A tile's sums run in FP32 and are then folded into a double-float
-// accumulator (Knuth's TwoSum: s = a + b, bb = s - a,
+// The sums of kLrfFold source groups run in FP32 and are then folded into a
+// double-float accumulator (Knuth's TwoSum: s = a + b, bb = s - a,
 // e = (a - (s - bb)) + (b - bb)) kept in shared memory, so the FP32 rounding
-// is kept to short runs.  At the end the warps' sums are added in
-// double-float in warp order through distributed shared memory, and each
-// block expands its share of the targets: no partial sums in global memory,
-// no second kernel.  The tiles are fixed by the topology alone, so a
+// is kept to short runs.  At the end the warps' sums are added in FP64 in
+// warp order, the blocks' in rank order through distributed shared memory, and
+// each block expands its share of the targets: no partial sums in global
+// memory, no second kernel.  The tiles are fixed by the topology alone, so a
 // window's coefficients do not depend on the launch or the number of windows.
 // Alone: 51 windows of the 25 A sphere 1.30 -> 0.95 ms, 8 of a 34 A sphere
 // 1.85 -> 1.18 ms, one of 25 A 140 -> 62 us (with a range of neighbouring
@@ -1098,21 +1098,19 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
 // from FP64 as before (2e-6 of their scale).
 constexpr int kLrfWarps = 4;
 constexpr int kLrfTgt = 64;    // targets per cluster
-constexpr int kLrfTile = kLrfTileGroups;   // source groups per staged tile and FP32 partial sum
+constexpr int kLrfTile = kLrfTileGroups;   // source groups per staged tile
 
 struct LrfSmem {   // of one warp; the staged atoms follow the blocks' warps
-    float2 hi[kLrfMom20][kWarp], lo[kLrfMom20][kWarp];
+    union {
+        struct {
+            float2 hi[kLrfMom20][kWarp], lo[kLrfMom20][kWarp];
+        };
+        double2 sum[kLrfMom20][kWarp];   // (warp 0's) the block's sums
+    };
     float4 xs[2][kLrfTile];
     int end[2][kLrfTile];   // last atom + 1 of the group in the tile | solute flag << 30
 };
 constexpr int kLrfTot = kLrfMom20 + 4;   // totals of a target: the 20 moments, F0, U(3)
-// (hi, lo) += (p, pl) in double-float
-__device__ __forceinline__ void df_add(float& hi, float& lo, float p, float pl) {
-    const float sum = __fadd_rn(hi, p), bb = __fsub_rn(sum, hi);
-    const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(sum, bb)), __fsub_rn(p, bb));
-    hi = sum;
-    lo = __fadd_rn(lo, __fadd_rn(pl, e));
-}
 // coefficient c (0..39) of the record from a target's totals: phi0, phi1(a),
 // phi2(a, b) = S2(ab) - delta_ab F0, phi3(a, b, c) = S3(abc) - delta_ab U(c) -
 // delta_ac U(b) - delta_bc U(a)
@@ -1228,7 +1226,18 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
         float2 n[kLrfMom20];
 #pragma unroll
         for (int k = 0; k < kLrfMom20; ++k) n[k] = f2(0.f);
+        auto fold = [&]() {   // TwoSum into the accumulators; n starts again
+#pragma unroll
+            for (int k = 0; k < kLrfMom20; ++k) {
+                const float2 hi = S.hi[k][lane], sum = __fadd2_rn(hi, n[k]), bb = fsub2(sum, hi);
+                const float2 e = __fadd2_rn(fsub2(hi, fsub2(sum, bb)), fsub2(n[k], bb));
+                S.hi[k][lane] = sum;
+                S.lo[k][lane] = __fadd2_rn(S.lo[k][lane], e);
+                n[k] = f2(0.f);
+            }
+        };
         for (int gi = 0, k1 = 0; gi < ng; ++gi) {
+            if (gi && gi % kLrfFold == 0) fold();   // warp-uniform
             const int k0 = k1, e = S.end[b][gi];
             const float4 xs = S.xs[b][gi];
             const bool ss = (e >> 30) != 0;   // solute source
@@ -1313,29 +1322,29 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
             }
             for (; k < k1; ++k) term(xi[k]);
         }
-#pragma unroll
-        for (int k = 0; k < kLrfMom20; ++k) {   // TwoSum fold
-            const float2 hi = S.hi[k][lane], sum = __fadd2_rn(hi, n[k]), bb = fsub2(sum, hi);
-            const float2 e = __fadd2_rn(fsub2(hi, fsub2(sum, bb)), fsub2(n[k], bb));
-            S.hi[k][lane] = sum;
-            S.lo[k][lane] = __fadd2_rn(S.lo[k][lane], e);
-        }
+        fold();
         __syncwarp();   // buffer b is refilled in the next iteration
     }
     cp_async_wait<0>();
-    // the block's warps in order, into warp 0's accumulators
+    // the block's warps in order, in FP64, in place of warp 0's accumulators
     __syncthreads();
-    for (int v = threadIdx.x; v < kLrfMom20 * kWarp; v += blockDim.x) {
-        float2 h = (&sm[0].hi[0][0])[v], l = (&sm[0].lo[0][0])[v];
+    constexpr int kSums = kLrfMom20 / kLrfWarps;   // per thread
+    static_assert(kLrfMom20 % kLrfWarps == 0, "");
+    double2 sum[kSums];
 #pragma unroll
-        for (int w = 1; w < kLrfWarps; ++w) {
-            const float2 h2 = (&sm[w].hi[0][0])[v], l2 = (&sm[w].lo[0][0])[v];
-            df_add(h.x, l.x, h2.x, l2.x);
-            df_add(h.y, l.y, h2.y, l2.y);
+    for (int u = 0; u < kSums; ++u) {
+        const int v = u * kLrfWarps * kWarp + threadIdx.x;
+        sum[u] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int w = 0; w < kLrfWarps; ++w) {
+            const float2 h = (&sm[w].hi[0][0])[v], l = (&sm[w].lo[0][0])[v];
+            sum[u].x += (double)h.x + (double)l.x;
+            sum[u].y += (double)h.y + (double)l.y;
         }
-        (&sm[0].hi[0][0])[v] = h;
-        (&sm[0].lo[0][0])[v] = l;
     }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kSums; ++u) (&sm[0].sum[0][0])[u * kLrfWarps * kWarp + threadIdx.x] = sum[u];
     cluster.sync();
     // the other blocks' sums of this block's share of the targets, in rank
     // order, all loads in flight together
@@ -1343,18 +1352,14 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
     const int nb = gridDim.z, share = kLrfTgt / nb, tg0 = blockIdx.z * share;
     for (int v = threadIdx.x; v < share * kLrfMom20; v += blockDim.x) {
         const int t = tg0 + v / kLrfMom20, k = v % kLrfMom20, half = t / kWarp, l = t % kWarp;
-        float2 h[kLrfClusterMax], o[kLrfClusterMax];
+        double2 h[kLrfClusterMax];
 #pragma unroll
         for (int r = 0; r < kLrfClusterMax; ++r)
-            if (r < nb) {
-                const LrfSmem* R = cluster.map_shared_rank(sm, r);
-                h[r] = R->hi[k][l], o[r] = R->lo[k][l];
-            }
-        float hi = 0.f, lo = 0.f;
+            if (r < nb) h[r] = cluster.map_shared_rank(sm, r)->sum[k][l];
+        double d = 0.0;
 #pragma unroll
         for (int r = 0; r < kLrfClusterMax; ++r)
-            if (r < nb) df_add(hi, lo, half ? h[r].y : h[r].x, half ? o[r].y : o[r].x);
-        const double d = (double)hi + (double)lo;
+            if (r < nb) d += half ? h[r].y : h[r].x;
         tot[(t - tg0) * kLrfTot + k] = k == 0 ? d : (k < 4 ? -d : (k < 10 ? 3.0 * d : -15.0 * d));
     }
     __syncthreads();

@@ -3832,6 +3832,7 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, BOX>()) k_rows_solu
         }
         }
         const float rwel = wel.x + wel.y, rwvdw = wvdw.x + wvdw.y;
+        float rpel = 0.f, rpvdw = 0.f;
         // plain partners: LJ code 1 with every row atom, no excluded or 1-4
         // pair; with the geometric rule A and B are the products of the atoms'
         // FP32 code-1 factors (the type table holds the same products).  The
@@ -3839,6 +3840,13 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, BOX>()) k_rows_solu
         // prefetched chunks
         {
           const int niter = (npf + kWarp - 1) / kWarp;
+          // a lane's energies of one chunk are summed by themselves, so that
+          // the FP32 rounding is that of short runs
+          auto fold = [&]() {
+              rpel += pel.x + pel.y, rpvdw += pvdw.x + pvdw.y;
+              pel = pvdw = f2(0.f);
+          };
+          fold();   // the special entries
           for (int it = 0; it < niter; ++it) {
             const int k = it * kWarp + lane;
             const float4 xb = BOX ? at_image(m, xbn, xsw, xrn) : xbn;
@@ -3875,11 +3883,12 @@ __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, BOX>()) k_rows_solu
                 pel = __fadd2_rn(pel, vel);
               }
             }
+            if (it % kIter == kIter - 1) fold();
           }
           cp_async_wait<0>();
+          fold();
         }
         __syncwarp();   // the staging buffers are refilled by the next row
-        const float rpel = pel.x + pel.y, rpvdw = pvdw.x + pvdw.y;
         // The row owns its atoms' pp and pw gradient and its energies: FP32
         // warp sums in a fixed shuffle order, stored without atomics
         // (k_apply_fixed converts each atom's sum once to 64-bit fixed point

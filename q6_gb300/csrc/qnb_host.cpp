@@ -2023,18 +2023,19 @@ int run_compute(qnb_context* c, double Tfree, int istep) {
 }
 // The evaluation of a single-window context between its host transfers: x
 // from h_stage, the gradient (cleared on the device) into h_stage, the energies
-// into h_e, all in one graph.
+// into h_e, all in one graph.  With profiling on, the transfers are launched
+// around run_compute's profiled graph, which has the kernel classes' events.
 int run_host_step(qnb_context* c, double Tfree, int istep) {
     const int n = 3 * c->natom;
+    const bool whole = c->use_graphs && !c->profiling;
     auto f = [&]() -> int {
         launch_host_in(c->h_stage, c->st[0].x, n, c->stream);
-        TRY(enqueue_compute(c, Tfree, istep));
+        TRY(whole ? enqueue_compute(c, Tfree, istep) : run_compute(c, Tfree, istep));
         launch_host_out(c->st[0].d, c->h_stage, n, c->e_all, c->h_e, 2 * kNumE * c->nwin, c->stream);
         c->launches += 2;
         return check_launch();
     };
-    if (!c->use_graphs || c->profiling) return f();
-    return replay(c, c->gslot_host[watpol_update_step(c, istep) ? 1 : 0], Tfree, f);
+    return whole ? replay(c, c->gslot_host[watpol_update_step(c, istep) ? 1 : 0], Tfree, f) : f();
 }
 
 // adds the energies of every window, as read into e, into E / EQ / Erst

@@ -304,12 +304,12 @@ int qnb_set_solvent_internal(qnb_context* ctx, int32_t n, const int32_t* ij, con
    (the evaluation's parallel branches off, so each class runs alone), the
    candidate blocks-per-SM of each per-step kernel class and of the list
    build, one parameter at a time, and keeps the fastest.  Results are
-   independent of these choices.  The Q chunk is kept: it set the grouping of
-   partial sums in earlier Q kernels and no kernel reads it.  Needs built lists;
-   restores the watpol running averages and clears the gradient
-   accumulators.  values (may be NULL) receives the QNB_TUNE_COUNT choices:
-   solute rows, water rows, qp, qw (blocks per SM), Q chunk (units), LRF
-   Taylor, LRF accumulation, row build (blocks per SM). */
+   independent of these choices.  Needs built lists; restores the watpol
+   running averages and clears the gradient accumulators.  values (may be
+   NULL) receives the QNB_TUNE_COUNT choices: solute rows, water rows, qp, qw
+   (blocks per SM), Q chunk, LRF Taylor (blocks per SM), LRF accumulation, row
+   build (blocks per SM).  No kernel reads the Q chunk or the LRF
+   accumulation's value: both are accepted and kept as they are. */
 enum { QNB_TUNE_COUNT = 8 };
 int qnb_autotune(qnb_context* ctx, int32_t reps, int32_t* values);
 int qnb_get_tuning(qnb_context* ctx, int32_t* values);

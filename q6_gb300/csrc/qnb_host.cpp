@@ -2159,14 +2159,12 @@ int qnb_set_tuning(qnb_context* c, const int32_t* values) {
 
 // Autotuner: coordinate search over the launch geometry of the per-step
 // kernels (blocks per SM of the solute rows, water rows, qp, qw and LRF
-// Taylor kernels) and of the list build (row build, LRF accumulation), each
-// candidate timed with CUDA events over `reps` evaluations (or builds) of the
-// current lists and coordinates after one untimed run.  Results do not
-// depend on these choices (the mixed form is bit-identical for every one).
-// The Q-kernel chunk size is not searched: it sets the grouping of the Q
-// energies' FP32 partial sums (qnb_set_tuning can still change it).  The
-// watpol running averages are restored afterwards; the gradient accumulators
-// are cleared.
+// Taylor kernels) and of the row build, each candidate timed with CUDA events
+// over `reps` evaluations (or builds) of the current lists and coordinates
+// after one untimed run.  Results do not depend on these choices (the mixed
+// form is bit-identical for every one).  T_QCHUNK and T_LRF, which no kernel
+// reads, keep their values.  The watpol running averages are restored
+// afterwards; the gradient accumulators are cleared.
 int qnb_autotune(qnb_context* c, int32_t reps, int32_t* values) {
     if (!c) return fail(QNB_ERR_ARG, "null context");
     if (!c->lists_built) return fail(QNB_ERR_STATE, "pair lists not built");
@@ -2224,7 +2222,6 @@ int qnb_autotune(qnb_context* c, int32_t reps, int32_t* values) {
         {T_TAYLOR, {8, 16, 24, 32, 48, 64}, B << K_LRF_TAYLOR, false},
     };
     if (c->mixed) plan.push_back({T_BUILD, {8, 16, 24, 32, 48, 64}, B << K_BUILD, true});
-    if (c->mixed && c->use_lrf) plan.push_back({T_LRF, {2, 3, 4, 6, 8, 12}, B << K_LRF_BUILD, true});
     int rc = QNB_OK;
     for (auto& p : plan) {
         int best = c->tune.v[p.t];

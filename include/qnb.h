@@ -653,7 +653,12 @@ typedef struct qnb_md_record {
 
 /* mass[natom] (amu); the constraints of molecule m are
    con_ij[2k], con_ij[2k+1] (0-based atoms) at distance con_dist[k] (A) for
-   k in [mol_first[m], mol_first[m+1]), m < nmol.  Velocities start at 0. */
+   k in [mol_first[m], mol_first[m+1]), m < nmol.  Velocities start at 0.
+   In the mixed form, list builds after this call sum the LRF moments in
+   another order than before it (the one the context's trajectories have
+   always had): at the same coordinates the records differ by FP32 rounding,
+   about 2e-6 of each coefficient order's largest value; both are equally
+   near to the FP64 form's. */
 int qnb_md_init(qnb_context* ctx, const qnb_md_params* p, const double* mass, int32_t nmol,
                 const int32_t* mol_first, const int32_t* con_ij, const double* con_dist);
 /* Thermostat and integrator (the input's thermostat / integrator keys,

@@ -502,18 +502,15 @@ int build_model(qnb_context* c, const qnb_topology* t) {
         if (!gallq[g]) c->maxg = std::max(c->maxg, gslot[g + 1] - gslot[g]);
     }
     TRY(c->upload((uint8_t**)&m.gallq, gallq));
-    std::vector<int> gnq_off{0}, gnq_atom;
+    std::vector<int> gnq_off{0};
     std::vector<int2> gnq_rec;
     for (int g = 0; g < t->ncgp_solute; ++g) {
         for (int a = gslot[g]; a < gslot[g + 1]; ++a)
-            if (iqatom[gatom[a]] < 0) {
-                gnq_atom.push_back(gatom[a]);
+            if (iqatom[gatom[a]] < 0)
                 gnq_rec.push_back(make_int2(gatom[a], (iac[gatom[a]] & 0xffff) | (a - gslot[g]) << 16));
-            }
-        gnq_off.push_back((int)gnq_atom.size());
+        gnq_off.push_back((int)gnq_rec.size());
     }
     TRY(c->upload((int**)&m.gnq_off, gnq_off));
-    TRY(c->upload((int**)&m.gnq_atom, gnq_atom));
     TRY(c->upload((int2**)&m.gnq_rec, gnq_rec));
     // must agree with k_rows_solute's template choice (MAXG <= 8)
     m.type_in_entry = (c->maxg <= 8 && t->natyps <= 0xffff) ? 1 : 0;
@@ -1326,10 +1323,10 @@ using SideWork = std::function<int(const Launch& terms, const Launch& boundary, 
 // of the 104 us step of a 1,358-atom droplet); a large batch fills the device
 // from any of them.  One stream when the branches are off.
 struct EvalBranches {
-    Launch main, ww, q, side, wat, bonded;
+    Launch ww, q, side, wat, bonded;
 };
 EvalBranches fork_branches(qnb_context* c, const Launch& L, bool parallel, bool bonded, int* rc) {
-    EvalBranches b{L, L, L, L, L, L};
+    EvalBranches b{L, L, L, L, L};
     *rc = QNB_OK;
     if (!parallel) return b;
     b.q.st = c->stream2;
@@ -2600,7 +2597,7 @@ int qnb_md_init(qnb_context* c, const qnb_md_params* p, const double* mass, int3
     CU(cudaMallocHost((void**)&c->h_md_rec, sizeof(double) * kMdChunk * c->nwin * kMdRec));
     if (c->mixed && c->use_lrf)
         for (int w = 0; w < c->nwin; ++w)
-            TRY(c->alloc(&c->st[w].lrf_part, (size_t)kLrfSplitMax * std::max(1, c->ncgp) * kLrfMoments));
+            TRY(c->alloc(&c->st[w].lrf_part, (size_t)kLrfSplitMax * std::max(1, c->ncgp) * kLrfMom20));
     // restrain_solvent of an MD step reads the window's Tfree on the device
     for (int w = 0; w < c->nwin; ++w) c->st[w].md_tfree = &md.win[w].tfree;
     TRY(upload_states(c));

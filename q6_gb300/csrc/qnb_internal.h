@@ -13,7 +13,7 @@ constexpr int kMaxSolv = 4;     // atoms per solvent molecule handled on device
 constexpr int kMaxStates = 8;   // FEP states
 constexpr int kMaxShell = 16;   // water polarisation shells
 constexpr int kLrfLen = 43;     // cgp_cent(3) phi0 phi1(3) phi2(9) phi3(27)
-constexpr int kLrfMoments = 24; // symmetric moments the LRF accumulation sums per target group
+constexpr int kLrfMom20 = 20;   // symmetric moments the LRF accumulation sums per target group (see lrf_moments24)
 constexpr int kLrfSplitMax = 8;     // source ranges of the mixed form's accumulation in MD contexts
 constexpr int kLrfTileGroups = 16;  // source groups it stages at a time
 constexpr int kLrfClusterMax = 4;   // blocks per cluster of the mixed form's LRF accumulation
@@ -134,8 +134,7 @@ struct DevModel {
     int geom;
     const ulonglong2* gtmask;           // [ncgp_solute] types 0-63 (x) and 64-127 (y)
     const int* gnq_off;                 // [ncgp_solute+1] non-Q atoms of each solute group
-    const int* gnq_atom;
-    const int2* gnq_rec;                // the same: atom, its type (16 bits) and its place in the group << 16
+    const int2* gnq_rec;                // atom, its type (16 bits: the natyps^2 tables keep it far below) and its place in the group << 16
     const uint8_t* gallq;               // [ncgp_solute] 1: every atom of the group is a Q atom (no pair row)
     const float2* ljf1;                 // [natom]
     // LRF sources grouped by charge group (mixed form's accumulation):
@@ -192,7 +191,7 @@ struct DevState {
     unsigned long long* efix;  // [kNumE] fixed-point energies (mixed form)
     double* lambda;      // [S]
     double* lrf;         // [ncgp*43]
-    double* lrf_part;    // mixed form, MD contexts: [kLrfSplitMax][ncgp][kLrfMoments] LRF moments per source range
+    double* lrf_part;    // mixed form, MD contexts: [kLrfSplitMax][ncgp][kLrfMom20] LRF moments per source range
     int* cnt;            // [C_NUM] list sizes (device-maintained)
     int2* ww; int64_t cap_ww;      // water pairs (iw, jw), iw < jw
     int2* pw; int64_t cap_pw;      // (solute atom, water)

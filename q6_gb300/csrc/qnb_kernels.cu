@@ -669,7 +669,7 @@ __device__ __forceinline__ int group_dist_atom(const DevModel& m, int g) {
 //   m[21..23] U(c)    += f2 r2 dr_c
 // with f0 = q/r^3, f1 = 3 f0/r^2, f2 = -f1/r^2.  lrf_expand rebuilds the 40
 // reference coefficients, including its diagonal corrections of phi3.
-constexpr int kLrfMom = kLrfMoments;
+constexpr int kLrfMom = 24;
 template <typename T>
 __device__ __forceinline__ void lrf_terms(T dx, T dy, T dz, T q, T* m) {
     T r2 = dx * dx + dy * dy + dz * dz;
@@ -755,7 +755,6 @@ __device__ __forceinline__ void lrf_expand(const double* m, double* L) {
 // U(c) = (S3(xxc) + S3(yyc) + S3(zzc)) / 5 (dr_x^2 + dr_y^2 + dr_z^2 = r2), so
 // they are formed in FP64 from the totals instead of summed per atom.
 //   n[0] phi0, n[1..3] phi1, n[4..9] S2, n[10..19] S3 (the order of lrf_terms)
-constexpr int kLrfMom20 = 20;
 // the 24 moments of lrf_expand from the 20 (FP64)
 __device__ __forceinline__ void lrf_moments24(const double* n, double* m) {
     for (int k = 0; k < 10; ++k) m[k] = n[k];
@@ -3597,9 +3596,6 @@ __device__ __forceinline__ float4 at_image(const DevModel& m, float4 p, float4 r
     return p;
 }
 
-#ifndef QNB_ROWS_MIN_BLOCKS
-#define QNB_ROWS_MIN_BLOCKS 0   // 0: the per-size default below
-#endif
 // resident 128-thread blocks per SM the row kernel is compiled for, groups of
 // up to 6 atoms, 51 windows of the 25 A sphere: 4 blocks (128 registers) 161 us
 // alone, 5 (96) 163, 6 (80, spilling inside the loop) 193; the box's lattice
@@ -3607,7 +3603,7 @@ __device__ __forceinline__ float4 at_image(const DevModel& m, float4 p, float4 r
 // step beside the other branches was the shorter (457 against 471 us a pass)
 template <int MAXG, bool BOX>
 constexpr int rows_min_blocks() {
-    return QNB_ROWS_MIN_BLOCKS ? QNB_ROWS_MIN_BLOCKS : (MAXG <= 6 ? (BOX ? 4 : 5) : (MAXG <= 8 ? 4 : 1));
+    return MAXG <= 6 ? (BOX ? 4 : 5) : (MAXG <= 8 ? 4 : 1);
 }
 template <int MAXG, bool GEOM, bool BOX>
 __global__ void __launch_bounds__(128, rows_min_blocks<MAXG, BOX>()) k_rows_solute(DevModel m, const DevState* __restrict__ states) {
@@ -4103,9 +4099,9 @@ __global__ void __launch_bounds__(128, 8) k_rows_water(DevModel m, const DevStat
             int b = m.gnq_off[g], nt = 0;
             float4 nx = make_float4(0.f, 0.f, 0.f, 0.f);
             auto load = [&](int b) {
-                const int j = m.gnq_atom[b];
-                nx = xq[j];
-                nt = m.iac[j];
+                const int2 rec = m.gnq_rec[b];
+                nx = xq[rec.x];
+                nt = rec.y & 0xffff;
             };
             if (b < a1) load(b);
             for (; b < a1; ++b) {

@@ -1215,7 +1215,7 @@ int grow_lists(qnb_context* c, bool* grew, bool* do_qp, bool* do_qw) {
     return QNB_OK;
 }
 
-constexpr int64_t kLrfBehindRows = 16384;   // rows of all windows from which the LRF moments follow the row build
+constexpr int64_t kLrfBehindRows = 32768;   // rows of all windows from which the LRF moments follow the row build
 
 int build_lists(qnb_context* c, const Cut& cut, int nw) {
     Launch L = nw == 1 ? c->one() : c->all();
@@ -1241,10 +1241,12 @@ int build_lists(qnb_context* c, const Cut& cut, int nw) {
         // a large batch, whose row build fills the device by itself, behind it
         // instead.  Side by side they also share each SM's 256 KB: rows built
         // while or after the accumulation holds 190 KB of it as shared memory
-        // have little L1 cache left.  51 windows of the 25 A sphere (87,000
-        // rows): 1,968 us side by side, 1,635 us one after the other; 16
-        // windows in a box (27,000): 1,000 and 888; one window (1,700): 139
-        // and 187.
+        // have little L1 cache left.  A list build of 25 A spheres (1,713 rows
+        // a window, side by side / one after the other): 1 window 102 / 141
+        // us, 4 158 / 194, 8 270 / 298, 12 374 / 392, 16 (27,408 rows) 497 /
+        // 494, 24 (41,112) 710 / 696, 51 (87,363) 1,968 / 1,635 before later
+        // steps.  Of 15 A droplets (451 rows, hardly any of them solute): 51
+        // windows (23,001) 211 / 232, 80 (36,080) 290 / 314.
         const bool rows = c->mixed && (!c->m.box || c->m.box_rows);
         const bool behind = rows && (int64_t)nw * (c->ncgp_solute + c->nwat) >= kLrfBehindRows;
         auto lrf = [&]() -> int {

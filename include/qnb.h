@@ -19,8 +19,10 @@
  *    sqrt(coulomb_constant) (Q6 src/simprep.f90:3714-3721).
  *  - Every function returns a qnb_status; 0 is success.  The library never
  *    falls back to a CPU path: without a usable CUDA device, qnb_create fails.
- *  - A context is used by one host thread at a time; all its work is issued on
- *    one CUDA stream owned by the context.
+ *  - A context is used by one host thread at a time.  Its work is issued on
+ *    CUDA streams of its own: one that every call's work starts and ends on
+ *    (qnb_stream), and further ones for the parallel branches of a list build
+ *    or an evaluation, which the first waits for.
  */
 #ifndef QNB_H
 #define QNB_H
@@ -363,9 +365,10 @@ int qnb_profile_collect(qnb_context* ctx);
 
 /* Branches of the evaluation (on by default): after the coordinate pack the
    solute pairs run on the context's stream; the water pairs, the
-   Q-environment terms, the LRF Taylor and further terms (qq, bonded,
-   restraints), and the solvent boundary terms on streams of their own, all
-   joined before the fixed-point gradient apply.  The FP64 form does the same
+   Q-environment terms, the LRF Taylor and further terms (qq, restraints), the
+   solvent boundary terms, and the bonded terms if there are any on streams of
+   their own, all joined before the fixed-point gradient apply (with excluded
+   atoms frozen the boundary and bonded terms are among the further terms).  The FP64 form does the same
    on the sphere unless excluded atoms are frozen; its box path runs in one
    stream.  The mixed form's sums are fixed point, so its results are the same
    with enable = 0, which runs everything in one stream (each kernel then has
@@ -408,7 +411,11 @@ int qnb_q_adjoint_dev(qnb_context* ctx, double* dq, double* dA, double* dB);
 int qnb_take_launch_count(qnb_context* ctx, int64_t* n);
 
 /* ---- event profiler (diagnostics; no counterpart in the reference) -------- */
-/* Kernel classes, in the order qnb_kernel_times reports them. */
+/* Kernel classes, in the order qnb_kernel_times reports them.  In
+   qnb_compute_dev, qnb_step_host, qnb_pot_energy_step and qnb_md_run the
+   radial restraint and watpol's angles are one kernel: RESTRAIN times it with
+   the shell and input restraints (and watpol's theta_corr update), WATPOL the
+   selection order, forces and averages. */
 enum {
     QNB_K_WW = 0, QNB_K_QW, QNB_K_PW, QNB_K_PP, QNB_K_QP, QNB_K_LRF_TAYLOR, QNB_K_QQ,
     QNB_K_RESTRAIN, QNB_K_WATPOL, QNB_K_PACK, QNB_K_APPLY, QNB_K_BUILD, QNB_K_LRF_BUILD,
@@ -416,8 +423,8 @@ enum {
     QNB_K_COUNT
 };
 
-/* Brackets every launch of each kernel class with CUDA events on the
-   context's stream while enable != 0. */
+/* Brackets every launch of each kernel class with CUDA events on the stream
+   it is issued on while enable != 0. */
 int qnb_profile(qnb_context* ctx, int32_t enable);
 /* Profiling of the kernel classes whose bits (1 << QNB_K_*) are set only;
    0 turns profiling off.  Fewer events, less perturbation of the timing. */

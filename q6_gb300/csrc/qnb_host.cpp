@@ -1320,10 +1320,11 @@ using SideWork = std::function<int(const Launch& terms, const Launch& boundary, 
 // terms and qq they made that branch the longest of an MD step: 25 steps of 16
 // windows of 3,379 atoms 5.67 -> 5.51 ms).  No branch reads what another
 // writes, and every sum is an atomic one (fixed point in the mixed form, so
-// its result does not depend on their interleaving).  A small system's step is as long as its longest branch
-// (the water rows, qq, restrain_solvent and watpol in one branch took 55 us
-// of the 104 us step of a 1,358-atom droplet); a large batch fills the device
-// from any of them.  One stream when the branches are off.
+// its result does not depend on their interleaving).  A small system's step is
+// as long as its longest branch (the water rows, qq, restrain_solvent and
+// watpol in one branch took 55 us of the 104 us step of a 1,358-atom droplet);
+// a large batch fills the device from any of them.  One stream when the
+// branches are off.
 struct EvalBranches {
     Launch ww, q, side, wat, bonded;
 };
@@ -1374,8 +1375,8 @@ int compute_nonbond(qnb_context* c, int md, int nw, const SideWork& side = SideW
     // kernels read them directly): one stream then
     const bool par = c->branches && (rows || (!mx && !c->m.box && !c->freeze));
     int rc = QNB_OK;
-    // with excluded_freeze the boundary and bonded terms stay behind the kernel
-    // that puts the excluded atoms back
+    // with excluded_freeze the boundary terms stay behind the kernel that puts
+    // the excluded atoms back, and the bonded terms ahead of it
     const bool bonded = side && c->have_bonded && !c->freeze;
     EvalBranches b = fork_branches(c, L, par, bonded, &rc);
     TRY(rc);

@@ -917,10 +917,9 @@ __device__ __forceinline__ void two_sum_fold(float& hi, float& lo, float& p) {
     p = 0.f;
 }
 
-// Its 20 moments in packed FP32x2 arithmetic: the source
+// Its 20 moments (n of lrf_moments24) in packed FP32x2 arithmetic: the source
 // atom's (x, y) and (z, q) arrive as register pairs from the staged float4,
-// and the 20 sums are held as 10 pairs, so 10 FFMA2 replace 20 FFMA.  Each
-// sum gets the same products in the same order as in lrf_terms20.  Slots
+// and the 20 sums are held as 10 pairs, so 10 FFMA2 replace 20 FFMA.  Slots
 // (lrf_slot):
 // (n1,n2) (n3,n0) (n4,n5) (n6,n9) (n7,n8) (n10,n11) (n12,n19) (n13,n16)
 // (n14,n17) (n15,n18).
@@ -1089,12 +1088,14 @@ __global__ void k_lrf_combine(DevModel m, const DevState* __restrict__ states, i
 // each block expands its share of the targets: no partial sums in global
 // memory, no second kernel.  The tiles are fixed by the topology alone, so a
 // window's coefficients do not depend on the launch or the number of windows.
-// Alone: 51 windows of the 25 A sphere 1.30 -> 0.95 ms, 8 of a 34 A sphere
-// 1.85 -> 1.18 ms, one of 25 A 140 -> 62 us (with a range of neighbouring
-// groups per warp: 1.06 and 1.28 ms, 70 us; tiles in turn, their indices read
-// only when they are staged: 0.97, 1.20, 64).  The FMA pipe is busy 54 % of
-// the time, the rest is latency at four warps per scheduler.  Records as far
-// from FP64 as before (2e-6 of their scale).
+// Alone: 51 windows of the 25 A sphere 1.30 -> 1.04 ms, 8 of a 34 A sphere
+// 1.85 -> 1.30 ms, one of 25 A 140 -> 68 us (with one fold per tile 0.95, 1.18
+// and 62; so folded, with a range of neighbouring groups per warp 1.06, 1.28
+// and 70, with the tiles' indices read only when they are staged 0.97, 1.20
+// and 64).  The FMA pipe is busy 57 % of the time, the rest is latency at four
+// warps per scheduler.  The records' root mean square distance from FP64 is
+// 0.94 to 1.02 times that of k_lrf_nbody's with charges of one sign, where the
+// sums' rounding shows (one fold per tile: 1.05 to 1.29).
 constexpr int kLrfWarps = 4;
 constexpr int kLrfTgt = 64;    // targets per cluster
 constexpr int kLrfTile = kLrfTileGroups;   // source groups per staged tile
@@ -1382,7 +1383,7 @@ __global__ void __launch_bounds__(kLrfWarps * kWarp, 4) k_lrf_pairs(DevModel m, 
 // FP64 form: one warp per target group reads the source atoms straight from
 // global memory (lanes stride over the atoms, so loads are coalesced); its
 // terms bound it (the FP64 pipe: 16 windows of the 25 A sphere 20.6 ms with
-// two divisions, a square root and 24 sums per term, 13.4 ms with these).
+// two divisions, a square root and 24 sums per term, 16.4 ms with these).
 template <bool BOX>
 __global__ void __launch_bounds__(128) k_lrf_accumulate64(DevModel m, const DevState* __restrict__ states, Cut c,
                                                           const int* __restrict__ lrf_src) {
@@ -1584,7 +1585,7 @@ __global__ void __launch_bounds__(128) k_lrf_accumulate_any_box(DevModel m, cons
 // form's kernels are bound by the FP64 pipe (84 % busy at two lanes per clock
 // and SM), where the reference's division and square root of the quotient
 // were 15 of a pair's 37 operations (16 windows of the 25 A sphere: pp 774 ->
-// 661 us, ww 269 -> 185, pw 212 -> 165).  See inv_dist for its rounding.
+// 695 us, ww 269 -> 197, pw 212 -> 176).  See inv_dist for its rounding.
 struct PairD {
     double tx, ty, tz, dv, vel, vdw;
 };
@@ -1796,25 +1797,6 @@ struct QPairF {
     }
 };
 
-// ---------------------------------------------------------------------------
-// Adjoint of the Q-atom energies with respect to the Q parameters: for every
-// Q atom iq and state s, dE_s/dqcrg(iq,s), dE_s/dqA(iq,s) and dE_s/dqB(iq,s),
-// where qA/qB are the Q atom's code-1 LJ factors (A_pair = qA * a_j,
-// B_pair = qB * b_j, geometric rule).  The pair terms are recomputed from the
-// lists: E_s = sum el/r + A/(r^6+alpha)^2 - B/(r^6+alpha) (nbe_qx,
-// src/nonbonded.f90:200-222), so
-//   dE/dqcrg += c_j / r,  dE/dqA += a_j / (r^6+alpha)^2,  dE/dqB -= b_j / (r^6+alpha).
-// One warp per environment unit, lane = Q atom, sums in FP64 registers.
-// ---------------------------------------------------------------------------
-// Mixed form, transposed: lane = environment unit (a listed solute atom or
-// water), each warp taking a fixed chunk of 32 consecutive units, and a loop
-// over the Q atoms with their coordinates in shared memory.  An environment
-// atom's gradient stays in its lane (stored once, no reduction); a Q atom's
-// gradient is a fixed-order warp sum per Q atom and chunk, added to the
-// block's fixed-point total; each unit's per-state energies are converted
-// once.  The sums do not depend on the grid.  qw's parameters are the same
-// for all lanes (broadcast); qp's come from the [Q atom][solute atom] table,
-// so lanes holding consecutive solute atoms read consecutive entries.
 // periodic box, mixed form's FP32 pair geometry: packed coordinates
 // (xpcent-centred) and an FP32 lattice shift of a against b (boxlength *
 // nint((a - b) / boxlength)); a pair vector is shift - (x_i - x_j)
@@ -1853,6 +1835,15 @@ __device__ __forceinline__ T reduce_scatter(T (&g)[N], int lane) {
 }
 constexpr int kQRed = 5;   // Q atoms per transposed reduction (15 of its 16 values)
 
+// Mixed form, transposed: lane = environment unit (a listed solute atom or
+// water), each warp taking a fixed chunk of 32 consecutive units, and a loop
+// over the Q atoms with their coordinates in shared memory.  An environment
+// atom's gradient stays in its lane (stored once, no reduction); a Q atom's
+// gradient is a fixed-order warp sum per Q atom and chunk, added to the
+// block's fixed-point total; each unit's per-state energies are converted
+// once.  The sums do not depend on the grid.  qw's parameters are the same
+// for all lanes (broadcast); qp's come from the [Q atom][solute atom] table,
+// so lanes holding consecutive solute atoms read consecutive entries.
 //
 // BOX (nonbond_qp_box, src/nonbondene.f90:5234-5335; nonbond_qw_box /
 // nonbond_qw_spc_box, 5422-5505, 5771-5881): each unit is taken at the image
@@ -2014,13 +2005,13 @@ __global__ void __launch_bounds__(kQLaneBlock) k_qenv_lanes(DevModel m, const De
 // water or solute atom) against kQRed Q atoms: the environment atoms'
 // gradients stay in the lane, the Q atoms' are summed over the warp in one
 // transposed butterfly, both are added with FP64 atomics.  The FP64 pipe bounds
-// it: r^6 is d2^3 instead of 1/(1/d2)^3, 1/distance one rsqrt, and states whose
-// soft-core alpha equals the state before's (compared bit for bit) share the
-// division.  Splitting the Q atoms over warps as well spreads a single window
+// it: r^6 is d2^3 instead of 1/(1/d2)^3, 1/distance and its square come from
+// one rsqrt (inv_dist), and states whose soft-core alpha equals the state
+// before's (compared bit for bit) share the division.  Splitting the Q atoms over warps as well spreads a single window
 // over the device (with lane = Q atom and eight units per warp, 6 Q atoms kept
 // 6 of 32 lanes busy on 56 warps: 118 us for 446 waters; 20 Q atoms and 16
-// windows of 1,020 waters 339 us, of 2,955 solute atoms 285 us; now 32, 109
-// and 137 us).
+// windows of 1,020 waters 339 us, of 2,955 solute atoms 285 us; now 33, 120
+// and 141 us).
 template <bool SPC, bool WATER, int NA, int SMAX, bool BOX>
 __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __restrict__ states,
                                                 const int* __restrict__ iwhich, double rcq2) {
@@ -2136,9 +2127,16 @@ __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __re
     }
 }
 
-// Adjoint of the Q-environment terms in FP64 in both precision forms: the
-// adjoint is an occasional call for parameter fitting, and FP64 geometry keeps
-// its gradients to the FP64 reference's rounding.  The FP64 pipe (two lanes
+// Adjoint of the Q-atom energies with respect to the Q parameters: for every
+// Q atom iq and state s, dE_s/dqcrg(iq,s), dE_s/dqA(iq,s) and dE_s/dqB(iq,s),
+// where qA/qB are the Q atom's code-1 LJ factors (A_pair = qA * a_j,
+// B_pair = qB * b_j, geometric rule).  The pair terms are recomputed from the
+// lists: E_s = sum el/r + A/(r^6+alpha)^2 - B/(r^6+alpha) (nbe_qx,
+// src/nonbonded.f90:200-222), so
+//   dE/dqcrg += c_j / r,  dE/dqA += a_j / (r^6+alpha)^2,  dE/dqB -= b_j / (r^6+alpha).
+// FP64 in both precision forms: the adjoint is an occasional call for
+// parameter fitting, and FP64 geometry keeps its gradients to the FP64
+// reference's rounding.  The FP64 pipe (two lanes
 // per clock and SM) bounds it.
 //
 // Lanes: P = the power of two that holds the Q atoms (at most 32; the rest of
@@ -2153,7 +2151,6 @@ __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __re
 // multiply-add and a load per state, an O one division instead of S.
 // With the windows' sums cleared and copied at once, 200 windows of 439 waters,
 // 30 Q atoms and 4 states: 3.35 -> 0.53 ms a call (lists apart).
-//
 constexpr int kQAdjSlots = 3 * kMaxQ * kMaxStates;
 template <bool FACTORED, bool SPC, bool WATER, int SMAX>
 __global__ void __launch_bounds__(kQBlock) k_qadj_env(DevModel m, const DevState* __restrict__ states, int P) {
@@ -2641,7 +2638,7 @@ __device__ __forceinline__ void watpol_theta(const DevModel& m, const DevState& 
     s.rkey[w] = 0.0;
     int i = m.nat_solute + m.sa * w;
     if (m.excl[i]) return;
-    double* v = s.wvec + 8 * (size_t)w;   // reused by k_watpol_force in the same call
+    double* v = s.wvec + 8 * (size_t)w;   // read by k_watpol_rank_force in the same call
     double rcd;
     if (MIX && m.sa == 3) {
         const double* x = s.x;
@@ -2829,6 +2826,9 @@ __global__ void k_watpol_force(DevModel m, const DevState* __restrict__ states, 
 // over.  As five kernels (reset, rank, force, average and the radial restraint
 // beside theta) the boundary branch was the longest of a small system's step.
 constexpr int kRankBlock = 256;
+// 4 parts: one window of the 25 A sphere 28 us (with the launch), 8 20; 8
+// windows of the 34 A sphere 203 and 178 us a step; 51 windows, which fill the
+// device with 4 as well, 18 and 22 us for 15 A, 38 for 25 A with both
 constexpr int kRankParts = 8;
 template <bool MIX>
 __global__ void __launch_bounds__(kRankBlock) k_watpol_rank_force(DevModel m, const DevState* __restrict__ states, SolventDev p) {
@@ -3534,8 +3534,8 @@ constexpr int kRowChunk = 128;   // entries per prefetched chunk
 //
 // All terms are packed (pair2), in the order of the scalar sums they replace,
 // and the row atoms' LJ factors and types are read from shared memory, so the
-// registers hold positions, charges and gradients only: 187 -> 163 us per
-// 51-window R25 step, 262 -> 178 us in the box (whose partners' reference
+// registers hold positions, charges and gradients only: 187 -> 166 us per
+// 51-window R25 step, 262 -> 184 us in the box (whose partners' reference
 // positions come from one array instead of two dependent loads).
 // Two row atoms against one partner in packed FP32x2 arithmetic (GB300's
 // FFMA2 / FMUL2 / FADD2; one rsqrt per atom on the SFU): the row kernels are
@@ -3598,9 +3598,11 @@ __device__ __forceinline__ float4 at_image(const DevModel& m, float4 p, float4 r
 
 // resident 128-thread blocks per SM the row kernel is compiled for, groups of
 // up to 6 atoms, 51 windows of the 25 A sphere: 4 blocks (128 registers) 161 us
-// alone, 5 (96) 163, 6 (80, spilling inside the loop) 193; the box's lattice
-// images hold more registers: 178, 223 and 245 us.  5 on the sphere, where the
-// step beside the other branches was the shorter (457 against 471 us a pass)
+// alone, 5 (96, with 112 bytes of spill stores) 163, 6 (80, spilling inside the
+// plain loop) 193; the box's lattice images hold more registers: 178, 223 and
+// 245 us (all before the energies' chunk sums, which cost 3 to 5 us).  5 on the
+// sphere, where the step beside the other branches was the shorter (457 against
+// 471 us a pass)
 template <int MAXG, bool BOX>
 constexpr int rows_min_blocks() {
     return MAXG <= 6 ? (BOX ? 4 : 5) : (MAXG <= 8 ? 4 : 1);
@@ -3956,7 +3958,7 @@ __device__ __forceinline__ float2 coul2(float2 tx, float2 ty, float2 tz, float2 
 // sum in the order of the scalar terms, so the gradient is theirs bit for bit
 // (a trajectory amplifies rounding).  A lane takes a listed group's non-Q atoms
 // one after the other, the next one's data loaded ahead.  51 windows of the 25 A
-// sphere 110 -> 86 us, of the 15 A droplet 44 -> 36 us.  (Solute partners as a
+// sphere 110 -> 84 us, of the 15 A droplet 44 -> 36 us.  (Solute partners as a
 // list of atoms instead of groups measured 73 us, but sums them in another
 // order.)
 template <bool SPC, bool BOX>
@@ -4300,8 +4302,9 @@ int launch_lrf_accumulate(const Launch& L, const Cut& c, int mixed, const int* l
         // blocks per cluster: ranges of at least one tile per warp, the split
         // set by the topology only, so a window's coefficients are the same in
         // a batch of any size.  At most 4: 8 sped up a single window (R25: 63
-        // -> 54 us) and slowed 51 windows (953 -> 1,191 us); 2, measured when
-        // each warp summed one range, the reverse (74 -> 130, 1,100 -> 1,085)
+        // -> 54 us) and slowed 51 windows (953 -> 1,191 us), both with one fold
+        // per tile; 2, measured when each warp summed one range, the reverse
+        // (74 -> 130, 1,100 -> 1,085)
         int nz = 1;
         while (nz < kLrfClusterMax && L.m.nlrf_groups >= 2 * nz * kLrfWarps * kLrfTile) nz *= 2;
         const int tile_atoms = std::max(96 / nz, (L.m.lrf_tile_atoms + 3) & ~3);   // 96 / nz: the totals' space

@@ -126,7 +126,7 @@ def _p(a):
 
 
 class NonbondedEngine:
-    """One qdyn system on one GPU (one CUDA stream)."""
+    """One qdyn system on one GPU."""
 
     def __init__(self, system: QSystem, precision: int = PREC_FP64, use_lrf: bool = True,
                  device: int = 0, windows: int = 1):

@@ -2002,7 +2002,7 @@ __global__ void __launch_bounds__(kQLaneBlock) k_qenv_lanes(DevModel m, const De
 // FP64 form of the Q-environment terms: nonbond_qw_spc / nonbond_qw
 // (src/nonbondene.f90:5658-5767, 5339-5418), nonbond_qp (5157-5230) and their
 // box forms (see k_qenv_lanes).  A warp takes 32 consecutive units (lane =
-// water or solute atom) against kQRed Q atoms: the environment atoms'
+// water or solute atom) against qb <= kQRed Q atoms: the environment atoms'
 // gradients stay in the lane, the Q atoms' are summed over the warp in one
 // transposed butterfly, both are added with FP64 atomics.  The FP64 pipe bounds
 // it: r^6 is d2^3 instead of 1/(1/d2)^3, 1/distance and its square come from
@@ -2010,20 +2010,20 @@ __global__ void __launch_bounds__(kQLaneBlock) k_qenv_lanes(DevModel m, const De
 // before's (compared bit for bit) share the division.  Splitting the Q atoms over warps as well spreads a single window
 // over the device (with lane = Q atom and eight units per warp, 6 Q atoms kept
 // 6 of 32 lanes busy on 56 warps: 118 us for 446 waters; 20 Q atoms and 16
-// windows of 1,020 waters 339 us, of 2,955 solute atoms 285 us; now 33, 120
+// windows of 1,020 waters 339 us, of 2,955 solute atoms 285 us; now 14, 120
 // and 141 us).
 template <bool SPC, bool WATER, int NA, int SMAX, bool BOX>
 __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __restrict__ states,
-                                                const int* __restrict__ iwhich, double rcq2) {
+                                                const int* __restrict__ iwhich, double rcq2, int qb) {
     const DevState& s = states[blockIdx.y];
     const double* __restrict__ x = s.x;
     Acc<false> acc = make_acc<false>(s);
     const int lane = threadIdx.x & 31, S = m.S, nq = m.nqat, na = WATER ? m.sa : 1;
     const int n = WATER ? min((int64_t)s.cnt[C_QW], s.cap_qw) : min((int64_t)s.cnt[C_QP], s.cap_qp);
-    const int nqb = (nq + kQRed - 1) / kQRed, items = (n + kWarp - 1) / kWarp * nqb;
+    const int nqb = (nq + qb - 1) / qb, items = (n + kWarp - 1) / kWarp * nqb;
     ESum<false> eel[SMAX], evdw[SMAX];
     for (int it = warp_id_global(); it < items; it += warps_total()) {
-        const int p = it / nqb * kWarp + lane, q0 = it % nqb * kQRed;
+        const int p = it / nqb * kWarp + lane, q0 = it % nqb * qb, q1 = min(nq, q0 + qb);
         const bool act = p < n;
         const int j0 = act ? (WATER ? m.nat_solute + m.sa * s.qw[p] : s.qp[p]) : 0;
         double xj[NA][3], gj[NA][3];
@@ -2052,7 +2052,7 @@ __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __re
 #pragma unroll
         for (int b = 0; b < kQRed; ++b) {
             const int iq = q0 + b;
-            if (iq >= nq) break;   // warp-uniform
+            if (iq >= q1) break;   // warp-uniform
             double xi[3], gx = 0.0, gy = 0.0, gz = 0.0;
             load_x(x, m.iqseq[iq], xi);
             if (act) {
@@ -2110,7 +2110,7 @@ __global__ void __launch_bounds__(128) k_qenv64(DevModel m, const DevState* __re
         }
         const double v = reduce_scatter<16>(g, lane);
         const int idx = lane >> 1;   // the component this lane pair holds
-        if (!(lane & 1) && idx < 3 * kQRed && 3 * q0 + idx < 3 * nq)
+        if (!(lane & 1) && idx < 3 * (q1 - q0))
             atomicAdd(s.d + 3 * m.iqseq[q0 + idx / 3] + idx % 3, v);
         if (act) {
 #pragma unroll
@@ -4415,9 +4415,16 @@ void launch_qenv(const Launch& L, int mixed, int per_sm, const int* iwhich, doub
 #undef QT
         return;
     }
-    const int64_t items = (int64_t)((units + 31) / 32) * ((L.m.nqat + kQRed - 1) / kQRed);
+    // Q atoms per warp: the fewest that keep all windows' warps to eight per
+    // SM.  Few warps wait for their own dependent chains, more only add rounds
+    // and atomics: waters of one 15 A droplet with 6 Q atoms 33 us in blocks of
+    // five, 14 one by one; one 25 A sphere with 20 34 and 18, eight 51 and 61
+    const int uw = (units + 31) / 32;
+    int qb = 1;
+    while (qb < kQRed && (int64_t)uw * L.nwin * ((L.m.nqat + qb - 1) / qb) > 8 * (int64_t)sms()) ++qb;
+    const int64_t items = (int64_t)uw * ((L.m.nqat + qb - 1) / qb);
     dim3 g = grid_for(items * 32, 128, 2 * per_sm, L.nwin);
-#define Q64(SPC, NA, SM, BX) k_qenv64<SPC, WATER, NA, SM, BX><<<g, 128, 0, L.st>>>(L.m, L.ds, iwhich, rcq2)
+#define Q64(SPC, NA, SM, BX) k_qenv64<SPC, WATER, NA, SM, BX><<<g, 128, 0, L.st>>>(L.m, L.ds, iwhich, rcq2, qb)
 #define Q6S(SPC, NA, BX) do { if (s4) Q64(SPC, NA, 4, BX); else Q64(SPC, NA, kMaxStates, BX); } while (0)
 #define Q6B(SPC, NA) do { if (box) Q6S(SPC, NA, true); else Q6S(SPC, NA, false); } while (0)
     if constexpr (!WATER) Q6B(true, 1);
